@@ -36,143 +36,12 @@
 #include <string>
 #include <utility>
 
+#include "pmx_dft.cuh"
 #include "pmx_internal.cuh"
 
 namespace pmx {
 
 namespace {
-
-constexpr double kPi = 3.141592653589793238462643383279502884;
-
-// cos/sin by their Taylor series on [-pi, pi], evaluated at compile time;
-// used only for the exact small-radix twiddles exp(-2 pi i k / R), R <= 32.
-constexpr double taylor_cos(double x) {
-    double term = 1.0, sum = 1.0;
-    for (int i = 1; i < 24; ++i) {
-        term *= -x * x / ((2.0 * i - 1.0) * (2.0 * i));
-        sum += term;
-    }
-    return sum;
-}
-constexpr double taylor_sin(double x) {
-    double term = x, sum = x;
-    for (int i = 1; i < 24; ++i) {
-        term *= -x * x / ((2.0 * i) * (2.0 * i + 1.0));
-        sum += term;
-    }
-    return sum;
-}
-
-struct Twiddle32 {
-    float c[32], s[32];  // cos / sin of 2 pi k / 32
-    constexpr Twiddle32() : c(), s() {
-        for (int k = 0; k < 32; ++k) {
-            double a = 2.0 * kPi * k / 32.0;
-            if (a > kPi) a -= 2.0 * kPi;
-            c[k] = (float)taylor_cos(a);
-            s[k] = (float)taylor_sin(a);
-        }
-    }
-};
-
-template <int R>
-struct Log2 {
-    static constexpr int v = R <= 1 ? 0 : 1 + Log2<R / 2>::v;
-};
-template <>
-struct Log2<1> {
-    static constexpr int v = 0;
-};
-
-// In-register DFT of length R (power of two, <= 32): natural-order input,
-// output in bit-reversed order (element k holds frequency brev(k)); radix-2
-// decimation in frequency.  The butterflies are generated by fold
-// expressions so every register index is a compile-time constant (the
-// arrays stay in registers).  INV selects exp(+2 pi i ...) (unnormalised).
-constexpr Twiddle32 kTw32 = Twiddle32();
-
-template <int R, bool INV, int S, int J>
-__device__ __forceinline__ void bfly(float (&re)[R], float (&im)[R]) {
-    constexpr int half = 1 << (S - 1), len = 1 << S;
-    constexpr int g = J / half, k = J % half;
-    constexpr int a = g * len + k, b = a + half, ti = k * (32 >> S);
-    const float ur = re[a], ui = im[a], vr = re[b], vi = im[b];
-    re[a] = ur + vr;
-    im[a] = ui + vi;
-    const float dr = ur - vr, di = ui - vi;
-    // twiddle exp(-+2 pi i ti / 32), a compile-time constant; 1 and -+i exactly
-    if constexpr (ti == 0) {
-        re[b] = dr;
-        im[b] = di;
-    } else if constexpr (ti == 8) {
-        re[b] = INV ? -di : di;
-        im[b] = INV ? dr : -dr;
-    } else {
-        constexpr float wc = kTw32.c[ti];
-        constexpr float ws = INV ? kTw32.s[ti] : -kTw32.s[ti];
-        re[b] = dr * wc - di * ws;
-        im[b] = dr * ws + di * wc;
-    }
-}
-
-template <int R, bool INV, int S, int... Js>
-__device__ __forceinline__ void dft_stage(float (&re)[R], float (&im)[R],
-                                          std::integer_sequence<int, Js...>) {
-    (bfly<R, INV, S, Js>(re, im), ...);
-}
-
-template <int R, bool INV, int... Ss>
-__device__ __forceinline__ void dft_stages(float (&re)[R], float (&im)[R],
-                                           std::integer_sequence<int, Ss...>) {
-    (dft_stage<R, INV, Log2<R>::v - Ss>(re, im, std::make_integer_sequence<int, R / 2>{}), ...);
-}
-
-template <int R, bool INV>
-__device__ __forceinline__ void dft(float (&re)[R], float (&im)[R]) {
-    dft_stages<R, INV>(re, im, std::make_integer_sequence<int, Log2<R>::v>{});
-}
-
-// bit reversal of the low `bits` bits
-__device__ __forceinline__ int brev(int k, int bits) { return (int)(__brev((unsigned)k) >> (32 - bits)); }
-
-
-constexpr int cbrev(int k, int bits) {
-    int r = 0;
-    for (int b = 0; b < bits; ++b) r |= ((k >> b) & 1) << (bits - 1 - b);
-    return r;
-}
-
-// out[i] = in[brev(i)]: bit-reversed register order -> natural order, with
-// compile-time indices (fold expression).
-template <int R, int... Is>
-__device__ __forceinline__ void unbrev_impl(const float2 (&in)[R], float2 (&out)[R],
-                                            std::integer_sequence<int, Is...>) {
-    ((out[Is] = in[cbrev(Is, Log2<R>::v)]), ...);
-}
-template <int R>
-__device__ __forceinline__ void unbrev(const float2 (&in)[R], float2 (&out)[R]) {
-    unbrev_impl<R>(in, out, std::make_integer_sequence<int, R>{});
-}
-
-// float2 wrappers of the split-array register DFT
-template <int R, bool INV, int... Is>
-__device__ __forceinline__ void dft2_impl(float2 (&v)[R], std::integer_sequence<int, Is...>) {
-    float re[R], im[R];
-    ((re[Is] = v[Is].x, im[Is] = v[Is].y), ...);
-    dft<R, INV>(re, im);
-    ((v[Is] = make_float2(re[Is], im[Is])), ...);
-}
-template <int R, bool INV>
-__device__ __forceinline__ void dft2(float2 (&v)[R]) {
-    dft2_impl<R, INV>(v, std::make_integer_sequence<int, R>{});
-}
-
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
-    return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
 
 template <int N>
 struct Split;  // N = R1 * R2

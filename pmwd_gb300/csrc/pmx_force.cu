@@ -114,6 +114,10 @@ struct pmx_workspace {
     // power-of-two meshes: slab-wise 2-D cuFFT over (y, z) plus the fused
     // x pass of pmx_fft.cu; meshes are then plane-interleaved (x, 3, n1, n2)
     bool xfast = false;
+    // every axis length supported by the mesh transforms of pmx_mesh_fft.cuh:
+    // they replace cuFFT and the x pass (meshes plane-interleaved as above)
+    bool own = false;
+    float2 *mtw = nullptr;      // their twiddle tables
     bool win = false;           // warp-window deposits (n2 % 4 == 0)
     int64_t slab = 0;           // x-planes per 2-D cuFFT execution
     float2 *tw = nullptr;       // exp(-2 pi i m / n0)
@@ -1643,11 +1647,49 @@ float green_c(const pmx_workspace *ws, double omega_m) {
     return (float)((double)s / (double)ws->M);
 }
 
+// The Poisson solve by the library's own mesh transforms: dens -> g (adj =
+// false), or mcot -> rcot_of(nslot) (adj = true).  ck holds the half rows; the
+// spectra live in g, which is free until the z axis writes it: the forward
+// c2r after the y axis has read them, the adjoint's rcot where D was.
+int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStream_t st) {
+    MeshGeom g;
+    g.n0 = ws->n0;
+    g.n1 = ws->n1;
+    g.n2h = (int)ws->n2h;
+    g.nzt = (int)(ws->n2p / 4);
+    g.unit = ws->n0 * ws->n1 * ws->n2p;
+    GreenTab gt;
+    for (int b = 0; b < nslot; ++b) gt.c[b] = c[b];
+    float2 *s0 = reinterpret_cast<float2 *>(ws->g), *s1 = s0 + nslot * g.unit;
+    const float2 *tx = ws->mtw, *ty = tx + 2 * ws->n0, *tz = ty + 2 * ws->n1;
+    const int64_t planes = nslot * ws->n0;
+    int e;
+    {
+        Stage sg(ws, adj ? 8 : 2, st, 2);
+        if ((e = mesh_rows(false, adj ? ws->mcot : ws->dens, ws->ck, tz, adj ? 3 * planes : planes,
+                           ws->n1, ws->n2, st)) ||
+            (e = mesh_cols(adj ? MESH_COLS_ADJ : MESH_COLS_FWD, nslot, g, ws->ck, s0, s1, ty, ws->ktab,
+                           st)))
+            return e;
+    }
+    {
+        Stage sg(ws, adj ? 9 : 3, st, 1);
+        if ((e = mesh_xaxis(adj, nslot, g, s0, s1, tx, ws->ktab, gt, st))) return e;
+    }
+    Stage sg(ws, adj ? 10 : 4, st, 2);
+    if ((e = mesh_cols(adj ? MESH_COLS_INV1 : MESH_COLS_INV3, nslot, g, ws->ck, s0, s1, ty, ws->ktab,
+                       st)))
+        return e;
+    return mesh_rows(true, ws->ck, adj ? ws->rcot_of(nslot) : ws->g, tz, adj ? planes : 3 * planes,
+                     ws->n1, ws->n2, st);
+}
+
 // Forward force up to the three acceleration meshes in ws->g, for the
 // densities of the first nslot slots (slot b: Green's constant c[b]); the
 // slots' spectra and meshes are consecutive, so each plane transform runs
 // over all their planes at once.
 int force_meshes_b(pmx_workspace *ws, int nslot, const float *c, cudaStream_t st) {
+    if (ws->own) return own_meshes(ws, false, nslot, c, st);
     if (ws->xfast) {
         float2 *H = reinterpret_cast<float2 *>(ws->g);  // g is free until the c2r
         const int64_t pc = ws->n0 * ws->n1 * ws->n2p;  // complex values per slot spectrum
@@ -1707,6 +1749,7 @@ int force_meshes_b(pmx_workspace *ws, int nslot, const float *c, cudaStream_t st
 // operator, c2r into rcot_of(nslot) (then rho_cot of each slot, scale
 // folded in).
 int force_adj_meshes_b(pmx_workspace *ws, int nslot, const float *c, cudaStream_t st) {
+    if (ws->own) return own_meshes(ws, true, nslot, c, st);
     if (ws->xfast) {
         float2 *Sk = reinterpret_cast<float2 *>(ws->g);  // g is dead after k_g3adj
         float *rcot = ws->rcot_of(nslot);
@@ -1838,6 +1881,7 @@ void ws_free(pmx_workspace *ws) {
     if (ws->cap) cudaStreamDestroy(ws->cap);
     if (ws->fork) cudaEventDestroy(ws->fork);
     cudaFree(ws->tw);
+    cudaFree(ws->mtw);
     cudaFree(ws->ptw);
     cudaFree(ws->pscr);
     cudaFree(ws->dens);
@@ -1856,8 +1900,19 @@ void ws_free(pmx_workspace *ws) {
     delete ws;
 }
 
+// Whether a workspace of this shape and flags uses the mesh transforms of
+// pmx_mesh_fft.cuh.  They are faster at every supported size (force + VJP at
+// 64^3 62 against 72 us of device time, 1024^3 35.6 against 43.6 ms), but one
+// force takes eight launches instead of six, which shows at 64^3, where the
+// host's launches are the bound (70 against 76 us per force).
+bool own_path(const int64_t s[3], int32_t flags) {
+    return mesh_fft_supported(s[0], s[1], s[2]) && s[0] * s[1] * s[2] > 64 * 64 * 64 &&
+           !(flags & (PMX_WS_CUFFT3D | PMX_WS_PLANE));
+}
+
 size_t buffers_bytes(const int64_t s[3], int32_t flags, int32_t slots) {
     int64_t M = s[0] * s[1] * s[2], Mc = s[0] * s[1] * (s[2] / 2 + 1);
+    if (own_path(s, flags)) Mc = s[0] * s[1] * padded_row(s[2] / 2 + 1);
     size_t b = (size_t)M * 4 + (size_t)Mc * 8 * 3 + (size_t)M * 4 * 3;
     if (flags & PMX_WS_ADJOINT) b += (size_t)M * 4 * 3;
     b += (size_t)NSLOT * (slots == 1 ? PART_ONE : PART_SLOT) * 8;
@@ -1911,6 +1966,7 @@ extern "C" int pmx_workspace_bytes(const int64_t mesh_shape[3], int32_t flags, s
     cufftType types[4] = {CUFFT_R2C, CUFFT_C2R, CUFFT_R2C, CUFFT_C2R};
     int64_t batches[4] = {1, 3, 3, 1};
     int nplans = (flags & PMX_WS_ADJOINT) ? 4 : 2;
+    if (own_path(mesh_shape, flags)) nplans = 0;   // no cuFFT work area
     for (int i = 0; i < nplans; ++i) {
         int n[3] = {(int)mesh_shape[0], (int)mesh_shape[1], (int)mesh_shape[2]};
         size_t w = 0;
@@ -1950,12 +2006,13 @@ static int ws_create(const int64_t mesh_shape[3], int32_t flags, int32_t slots,
         }
         return PMX_OK;
     };
-    ws->xfast = xpass_supported(ws->n0) && !(flags & PMX_WS_CUFFT3D);
+    ws->own = own_path(mesh_shape, flags);
+    ws->xfast = ws->own || (xpass_supported(ws->n0) && !(flags & PMX_WS_CUFFT3D));
     ws->plane = ws->xfast && plane_supported(ws->n1, ws->n2) && (flags & PMX_WS_PLANE);
     ws->plane16 = (flags & PMX_WS_PLANE16) != 0;
     ws->vec = ws->n2 % 4 == 0 && (flags & PMX_WS_VEC);
     ws->agg = (flags & PMX_WS_AGG) && (uint64_t)ws->M * (uint64_t)slots < 0xFFFFFFE0ull;
-    ws->n2p = ws->plane ? padded_row(ws->n2h) : ws->n2h;
+    ws->n2p = ws->plane || ws->own ? padded_row(ws->n2h) : ws->n2h;
     int64_t ktn = 2 * (ws->n0 + ws->n1 + ws->n2h);
     const int64_t B = slots;
     if ((st = alloc((void **)&ws->dens, B * ws->M * 4)) ||
@@ -1994,7 +2051,26 @@ static int ws_create(const int64_t mesh_shape[3], int32_t flags, int32_t slots,
             return fail(PMX_ERR_CUDA, "plane twiddle upload failed");
         }
     }
-    if (ws->xfast) {
+    if (ws->own) {
+        const int64_t nt = mesh_fft_twiddles(ws->n0, ws->n1, ws->n2, nullptr);
+        std::vector<float2> t(nt);
+        mesh_fft_twiddles(ws->n0, ws->n1, ws->n2, t.data());
+        if ((st = alloc((void **)&ws->mtw, nt * sizeof(float2)))) { ws_free(ws); return st; }
+        if (cudaMemcpy(ws->mtw, t.data(), nt * sizeof(float2), cudaMemcpyHostToDevice) !=
+            cudaSuccess) {
+            ws_free(ws);
+            return fail(PMX_ERR_CUDA, "mesh transform twiddle upload failed");
+        }
+        if ((st = mesh_rows_prepare(ws->n2)) || (st = mesh_cols_prepare(ws->n1)) ||
+            (st = mesh_xaxis_prepare(ws->n0))) {
+            ws_free(ws);
+            return st;
+        }
+        for (int i = 0; i < 4; ++i) {
+            ph[i] = nullptr;
+            hv[i] = nullptr;
+        }
+    } else if (ws->xfast) {
         ws->slab = choose_slab(ws->n0, ws->n1, ws->n2, (flags >> PMX_WS_SLAB_SHIFT) & 15);
         const int64_t S = ws->slab;
         if (!ws->plane) {

@@ -73,6 +73,36 @@ struct EmParams {
 
 int make_em_params(const pmx_enmesh_spec *spec, EmParams *p);
 
+// 3-D mesh transforms of the Poisson solve by this library's own kernels
+// (pmx_mesh_fft.cuh; pmx_mesh_rows.cu, pmx_mesh_cols.cu, pmx_mesh_x.cu).
+struct MeshGeom {
+    int64_t n0, n1;      // planes and rows
+    int nzt;             // blocks of 4 kz values: ceil((n2 / 2 + 1) / 4)
+    int n2h;
+    int64_t unit;        // complex values of one spectrum: n0 n1 4 nzt
+};
+
+constexpr int MESH_SLOTS = 16;
+struct GreenTab {
+    float c[MESH_SLOTS];   // 1.5 Omega_m / N of each slot
+};
+bool mesh_fft_supported(int64_t n0, int64_t n1, int64_t n2);
+// Writes the twiddle tables to t (unless NULL); returns their length.
+int64_t mesh_fft_twiddles(int64_t n0, int64_t n1, int64_t n2, float2 *t);
+int mesh_rows_prepare(int64_t n2);   // once per workspace: shared-memory opt-ins
+int mesh_rows_factors(int64_t n2, int *R1, int *R2);   // of the half length
+int mesh_cols_prepare(int64_t n1);
+int mesh_xaxis_prepare(int64_t n0);
+// z axis of `planes` consecutive planes: real <-> nat.
+int mesh_rows(bool inv, const void *in, void *out, const float2 *tw, int64_t planes, int64_t n1,
+              int64_t n2, cudaStream_t st);
+enum { MESH_COLS_FWD, MESH_COLS_ADJ, MESH_COLS_INV1, MESH_COLS_INV3 };
+// y axis of nslot slots: nat <-> spectra (one, or two: spec0 and spec1).
+int mesh_cols(int kind, int nslot, const MeshGeom &g, float2 *nat, float2 *spec0, float2 *spec1,
+              const float2 *tw, const float *kt, cudaStream_t st);
+int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, const float2 *tw,
+               const float *kt, const GreenTab &gt, cudaStream_t st);
+
 // Fused x-axis pass of the Poisson solve (pmx_fft.cu).  Forward (adj =
 // false): in = FFT_yz(rho) (n0, n1, n2h), out = the three gradient spectra
 // (n0, 3, n1, n2h) after the inverse x transform.  Adjoint: in = FFT_yz of

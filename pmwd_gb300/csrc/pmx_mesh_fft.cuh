@@ -1,0 +1,168 @@
+// 3-D mesh transforms of the Poisson solve, axis by axis, with the
+// Fourier-space operators of pmwd/gravity.py:9-72 fused into the x axis.
+//
+// Forward force (rho -> three acceleration meshes):
+//   k_rows_r2c   z axis:  real rows -> half rows
+//   k_cols_fwd   y axis:  half rows -> H(x; ky, kz)
+//   k_xaxis_fwd  x axis:  P = -(c / k^2) FFT_x(H),  G_0 = IFFT_x(-i kx P),
+//                         Q = IFFT_x(P)
+//   k_cols_inv   y axis:  IFFT_y of G_0, -i ky Q and -i kz Q (ky and kz are
+//                         constant along x, so Q serves both)
+//   k_rows_c2r   z axis:  half rows -> real rows
+// Force VJP (cotangents of the three meshes -> cotangent of rho), the exact
+// transpose:
+//   k_rows_r2c; k_cols_adj (C_0 = FFT_y, D = i ky FFT_y(C_1) + i kz FFT_y(C_2));
+//   k_xaxis_adj (S = IFFT_x(-(c / k^2) [i kx FFT_x(C_0) + FFT_x(D)]));
+//   k_cols_inv; k_rows_c2r.
+// Two spectra instead of three pass through the x axis in either direction.
+//
+// Every length-N transform is N = R1 * R2: radix-R1 DFTs of R2-strided
+// elements in registers, twiddles, ONE exchange through shared memory,
+// radix-R2 DFTs, straight from and to global memory -- no staging copies.
+// At N = 1024 a block of 128 threads holds 4 columns (34 KB), so several
+// blocks share an SM and one's loads overlap another's arithmetic.
+//
+// Measured at 1024^3 (GB300, ms): rows r2c 1.43, cols fwd 1.50, x fwd 4.2,
+// cols inv3 5.35, rows c2r 3 x 1.30; adjoint rows 4.27, cols 5.85, x 4.1,
+// cols inv1 1.88, rows 1.30.  The cuFFT plane transforms and the tiled x pass
+// that they replace: r2c 3.4, x 6.8, c2r 11.1; adjoint 10.1, 8.5, 3.7.
+//
+// Layouts.  Strided axes make the memory system, not the arithmetic, the
+// bound: at 1024^3 an x-axis column in a natural (x, ky, kz) array is read in
+// 64-byte pieces 4.2 MB apart, 2.5 TB/s at best.  Two blocked layouts of
+// complex64 in units of 32 values (256 bytes, one warp-wide access) avoid
+// that; kz is padded to a multiple of 4:
+//   half rows ("nat"):  (plane, y / 8, kz / 4, y % 8, kz % 4)
+//   spectra ("spec"):   (x / 8, ky, kz / 4, x % 8, kz % 4)
+// The z kernels write nat from 8 rows at a time and the x kernels touch spec
+// in whole 256-byte blocks; only the y kernels see 32-byte pieces (on the
+// spec side), and the blocks of eight x-planes that fill one 256-byte block
+// run next to each other, so L2 merges them.
+
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "pmx_dft.cuh"
+#include "pmx_internal.cuh"
+
+namespace pmx {
+
+// N = R1 * R2, R1 >= R2 except 768; T columns per block.
+template <int N>
+struct Fac;
+template <> struct Fac<64> { static constexpr int R1 = 8, R2 = 8; };
+template <> struct Fac<96> { static constexpr int R1 = 12, R2 = 8; };
+template <> struct Fac<128> { static constexpr int R1 = 16, R2 = 8; };
+template <> struct Fac<192> { static constexpr int R1 = 24, R2 = 8; };
+template <> struct Fac<256> { static constexpr int R1 = 16, R2 = 16; };
+template <> struct Fac<384> { static constexpr int R1 = 24, R2 = 16; };
+template <> struct Fac<512> { static constexpr int R1 = 32, R2 = 16; };
+template <> struct Fac<768> { static constexpr int R1 = 24, R2 = 32; };
+template <> struct Fac<1024> { static constexpr int R1 = 32, R2 = 32; };
+
+template <int N>
+struct ColCfg {
+    static constexpr int R1 = Fac<N>::R1, R2 = Fac<N>::R2;
+    static constexpr int T = 128 / R2 < 4 ? 4 : 128 / R2;   // columns per block
+    static constexpr int TH = T * R2;                       // stage 1: one radix-R1 DFT per thread
+    // shared exchange buffer: element (k1, b) of column t at k1 * GS + b * T + t;
+    // R2 + 1 odd keeps both sides free of bank conflicts
+    static constexpr int GS = (R2 + 1) * T;
+    static constexpr int BUF = R1 * GS;
+};
+
+// Twiddle tables of a length-N transform (float2): w^(b k1) at k1 * R2 + b,
+// then the same at b * R1 + k1 (w = exp(-2 pi i / N)).
+template <int N>
+__device__ __forceinline__ const float2 *tw_fwd(const float2 *tw) { return tw; }
+template <int N>
+__device__ __forceinline__ const float2 *tw_tr(const float2 *tw) { return tw + N; }
+
+// R1 and R2 of a supported axis length (or half length), on the host.
+template <class F>
+void mesh_axis_r(int64_t n, F &&f) {
+    switch (n) {
+        case 64: f(Fac<64>::R1, Fac<64>::R2); break;
+        case 96: f(Fac<96>::R1, Fac<96>::R2); break;
+        case 128: f(Fac<128>::R1, Fac<128>::R2); break;
+        case 192: f(Fac<192>::R1, Fac<192>::R2); break;
+        case 256: f(Fac<256>::R1, Fac<256>::R2); break;
+        case 384: f(Fac<384>::R1, Fac<384>::R2); break;
+        case 512: f(Fac<512>::R1, Fac<512>::R2); break;
+        case 768: f(Fac<768>::R1, Fac<768>::R2); break;
+        case 1024: f(Fac<1024>::R1, Fac<1024>::R2); break;
+    }
+}
+
+__device__ __forceinline__ int64_t spec_at(const MeshGeom &g, int64_t x, int ky, int l) {
+    return (((x >> 3) * g.n1 + ky) * g.nzt + (l >> 2)) * 32 + (x & 7) * 4 + (l & 3);
+}
+
+
+// Stage 1 of T columns: v holds elements b + a R2 of column t; radix-R1 DFT,
+// twiddles, exchange buffer.
+template <int N, bool INV>
+__device__ __forceinline__ void col_stage1(float2 (&v)[Fac<N>::R1], float2 *buf, int t, int b,
+                                           const float2 *__restrict__ tw) {
+    using C = ColCfg<N>;
+    reg_dft<C::R1, INV>(v);
+    static_for<C::R1>([&](auto E) {
+        constexpr int k1 = reg_freq<C::R1>(E);
+        float2 x = v[E];
+        if constexpr (k1 != 0) {
+            const float2 w = __ldg(tw + k1 * C::R2 + b);
+            x = INV ? cmulc(x, w) : cmul(x, w);
+        }
+        buf[k1 * C::GS + b * C::T + t] = x;
+    });
+}
+
+// Stage 2 of group (t, k1): u[e] holds frequency k1 + R1 reg_freq(e).
+template <int N, bool INV>
+__device__ __forceinline__ void col_stage2(float2 (&u)[Fac<N>::R2], const float2 *buf, int t,
+                                           int k1) {
+    using C = ColCfg<N>;
+#pragma unroll
+    for (int b = 0; b < C::R2; ++b) u[b] = buf[k1 * C::GS + b * C::T + t];
+    reg_dft<C::R2, INV>(u);
+}
+
+// Keeps values parked in shared memory there: without it the compiler forwards
+// the stores to the later loads in registers, which costs a block per SM.
+__device__ __forceinline__ void parked() { asm volatile("" ::: "memory"); }
+
+// Blocks per SM that `bufs` exchange buffers leave room for, at most 8.
+template <int N>
+constexpr int col_blocks(int bufs) {
+    const int by_smem = 227 * 1024 / (bufs * ColCfg<N>::BUF * 8 + 1024);
+    return by_smem < 1 ? 1 : (by_smem > 8 ? 8 : by_smem);
+}
+
+template <class K>
+int smem_opt_in(K *fn, size_t bytes) {
+    if (bytes <= 48 * 1024) return PMX_OK;
+    PMX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return PMX_OK;
+}
+template <int N>
+constexpr size_t cols_smem(int bufs) { return (size_t)bufs * ColCfg<N>::BUF * sizeof(float2); }
+
+// Calls f(integral_constant<int, N>{}) for the supported length n.
+template <class F>
+int mesh_axis_dispatch(int64_t n, F &&f) {
+    switch (n) {
+        case 64: return f(std::integral_constant<int, 64>{});
+        case 96: return f(std::integral_constant<int, 96>{});
+        case 128: return f(std::integral_constant<int, 128>{});
+        case 192: return f(std::integral_constant<int, 192>{});
+        case 256: return f(std::integral_constant<int, 256>{});
+        case 384: return f(std::integral_constant<int, 384>{});
+        case 512: return f(std::integral_constant<int, 512>{});
+        case 768: return f(std::integral_constant<int, 768>{});
+        case 1024: return f(std::integral_constant<int, 1024>{});
+        default: return fail(PMX_ERR_SHAPE, "mesh transform length not supported");
+    }
+}
+
+}  // namespace pmx

@@ -1,0 +1,221 @@
+// x-axis transforms of the Poisson solve, fused with the Green's function and
+// the gradients (see pmx_mesh_fft.cuh).
+
+#include <cmath>
+
+#include "pmx_mesh_fft.cuh"
+
+namespace pmx {
+
+namespace {
+
+// Inverse first step on a register group in natural order: radix-R2 inverse
+// DFT, conjugate twiddles, back into the group's own place in the buffer.
+template <int N>
+__device__ __forceinline__ void x_inv_step2(const float2 (&w)[Fac<N>::R2], float2 *buf, int t,
+                                            int k1, const float2 *__restrict__ twt) {
+    using C = ColCfg<N>;
+    float2 u[C::R2];
+    reg_natural<C::R2>(w, u);
+    reg_dft<C::R2, true>(u);
+    static_for<C::R2>([&](auto E) {
+        constexpr int b = reg_freq<C::R2>(E);
+        float2 x = u[E];
+        if constexpr (b != 0) x = cmulc(x, __ldg(twt + b * C::R1 + k1));
+        buf[k1 * C::GS + b * C::T + t] = x;
+    });
+}
+
+// Inverse second step: radix-R1 inverse DFTs over k1, stored to column t at
+// x = b + a R2.
+template <int N>
+__device__ __forceinline__ void x_inv_step1(const float2 *buf, int t, int b, float2 *dst,
+                                            int64_t xbs) {
+    using C = ColCfg<N>;
+    float2 v[C::R1];
+#pragma unroll
+    for (int k1 = 0; k1 < C::R1; ++k1) v[k1] = buf[k1 * C::GS + b * C::T + t];
+    reg_dft<C::R1, true>(v);
+    static_for<C::R1>([&](auto E) {
+        const int x = b + reg_freq<C::R1>(E) * C::R2;
+        dst[(x >> 3) * xbs + (x & 7) * 4] = v[E];
+    });
+}
+
+// s0: H in, G_0 out (in place: a block reads its whole tile before it
+// writes); s1: Q out.
+template <int N>
+__global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_fwd(float2 *s0, float2 *s1,
+                                                             const float2 *__restrict__ tw,
+                                                             const float *__restrict__ kt,
+                                                             const __grid_constant__ GreenTab gt,
+                                                             MeshGeom g) {
+    using C = ColCfg<N>;
+    constexpr int R1 = C::R1, R2 = C::R2;
+    extern __shared__ __align__(16) float2 sm[];
+    float2 *A = sm, *B = sm + C::BUF;
+    const int nct = (4 * g.nzt + C::T - 1) / C::T;
+    const int t = threadIdx.x % C::T, b = threadIdx.x / C::T;
+    const int ky = blockIdx.x / nct, l = (blockIdx.x % nct) * C::T + t;
+    const bool ok = l < 4 * g.nzt;
+    const int64_t xbs = g.n1 * g.nzt * 32;                  // 8 x-planes
+    const int64_t at = blockIdx.y * g.unit + ((int64_t)ky * g.nzt + (ok ? l >> 2 : 0)) * 32 + (l & 3);
+    float2 *p0 = s0 + at, *p1 = s1 + at;
+    {
+        float2 v[R1];
+#pragma unroll
+        for (int a = 0; a < R1; ++a) {
+            const int x = b + a * R2;
+            v[a] = p0[(x >> 3) * xbs + (x & 7) * 4];
+        }
+        col_stage1<N, false>(v, A, t, b, tw_fwd<N>(tw));
+    }
+    __syncthreads();
+    const int64_t tot = g.n0 + g.n1 + g.n2h;
+    const float kyj = __ldg(kt + g.n0 + ky), kzl = l < g.n2h ? __ldg(kt + g.n0 + g.n1 + l) : 0.f;
+    const float ky2 = __fmul_rn(kyj, kyj), kz2 = __fmul_rn(kzl, kzl);
+    const float cc = gt.c[blockIdx.y];
+    for (int k1 = b; k1 < R1; k1 += R2) {
+        float2 v[R2];
+        col_stage2<N, false>(v, A, t, k1);
+        float2 w[R2];
+        static_for<R2>([&](auto E) {
+            const int ix = k1 + R1 * reg_freq<R2>(E);
+            const float kxi = __ldg(kt + ix), mxi = __ldg(kt + tot + ix);
+            const float k2v = __fadd_rn(__fadd_rn(__fmul_rn(kxi, kxi), ky2), kz2);
+            // laplace (k = 0 -> 0); c / k^2 to within 2 ulp
+            const float rk = k2v != 0.f ? __fdividef(cc, k2v) : 0.f;
+            const float pr = -__fmul_rn(v[E].x, rk), pi = -__fmul_rn(v[E].y, rk);
+            // P waits in the thread's own group of A while G_0 is transformed
+            A[k1 * C::GS + E * C::T + t] = make_float2(pr, pi);
+            w[E] = make_float2(__fmul_rn(mxi, pi), -__fmul_rn(mxi, pr));  // -i kx P
+        });
+        x_inv_step2<N>(w, B, t, k1, tw_tr<N>(tw));
+        parked();
+        static_for<R2>([&](auto E) { v[E] = A[k1 * C::GS + E * C::T + t]; });
+        x_inv_step2<N>(v, A, t, k1, tw_tr<N>(tw));
+    }
+    __syncthreads();
+    if (!ok) return;
+    x_inv_step1<N>(B, t, b, p0, xbs);
+    x_inv_step1<N>(A, t, b, p1, xbs);
+}
+
+// s0: C_0 in, S out (in place); s1: D in.
+template <int N>
+__global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_adj(float2 *s0, const float2 *s1,
+                                                             const float2 *__restrict__ tw,
+                                                             const float *__restrict__ kt,
+                                                             const __grid_constant__ GreenTab gt,
+                                                             MeshGeom g) {
+    using C = ColCfg<N>;
+    constexpr int R1 = C::R1, R2 = C::R2;
+    extern __shared__ __align__(16) float2 sm[];
+    float2 *A = sm, *B = sm + C::BUF;
+    const int nct = (4 * g.nzt + C::T - 1) / C::T;
+    const int t = threadIdx.x % C::T, b = threadIdx.x / C::T;
+    const int ky = blockIdx.x / nct, l = (blockIdx.x % nct) * C::T + t;
+    const bool ok = l < 4 * g.nzt;
+    const int64_t xbs = g.n1 * g.nzt * 32;
+    const int64_t at = blockIdx.y * g.unit + ((int64_t)ky * g.nzt + (ok ? l >> 2 : 0)) * 32 + (l & 3);
+    float2 *p0 = s0 + at;
+#pragma unroll 1
+    for (int j = 0; j < 2; ++j) {
+        const float2 *p = j ? s1 + at : p0;
+        float2 v[R1];
+#pragma unroll
+        for (int a = 0; a < R1; ++a) {
+            const int x = b + a * R2;
+            v[a] = p[(x >> 3) * xbs + (x & 7) * 4];
+        }
+        col_stage1<N, false>(v, sm + j * C::BUF, t, b, tw_fwd<N>(tw));
+    }
+    __syncthreads();
+    const int64_t tot = g.n0 + g.n1 + g.n2h;
+    const float kyj = __ldg(kt + g.n0 + ky), kzl = l < g.n2h ? __ldg(kt + g.n0 + g.n1 + l) : 0.f;
+    const float ky2 = __fmul_rn(kyj, kyj), kz2 = __fmul_rn(kzl, kzl);
+    const float cc = gt.c[blockIdx.y];
+    for (int k1 = b; k1 < R1; k1 += R2) {
+        float2 v[R2];
+        col_stage2<N, false>(v, A, t, k1);
+        static_for<R2>([&](auto E) { A[k1 * C::GS + E * C::T + t] = v[E]; });
+        parked();
+        col_stage2<N, false>(v, B, t, k1);
+        static_for<R2>([&](auto E) {
+            const int ix = k1 + R1 * reg_freq<R2>(E);
+            const float kxi = __ldg(kt + ix), mxi = __ldg(kt + tot + ix);
+            const float k2v = __fadd_rn(__fadd_rn(__fmul_rn(kxi, kxi), ky2), kz2);
+            const float2 c0 = A[k1 * C::GS + E * C::T + t];
+            const float re = __fadd_rn(-__fmul_rn(mxi, c0.y), v[E].x);
+            const float im = __fadd_rn(__fmul_rn(mxi, c0.x), v[E].y);
+            const float rk = k2v != 0.f ? __fdividef(cc, k2v) : 0.f;
+            v[E] = make_float2(-__fmul_rn(re, rk), -__fmul_rn(im, rk));
+        });
+        x_inv_step2<N>(v, A, t, k1, tw_tr<N>(tw));
+    }
+    __syncthreads();
+    if (!ok) return;
+    x_inv_step1<N>(A, t, b, p0, xbs);
+}
+
+}  // namespace
+
+int mesh_xaxis_prepare(int64_t n0) {
+    return mesh_axis_dispatch(n0, [&](auto N) -> int {
+        int st = smem_opt_in(k_xaxis_fwd<N>, cols_smem<N>(2));
+        return st ? st : smem_opt_in(k_xaxis_adj<N>, cols_smem<N>(2));
+    });
+}
+
+int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, const float2 *tw,
+               const float *kt, const GreenTab &gt, cudaStream_t st) {
+    return mesh_axis_dispatch(g.n0, [&](auto N) -> int {
+        using C = ColCfg<N>;
+        const dim3 grid((unsigned)(g.n1 * ((4 * g.nzt + C::T - 1) / C::T)), nslot);
+        if (adj)
+            k_xaxis_adj<N><<<grid, C::TH, cols_smem<N>(2), st>>>(s0, s1, tw, kt, gt, g);
+        else
+            k_xaxis_fwd<N><<<grid, C::TH, cols_smem<N>(2), st>>>(s0, s1, tw, kt, gt, g);
+        PMX_LAUNCH_CHECK("mesh transform, x axis");
+        return PMX_OK;
+    });
+}
+
+// Tables in tw: the x axis' 2 n0 entries, the y axis' 2 n1, then the z axis'
+// 2 L and the split's L + 1 (L = n2 / 2); float64 on the host, then float32.
+static void axis_table(int64_t n, int R1, int R2, float2 *t) {
+    for (int k1 = 0; k1 < R1; ++k1)
+        for (int b = 0; b < R2; ++b) {
+            const double a = -2.0 * kPi * (double)(b * k1) / (double)n;
+            const float2 w = make_float2((float)std::cos(a), (float)std::sin(a));
+            t[k1 * R2 + b] = w;
+            t[n + b * R1 + k1] = w;
+        }
+}
+
+bool mesh_fft_supported(int64_t n0, int64_t n1, int64_t n2) {
+    for (int64_t n : {n0, n1, n2})
+        if (n != 64 && n != 96 && n != 128 && n != 192 && n != 256 && n != 384 && n != 512 &&
+            n != 768 && n != 1024)
+            return false;
+    return true;
+}
+
+int64_t mesh_fft_twiddles(int64_t n0, int64_t n1, int64_t n2, float2 *t) {
+    const int64_t L = n2 / 2;
+    if (t) {
+        mesh_axis_r(n0, [&](int R1, int R2) { axis_table(n0, R1, R2, t); });
+        mesh_axis_r(n1, [&](int R1, int R2) { axis_table(n1, R1, R2, t + 2 * n0); });
+        int R1 = 1, R2 = 1;
+        mesh_rows_factors(n2, &R1, &R2);
+        axis_table(L, R1, R2, t + 2 * n0 + 2 * n1);
+        float2 *s = t + 2 * n0 + 2 * n1 + 2 * L;
+        for (int64_t k = 0; k <= L; ++k) {
+            const double a = -2.0 * kPi * (double)k / (double)n2;
+            s[k] = make_float2((float)std::cos(a), (float)std::sin(a));
+        }
+    }
+    return 2 * n0 + 2 * n1 + 3 * L + 1;
+}
+
+}  // namespace pmx
