@@ -323,10 +323,22 @@ __global__ void k_poisson_adj(float2 *ck, int64_t n0, int64_t n1, int64_t n2h, i
 // particle kernels of the hot path (3-D, default enmesh branch)
 // ---------------------------------------------------------------------------
 
+// How a particle's two z neighbours are added to a mesh row.  DEP_V2 where
+// the mesh has at least four cells per particle (neighbouring lanes are then
+// about two cells apart): with an even lower index one 8-byte reduction covers
+// both, and clustered deposits take 0.54 instead of 0.64 ms (256^3 particles on
+// 512^3).  At one cell per particle the parity alternates from lane to lane, which
+// splits a warp's contiguous reductions (0.72 against 0.59 ms on 384^3):
+// there DEP_JOIN hands a lane's upper value to the next lane when that one's
+// lower cell is the same.  DEP_V4 (opt-in, PMX_WS_VEC): one 16-byte reduction
+// inside an aligned group of four floats, two of them zeros.
+enum Dep { DEP_SCALAR, DEP_V2, DEP_JOIN, DEP_V4 };
+
 struct Hot {
     int wrap[3];
     int64_t stride[3];
     float cell;   // f32(conf.cell_size), also the disp_cot divisor
+    float inv;    // 1 / cell where that is exact (cell a power of two), else 0
     float val;    // f32(mesh_size / ptcl_num)
     // component j of the acceleration meshes (and their cotangents) at cell
     // c with x index x lives at c + x*gxs + j*gjs: planar (0, M) or
@@ -336,33 +348,75 @@ struct Hot {
     float *dcomp, *vcomp;
     // deposit through per-warp shared-memory windows (needs n2 % 4 == 0)
     bool win;
-    // n2 % 4 == 0: every mesh row starts on 16 bytes, so z-neighbour pairs
-    // inside one aligned group of four floats take one vector reduction
-    bool vec;
+    // how z-neighbour pairs are deposited (enum Dep)
+    int dep;
     // warp-aggregated deposits (mesh indices below 2^32 - 32)
     bool agg;
     // per-block partial sums: slot s of block b at part[s * pstride + b]
     int64_t pstride;
 };
 
+// x / cell as IEEE division gives it: a multiplication where 1 / cell is exact.
+__device__ __forceinline__ float hot_div(const Hot &h, float x) {
+    return h.inv != 0.f ? __fmul_rn(x, h.inv) : __fdiv_rn(x, h.cell);
+}
+
+// i modulo n; positions within one period of the box, the usual ones, take an
+// addition instead of an integer division.
+__device__ __forceinline__ int hot_wrap(int i, int n) {
+    if ((unsigned)i < (unsigned)n) return i;
+    i += i < 0 ? n : -n;
+    return (unsigned)i < (unsigned)n ? i : pymod(i, n);
+}
+
+// Neighbours of one axis, as enmesh_axis (pm_util.py:119-149) computes them:
+// d2 = x - index is in [0, 1) for the lower and in [-1, 0) for the upper
+// neighbour, so sign(-d2) is -1 or -0 and 1 (NaN stays NaN).
 __device__ __forceinline__ void hot_axis(const Hot &h, int a, int pm, float d, Axis &ax) {
-    float x = __fdiv_rn(d, h.cell);
-    int fl = (int)floorf(x);
-#pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-        int ii = fl + nb;
-        float d2 = __fsub_rn(x, (float)ii);
-        ax.w[nb] = __fsub_rn(1.f, fabsf(d2));
-        ax.s[nb] = sgnf(-d2);
-        ax.i[nb] = pymod(ii + pm, h.wrap[a]);
-    }
+    const float x = hot_div(h, d);
+    const int fl = (int)floorf(x);
+    const float d0 = __fsub_rn(x, (float)fl), d1 = __fsub_rn(x, (float)(fl + 1));
+    ax.w[0] = __fsub_rn(1.f, fabsf(d0));
+    ax.w[1] = __fsub_rn(1.f, fabsf(d1));
+    ax.s[0] = d0 > 0.f ? -1.f : -d0;
+    ax.s[1] = d1 < 0.f ? 1.f : -d1;
     ax.u = fl + pm;
+    ax.i[0] = hot_wrap(ax.u, h.wrap[a]);
+    ax.i[1] = ax.i[0] + 1 == h.wrap[a] ? 0 : ax.i[0] + 1;
+}
+
+// Offset of neighbour (y bit, z bit) = (k >> 1) & 1, k >> 2 within an x-plane;
+// a plane has at most 2^32 cells (check_hot), so one 32-bit offset serves both
+// x-planes and every component.
+__device__ __forceinline__ unsigned hot_off(const Hot &h, const Axis ax[3], int k) {
+    return (unsigned)ax[1].i[(k >> 1) & 1] * (unsigned)h.stride[1] + (unsigned)ax[2].i[k >> 2];
 }
 
 __device__ __forceinline__ int64_t hot_cell(const Hot &h, const Axis ax[3], int k) {
-    return (int64_t)ax[0].i[k & 1] * h.stride[0] + (int64_t)ax[1].i[(k >> 1) & 1] * h.stride[1] +
-           (int64_t)ax[2].i[(k >> 2) & 1];
+    return ax[0].i[k & 1] * h.stride[0] + hot_off(h, ax, k);
 }
+
+// x-plane of neighbour bit b of a mesh whose planes are xs apart.
+template <typename T>
+__device__ __forceinline__ T *hot_plane(T *base, const Axis ax[3], int b, int64_t xs) {
+    return base + ax[0].i[b] * xs;
+}
+
+// The two x-planes of the three components of a plane-interleaved or planar
+// array of meshes (the accelerations or their cotangents).
+template <typename T>
+struct Planes3 {
+    T *p[3][2];
+    __device__ __forceinline__ Planes3(const Hot &h, T *base, const Axis ax[3]) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            T *x = hot_plane(base, ax, b, h.stride[0] + h.gxs);
+            p[0][b] = x;
+            p[1][b] = x + h.gjs;
+            p[2][b] = x + 2 * h.gjs;
+        }
+    }
+};
 
 __device__ __forceinline__ float3 ld3(const float *p, int64_t q) {
     return make_float3(p[3 * q], p[3 * q + 1], p[3 * q + 2]);
@@ -394,8 +448,21 @@ __device__ __forceinline__ float3 kahan_axpy(float3 y, float3 x, float a, float 
     return t;
 }
 
-__device__ __forceinline__ double dot3d(float3 a, float3 b) {
-    return (double)a.x * (double)b.x + (double)a.y * (double)b.y + (double)a.z * (double)b.z;
+// (double)x: the exponent rebiased and the mantissa shifted by integer
+// operations for normal numbers.  The float64 unit, which also converts, runs
+// at about two operations per clock and SM here: dot products of six
+// conversions and four operations held up the kick/drift adjoint passes (256^3
+// particles on 256^3: 0.68 against 0.63 ms with these three operations).
+__device__ __forceinline__ double to_f64(float x) {
+    const unsigned u = __float_as_uint(x), e = u & 0x7f800000u;
+    if (e == 0u || e == 0x7f800000u) return (double)x;   // zero, subnormal, inf, NaN
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)),
+                            (int)(u << 29));
+}
+
+// s + a . b
+__device__ __forceinline__ double dot3d(float3 a, float3 b, double s) {
+    return fma(to_f64(a.x), to_f64(b.x), fma(to_f64(a.y), to_f64(b.y), fma(to_f64(a.z), to_f64(b.z), s)));
 }
 
 __device__ __forceinline__ void hot_enmesh(const Hot &h, const int16_t *pmid, int64_t q, float3 d,
@@ -405,36 +472,172 @@ __device__ __forceinline__ void hot_enmesh(const Hot &h, const int16_t *pmid, in
     hot_axis(h, 2, pmid[3 * q + 2], d.z, ax[2]);
 }
 
+// The gathers walk the four (x, y) neighbour rows and read both z neighbours
+// of a row at once, interpolating along z first: the two values share a cache
+// line, which is gone again when the upper neighbours are read in a second
+// sweep (256^3 clustered particles on 512^3: 0.68 against 1.10 ms).  An
+// aligned 16-byte load that holds both is slower by far (1.08 against 0.44 ms
+// near the lattice): four times the bytes through L1.
+
+// a = acceleration at the particle.
+__device__ __forceinline__ float3 gather_acc(const Hot &h, const Axis ax[3], const float *g) {
+    const Planes3<const float> gp(h, g, ax);
+    float3 a = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const unsigned y = (unsigned)ax[1].i[p >> 1] * (unsigned)h.stride[1];
+        const unsigned o0 = y + (unsigned)ax[2].i[0], o1 = y + (unsigned)ax[2].i[1];
+        const float f = ax[0].w[p & 1] * ax[1].w[p >> 1];
+        float t[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            t[j] = fmaf(__ldg(gp.p[j][p & 1] + o1), ax[2].w[1],
+                        __ldg(gp.p[j][p & 1] + o0) * ax[2].w[0]);
+        a = make_float3(fmaf(f, t[0], a.x), fmaf(f, t[1], a.y), fmaf(f, t[2], a.z));
+    }
+    return a;
+}
+
+// The acceleration, and the gather VJP's position term before its division by
+// the cell size: c_a = sum_k (vc . m_k) dfrac_k / d(x_a / cell).
+__device__ __forceinline__ float3 gather_acc_vjp(const Hot &h, const Axis ax[3], const float *g,
+                                                 float3 vc, float3 &c) {
+    const Planes3<const float> gp(h, g, ax);
+    float3 a = make_float3(0.f, 0.f, 0.f);
+    c = a;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int bx = p & 1, by = p >> 1;
+        const unsigned y = (unsigned)ax[1].i[by] * (unsigned)h.stride[1];
+        const unsigned o0 = y + (unsigned)ax[2].i[0], o1 = y + (unsigned)ax[2].i[1];
+        float t[3], d[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const float m0 = __ldg(gp.p[j][bx] + o0), m1 = __ldg(gp.p[j][bx] + o1);
+            t[j] = fmaf(m1, ax[2].w[1], m0 * ax[2].w[0]);
+            d[j] = fmaf(m1, ax[2].s[1], m0 * ax[2].s[0]);
+        }
+        const float f = ax[0].w[bx] * ax[1].w[by];
+        a = make_float3(fmaf(f, t[0], a.x), fmaf(f, t[1], a.y), fmaf(f, t[2], a.z));
+        const float T = fmaf(vc.z, t[2], fmaf(vc.y, t[1], vc.x * t[0]));
+        const float D = fmaf(vc.z, d[2], fmaf(vc.y, d[1], vc.x * d[0]));
+        c = make_float3(fmaf(ax[0].s[bx] * ax[1].w[by], T, c.x),
+                        fmaf(ax[0].w[bx] * ax[1].s[by], T, c.y), fmaf(f, D, c.z));
+    }
+    return a;
+}
+
+// The scatter VJP's position term before its division by the cell size:
+// c_a = sum_k rho_cot_k val dfrac_k / d(x_a / cell).
+__device__ __forceinline__ float3 gather_grad(const Hot &h, const Axis ax[3],
+                                              const float *rho_cot) {
+    float3 c = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int bx = p & 1, by = p >> 1;
+        const float *r = hot_plane(rho_cot, ax, bx, h.stride[0]);
+        const unsigned y = (unsigned)ax[1].i[by] * (unsigned)h.stride[1];
+        const float m0 = __ldg(r + (y + (unsigned)ax[2].i[0])) * h.val;
+        const float m1 = __ldg(r + (y + (unsigned)ax[2].i[1])) * h.val;
+        const float T = fmaf(m1, ax[2].w[1], m0 * ax[2].w[0]);
+        const float D = fmaf(m1, ax[2].s[1], m0 * ax[2].s[0]);
+        c = make_float3(fmaf(ax[0].s[bx] * ax[1].w[by], T, c.x),
+                        fmaf(ax[0].w[bx] * ax[1].s[by], T, c.y),
+                        fmaf(ax[0].w[bx] * ax[1].w[by], D, c.z));
+    }
+    return c;
+}
+
 // Adds a at z index i0 and b at z index i1 (a particle's two z neighbours)
-// of one mesh row: one 16-byte red.global.add.v4.f32 (the other two lanes
-// add zero) when both cells lie in the same aligned group of four floats,
-// else two scalar atomics.  3 of 4 lower-neighbour positions qualify.
-__device__ __forceinline__ void zpair_add(float *row, int i0, int i1, float a, float b, bool vec) {
+// of the mesh row at offset y of a plane, as dep says.  Rows start on 16 bytes
+// for DEP_V4 (n2 % 4 == 0; 3 of 4 lower positions qualify), on 8 for DEP_V2.
+__device__ __forceinline__ void zpair_add(float *plane, unsigned y, int i0, int i1, float a, float b,
+                                          int dep) {
     const int r = i0 & 3;
-    if (vec && i1 == i0 + 1 && r != 3) {
+    if (dep == DEP_V4 && i1 == i0 + 1 && r != 3) {
         const float4 v = make_float4(r == 0 ? a : 0.f, r == 0 ? b : (r == 1 ? a : 0.f),
                                      r == 1 ? b : (r == 2 ? a : 0.f), r == 2 ? b : 0.f);
-        atomicAdd(reinterpret_cast<float4 *>(row + (i0 - r)), v);
+        atomicAdd(reinterpret_cast<float4 *>(plane + (y + (unsigned)(i0 - r))), v);
+    } else if (dep == DEP_V2 && (i0 & 1) == 0) {
+        atomicAdd(reinterpret_cast<float2 *>(plane + (y + (unsigned)i0)), make_float2(a, b));
     } else {
-        atomicAdd(row + i0, a);
-        atomicAdd(row + i1, b);
+        atomicAdd(plane + (y + (unsigned)i0), a);
+        atomicAdd(plane + (y + (unsigned)i1), b);
     }
 }
 
 // Offset of the (x, y) mesh row of neighbour pair p (bit 0: x, bit 1: y).
 __device__ __forceinline__ int64_t hot_row(const Hot &h, const Axis ax[3], int p) {
-    return (int64_t)ax[0].i[p & 1] * h.stride[0] + (int64_t)ax[1].i[(p >> 1) & 1] * h.stride[1];
+    return ax[0].i[p & 1] * h.stride[0] + (unsigned)ax[1].i[(p >> 1) & 1] * (unsigned)h.stride[1];
 }
 
-// CIC deposit of val * frac_k, frac_k = (w_x w_y) w_z as frac_of.
-__device__ __forceinline__ void hot_deposit(const Hot &h, const Axis ax[3], float *dens) {
+// Adds v[c] * frac_k, frac_k = (w_x w_y) w_z as frac_of, to component c of the
+// particle's eight neighbours; pl[c][b] is the x-plane of neighbour bit b.
+template <int NC>
+__device__ __forceinline__ void hot_add1(const Hot &h, const Axis ax[3], const float (&v)[NC],
+                                         float *const (&pl)[NC][2]) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-        const float fxy = __fmul_rn(ax[0].w[p & 1], ax[1].w[(p >> 1) & 1]);
-        zpair_add(dens + hot_row(h, ax, p), ax[2].i[0], ax[2].i[1],
-                  __fmul_rn(h.val, __fmul_rn(fxy, ax[2].w[0])),
-                  __fmul_rn(h.val, __fmul_rn(fxy, ax[2].w[1])), h.vec);
+        const float fxy = __fmul_rn(ax[0].w[p & 1], ax[1].w[p >> 1]);
+        const float fa = __fmul_rn(fxy, ax[2].w[0]), fb = __fmul_rn(fxy, ax[2].w[1]);
+        const unsigned y = (unsigned)ax[1].i[p >> 1] * (unsigned)h.stride[1];
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            zpair_add(pl[c][p & 1], y, ax[2].i[0], ax[2].i[1], __fmul_rn(v[c], fa),
+                      __fmul_rn(v[c], fb), h.dep);
     }
+}
+
+// The same by a whole warp (every lane calls it; inactive ones add nothing),
+// with DEP_JOIN.
+template <int NC>
+__device__ __forceinline__ void hot_add(const Hot &h, bool act, const Axis ax[3],
+                                        const float (&v)[NC], float *const (&pl)[NC][2]) {
+    const int i0 = ax[2].i[0], i1 = ax[2].i[1];
+    if (h.dep != DEP_JOIN) {
+        if (act) hot_add1<NC>(h, ax, v, pl);
+        return;
+    }
+    // join: the previous lane's upper cells are this lane's lower ones
+    const int lane = threadIdx.x & 31;
+    const unsigned o = act ? (unsigned)ax[1].i[0] * (unsigned)h.stride[1] + (unsigned)i0 : 0u;
+    const int x = act ? ax[0].i[0] : -1;
+    const unsigned po = __shfl_up_sync(0xffffffffu, o, 1);
+    const int px = __shfl_up_sync(0xffffffffu, x, 1);
+    const bool join = act && lane > 0 && px == x && po + 1 == o && i0 != 0;
+    const bool next = (__ballot_sync(0xffffffffu, join) >> lane >> 1) & 1;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const float fxy = __fmul_rn(ax[0].w[p & 1], ax[1].w[p >> 1]);
+        const float fa = __fmul_rn(fxy, ax[2].w[0]), fb = __fmul_rn(fxy, ax[2].w[1]);
+        const unsigned y = (unsigned)ax[1].i[p >> 1] * (unsigned)h.stride[1];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            float a = __fmul_rn(v[c], fa);
+            const float b = __fmul_rn(v[c], fb);
+            const float pb = __shfl_up_sync(0xffffffffu, b, 1);
+            if (join) a += pb;
+            if (act) {
+                atomicAdd(pl[c][p & 1] + (y + (unsigned)i0), a);
+                if (!next) atomicAdd(pl[c][p & 1] + (y + (unsigned)i1), b);
+            }
+        }
+    }
+}
+
+// CIC deposit of the density (val * frac_k) by one lane; by a whole warp.  The
+// joined passes of multi-step runs (k_gk_kds, k_sa_ka) use the former: a
+// warp-uniform loop for DEP_JOIN costs them more than it saves (384^3, 1.18
+// against 1.12 ms).
+__device__ __forceinline__ void hot_deposit1(const Hot &h, const Axis ax[3], float *dens) {
+    const float v[1] = {h.val};
+    float *const pl[1][2] = {{hot_plane(dens, ax, 0, h.stride[0]), hot_plane(dens, ax, 1, h.stride[0])}};
+    hot_add1<1>(h, ax, v, pl);
+}
+__device__ __forceinline__ void hot_deposit(const Hot &h, bool act, const Axis ax[3], float *dens) {
+    const float v[1] = {h.val};
+    float *const pl[1][2] = {{hot_plane(dens, ax, 0, h.stride[0]), hot_plane(dens, ax, 1, h.stride[0])}};
+    hot_add<1>(h, act, ax, v, pl);
 }
 
 // ---------------------------------------------------------------------------
@@ -475,8 +678,8 @@ __device__ __forceinline__ void agg_deposit(const Hot &h, bool act, const Axis a
                 float *row = base + hot_row(h, ax, p) + (int64_t)ax[0].i[p & 1] * xs;
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
-                    zpair_add(row + c * cs, ax[2].i[0], ax[2].i[1], __fmul_rn(s[c], fa),
-                              __fmul_rn(s[c], fb), h.vec);
+                    zpair_add(row + c * cs, 0u, ax[2].i[0], ax[2].i[1], __fmul_rn(s[c], fa),
+                              __fmul_rn(s[c], fb), h.dep);
             }
         }
         return;
@@ -503,7 +706,7 @@ __device__ __forceinline__ void agg_deposit(const Hot &h, bool act, const Axis a
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 float *a = slot + (2 * p) * NC + c, *b = slot + (2 * p + 1) * NC + c;
-                zpair_add(row + c * cs, ax[2].i[0], ax[2].i[1], *a, *b, h.vec);
+                zpair_add(row + c * cs, 0u, ax[2].i[0], ax[2].i[1], *a, *b, h.dep);
                 *a = 0.f;
                 *b = 0.f;
             }
@@ -641,7 +844,7 @@ __device__ __forceinline__ void kds_body(Hot h, const int16_t *__restrict__ pmid
          q0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = q0 + lane;
         const bool act = q < n;
-        Axis ax[3];
+        Axis ax[3] = {};
         if (act) {
             float3 d = ld3(disp, q);
             if (KD) {
@@ -658,7 +861,7 @@ __device__ __forceinline__ void kds_body(Hot h, const int16_t *__restrict__ pmid
             continue;
         }
         if (!WIN) {
-            if (act) hot_deposit(h, ax, dens);
+            hot_deposit(h, act, ax, dens);
             continue;
         }
         const Win w = win_origin(act, ax);
@@ -776,29 +979,23 @@ __global__ void __launch_bounds__(PT) k_gather3_tma(Hot h, const __grid_constant
             }
         }
         if (act) {
-            float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+            float3 a;
+            if (staged) {   // the products of gather_acc, in its order
+                a = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float f = frac_of(ax, k);
-                float m0, m1, m2;
-                if (staged) {
-                    const int xi = ax[0].u + (k & 1) - x0, yi = ax[1].u + ((k >> 1) & 1) - y0;
-                    const int zi = ax[2].u + ((k >> 2) & 1) - z0;
-                    const float *b = box + ((xi * 3) * TBY + yi) * TBZ + zi;
-                    m0 = b[0];
-                    m1 = b[TBY * TBZ];
-                    m2 = b[2 * TBY * TBZ];
-                } else {
-                    const float *gc = g + hot_cell(h, ax, k) + (int64_t)ax[0].i[k & 1] * h.gxs;
-                    m0 = __ldg(gc);
-                    m1 = __ldg(gc + h.gjs);
-                    m2 = __ldg(gc + 2 * h.gjs);
+                for (int p = 0; p < 4; ++p) {
+                    const int xi = ax[0].u + (p & 1) - x0, yi = ax[1].u + (p >> 1) - y0;
+                    const float *b = box + ((xi * 3) * TBY + yi) * TBZ + (ax[2].u - z0);
+                    const float f = ax[0].w[p & 1] * ax[1].w[p >> 1];
+                    float t[3];
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                        t[j] = fmaf(b[j * TBY * TBZ + 1], ax[2].w[1], b[j * TBY * TBZ] * ax[2].w[0]);
+                    a = make_float3(fmaf(f, t[0], a.x), fmaf(f, t[1], a.y), fmaf(f, t[2], a.z));
                 }
-                a0 = __fadd_rn(a0, __fmul_rn(m0, f));
-                a1 = __fadd_rn(a1, __fmul_rn(m1, f));
-                a2 = __fadd_rn(a2, __fmul_rn(m2, f));
+            } else {
+                a = gather_acc(h, ax, g);
             }
-            float3 a = make_float3(a0, a1, a2);
             st3(acc, q, a);
             if (KICK) st3(vel, q, axpy3(ld3(vel, q), a, K2));
         }
@@ -816,17 +1013,7 @@ __device__ __forceinline__ void gather3_body(Hot h, const int16_t *__restrict__ 
          q += (int64_t)gridDim.x * blockDim.x) {
         Axis ax[3];
         hot_enmesh(h, pmid, q, ld3(disp, q), ax);
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            int64_t c = hot_cell(h, ax, k);
-            float f = frac_of(ax, k);
-            const float *gc = g + c + (int64_t)ax[0].i[k & 1] * h.gxs;
-            a0 = __fadd_rn(a0, __fmul_rn(__ldg(gc), f));
-            a1 = __fadd_rn(a1, __fmul_rn(__ldg(gc + h.gjs), f));
-            a2 = __fadd_rn(a2, __fmul_rn(__ldg(gc + 2 * h.gjs), f));
-        }
-        float3 a = make_float3(a0, a1, a2);
+        const float3 a = gather_acc(h, ax, g);
         st3(acc, q, a);
         if (KICK) st3(vel, q, kahan_axpy(ld3(vel, q), a, K2, KAHAN ? h.vcomp : nullptr, q));
     }
@@ -863,7 +1050,7 @@ __device__ __forceinline__ void ka_body(Hot h, const int16_t *__restrict__ pmid,
          q0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = q0 + lane;
         const bool act = q < n;
-        Axis ax[3];
+        Axis ax[3] = {};
         if (act) {
             float3 d = ld3(disp, q);
             if (KD) {
@@ -871,10 +1058,10 @@ __device__ __forceinline__ void ka_body(Hot h, const int16_t *__restrict__ pmid,
                 float3 vc = ld3(vel_cot, q);
                 float3 v = kahan_axpy(ld3(vel, q), a, K1, vcomp, q);
                 float3 dc = axmy3(ld3(disp_cot, q), ld3(alpha, q), K1);
-                s0 += dot3d(vc, a);
+                s0 = dot3d(vc, a, s0);
                 d = kahan_axpy(d, v, D, dcomp, q);
                 vc = axmy3(vc, dc, D);
-                s1 += dot3d(dc, v);
+                s1 = dot3d(dc, v, s1);
                 st3(vel, q, v);
                 st3(disp, q, d);
                 st3(disp_cot, q, dc);
@@ -888,7 +1075,7 @@ __device__ __forceinline__ void ka_body(Hot h, const int16_t *__restrict__ pmid,
             continue;
         }
         if (!WIN) {
-            if (act) hot_deposit(h, ax, dens);
+            hot_deposit(h, act, ax, dens);
             continue;
         }
         const Win w = win_origin(act, ax);
@@ -945,56 +1132,29 @@ __device__ __forceinline__ void g3adj_body(Hot h, const int16_t *__restrict__ pm
          q0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = q0 + lane;
         const bool act = q < n;
-        Axis ax[3];
+        Axis ax[3] = {};
         float3 vc = make_float3(0.f, 0.f, 0.f);
         if (act) {
             hot_enmesh(h, pmid, q, ld3(disp, q), ax);
             vc = ld3(vel_cot, q);
-            float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-            float c0 = 0.f, c1 = 0.f, c2 = 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                int64_t c = hot_cell(h, ax, k);
-                float f = frac_of(ax, k);
-                float fg[3];
-                frac_grad_of(ax, k, fg);
-                const int64_t gc = c + (int64_t)ax[0].i[k & 1] * h.gxs;
-                float m0 = __ldg(g + gc), m1 = __ldg(g + gc + h.gjs), m2 = __ldg(g + gc + 2 * h.gjs);
-                a0 = __fadd_rn(a0, __fmul_rn(m0, f));
-                a1 = __fadd_rn(a1, __fmul_rn(m1, f));
-                a2 = __fadd_rn(a2, __fmul_rn(m2, f));
-                float t = __fadd_rn(__fadd_rn(__fmul_rn(vc.x, m0), __fmul_rn(vc.y, m1)),
-                                    __fmul_rn(vc.z, m2));
-                c0 = __fadd_rn(c0, __fmul_rn(t, fg[0]));
-                c1 = __fadd_rn(c1, __fmul_rn(t, fg[1]));
-                c2 = __fadd_rn(c2, __fmul_rn(t, fg[2]));
-            }
-            if (!WIN && !AGG) {
-                // gather-VJP mesh term mcot_j[k] += vc_j frac_k
-#pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const float fxy = __fmul_rn(ax[0].w[p & 1], ax[1].w[(p >> 1) & 1]);
-                    const float fa = __fmul_rn(fxy, ax[2].w[0]), fb = __fmul_rn(fxy, ax[2].w[1]);
-                    float *row = mcot + hot_row(h, ax, p) + (int64_t)ax[0].i[p & 1] * h.gxs;
-                    const int i0 = ax[2].i[0], i1 = ax[2].i[1];
-                    zpair_add(row, i0, i1, __fmul_rn(vc.x, fa), __fmul_rn(vc.x, fb), h.vec);
-                    zpair_add(row + h.gjs, i0, i1, __fmul_rn(vc.y, fa), __fmul_rn(vc.y, fb), h.vec);
-                    zpair_add(row + 2 * h.gjs, i0, i1, __fmul_rn(vc.z, fa), __fmul_rn(vc.z, fb),
-                              h.vec);
-                }
-            }
-            float3 a = make_float3(a0, a1, a2);
+            float3 c;
+            const float3 a = gather_acc_vjp(h, ax, g, vc, c);
             st3(acc, q, a);
-            st3(alpha, q, make_float3(__fdiv_rn(c0, h.cell), __fdiv_rn(c1, h.cell),
-                                      __fdiv_rn(c2, h.cell)));
-            s2 += dot3d(vc, a);
+            st3(alpha, q, make_float3(hot_div(h, c.x), hot_div(h, c.y), hot_div(h, c.z)));
+            s2 = dot3d(vc, a, s2);
         }
         if constexpr (AGG) {
             const float sv[3] = {vc.x, vc.y, vc.z};
             agg_deposit<3>(h, act, ax, sv, mcot, h.gxs, h.gjs, abuf);
             continue;
         }
-        if (!WIN) continue;
+        if (!WIN) {
+            // gather-VJP mesh term mcot_j[k] += vc_j frac_k
+            const float v[3] = {vc.x, vc.y, vc.z};
+            const Planes3<float> mp(h, mcot, ax);
+            hot_add<3>(h, act, ax, v, mp.p);
+            continue;
+        }
         // gather-VJP mesh term through the warp window, three components
         const Win w = win_origin(act, ax);
         if (act) {
@@ -1016,7 +1176,7 @@ __device__ __forceinline__ void g3adj_body(Hot h, const int16_t *__restrict__ pm
 }
 
 template <bool WIN, bool AGG = false>
-__global__ void __launch_bounds__(PT) k_g3adj(Hot h, const int16_t *__restrict__ pmid,
+__global__ void __launch_bounds__(PT, 4) k_g3adj(Hot h, const int16_t *__restrict__ pmid,
                                               const float *__restrict__ disp,
                                               const float *__restrict__ vel_cot, float *acc,
                                               float *alpha, int64_t n, int64_t M,
@@ -1038,21 +1198,10 @@ __device__ __forceinline__ void sadj_body(Hot h, const int16_t *__restrict__ pmi
          q += (int64_t)gridDim.x * blockDim.x) {
         Axis ax[3];
         hot_enmesh(h, pmid, q, ld3(disp, q), ax);
-        float c0 = 0.f, c1 = 0.f, c2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            int64_t c = hot_cell(h, ax, k);
-            float fg[3];
-            frac_grad_of(ax, k, fg);
-            float t = __fmul_rn(__ldg(rho_cot + c), h.val);
-            c0 = __fadd_rn(c0, __fmul_rn(t, fg[0]));
-            c1 = __fadd_rn(c1, __fmul_rn(t, fg[1]));
-            c2 = __fadd_rn(c2, __fmul_rn(t, fg[2]));
-        }
+        const float3 c = gather_grad(h, ax, rho_cot);
         float3 al = ld3(alpha, q);
-        al = make_float3(__fadd_rn(al.x, __fdiv_rn(c0, h.cell)),
-                         __fadd_rn(al.y, __fdiv_rn(c1, h.cell)),
-                         __fadd_rn(al.z, __fdiv_rn(c2, h.cell)));
+        al = make_float3(__fadd_rn(al.x, hot_div(h, c.x)), __fadd_rn(al.y, hot_div(h, c.y)),
+                         __fadd_rn(al.z, hot_div(h, c.z)));
         st3(alpha, q, al);
         if (KICK) {
             st3(vel, q, kahan_axpy(ld3(vel, q), ld3(acc, q), K2, KAHAN ? h.vcomp : nullptr, q));
@@ -1089,17 +1238,7 @@ __device__ __forceinline__ void gk_kds_particle(const Hot &h, const int16_t *__r
     {
         float3 d = ld3(disp, q);
         hot_enmesh(h, pmid, q, d, ax);
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            int64_t c = hot_cell(h, ax, k);
-            float f = frac_of(ax, k);
-            const float *gc = g + c + (int64_t)ax[0].i[k & 1] * h.gxs;
-            a0 = __fadd_rn(a0, __fmul_rn(__ldg(gc), f));
-            a1 = __fadd_rn(a1, __fmul_rn(__ldg(gc + h.gjs), f));
-            a2 = __fadd_rn(a2, __fmul_rn(__ldg(gc + 2 * h.gjs), f));
-        }
-        const float3 a = make_float3(a0, a1, a2);
+        const float3 a = gather_acc(h, ax, g);
         float3 v = axpy3(ld3(vel, q), a, K2);   // kick, step i
         v = axpy3(v, a, K1n);                   // kick, step i+1
         d = axpy3(d, v, Dn);                    // drift, step i+1
@@ -1118,7 +1257,7 @@ __device__ __forceinline__ void gk_kds_body(Hot h, const int16_t *__restrict__ p
              q += (int64_t)gridDim.x * blockDim.x) {
             Axis ax[3];
             gk_kds_particle(h, pmid, disp, vel, g, K2, K1n, Dn, q, ax);
-            hot_deposit(h, ax, dens);
+            hot_deposit1(h, ax, dens);
         }
     } else {
         float *abuf = agg_buffer<1>();
@@ -1155,31 +1294,20 @@ __device__ __forceinline__ void sa_ka_particle(const Hot &h, const int16_t *__re
     {
         float3 d = ld3(disp, q);
         hot_enmesh(h, pmid, q, d, ax);
-        float c0 = 0.f, c1 = 0.f, c2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            int64_t c = hot_cell(h, ax, k);
-            float fg[3];
-            frac_grad_of(ax, k, fg);
-            float t = __fmul_rn(__ldg(rho_cot + c), h.val);
-            c0 = __fadd_rn(c0, __fmul_rn(t, fg[0]));
-            c1 = __fadd_rn(c1, __fmul_rn(t, fg[1]));
-            c2 = __fadd_rn(c2, __fmul_rn(t, fg[2]));
-        }
+        const float3 c = gather_grad(h, ax, rho_cot);
         float3 al = ld3(alpha, q);
-        al = make_float3(__fadd_rn(al.x, __fdiv_rn(c0, h.cell)),
-                         __fadd_rn(al.y, __fdiv_rn(c1, h.cell)),
-                         __fadd_rn(al.z, __fdiv_rn(c2, h.cell)));
+        al = make_float3(__fadd_rn(al.x, hot_div(h, c.x)), __fadd_rn(al.y, hot_div(h, c.y)),
+                         __fadd_rn(al.z, hot_div(h, c.z)));
         const float3 a = ld3(acc, q);
         float3 v = axpy3(ld3(vel, q), a, K2);            // kick_adj, step i
         float3 dc = axmy3(ld3(disp_cot, q), al, K2);
         float3 vc = ld3(vel_cot, q);
         v = axpy3(v, a, K1n);                            // kick_adj, step i+1
         dc = axmy3(dc, al, K1n);
-        s0 += dot3d(vc, a);
+        s0 = dot3d(vc, a, s0);
         d = axpy3(d, v, Dn);                             // drift_adj, step i+1
         vc = axmy3(vc, dc, Dn);
-        s1 += dot3d(dc, v);
+        s1 = dot3d(dc, v, s1);
         st3(vel, q, v);
         st3(disp, q, d);
         st3(disp_cot, q, dc);
@@ -1204,7 +1332,7 @@ __device__ __forceinline__ void sa_ka_body(Hot h, const int16_t *__restrict__ pm
             Axis ax[3];
             sa_ka_particle(h, pmid, disp, vel, acc, disp_cot, vel_cot, alpha, rho_cot, K2, K1n,
                            Dn, q, ax, s0, s1);
-            hot_deposit(h, ax, dens);
+            hot_deposit1(h, ax, dens);
         }
     } else {
         float *abuf = agg_buffer<1>();
@@ -1517,6 +1645,12 @@ int device_scratch(double **out) {
     } while (0)
 #define PMX_UNPAREN(...) __VA_ARGS__
 
+// The rule of enum Dep: n particles on the workspace's mesh.
+int deposit_mode(const pmx_workspace *ws, int64_t n) {
+    if (ws->M < 4 * n) return DEP_JOIN;
+    return ws->n2 % 2 == 0 ? DEP_V2 : DEP_SCALAR;
+}
+
 int check_hot(pmx_workspace *ws, const pmx_enmesh_spec *spec, const void *pmid, const void *disp,
               int64_t n, int64_t ptcl_num, Hot *h) {
     if (!ws) return fail(PMX_ERR_ARG, "null workspace");
@@ -1528,6 +1662,8 @@ int check_hot(pmx_workspace *ws, const pmx_enmesh_spec *spec, const void *pmid, 
         spec->wrap_shape[0] != ws->n0 || spec->wrap_shape[1] != ws->n1 || spec->wrap_shape[2] != ws->n2)
         return fail(PMX_ERR_SHAPE, "mesh shape differs from the workspace's");
     if (!(spec->conf_cell_size > 0)) return fail(PMX_ERR_ARG, "conf_cell_size must be > 0");
+    if (ws->n1 * ws->n2 > (int64_t)1 << 32)   // hot_off; int16 pmid reaches sides of 2^15
+        return fail(PMX_ERR_SHAPE, "the force path takes planes of up to 2^32 cells");
     if (n < 0 || ptcl_num <= 0) return fail(PMX_ERR_ARG, "bad particle counts");
     if (n > 0 && (!pmid || !disp)) return fail(PMX_ERR_ARG, "null pmid/disp");
     int dev = 0;
@@ -1538,13 +1674,13 @@ int check_hot(pmx_workspace *ws, const pmx_enmesh_spec *spec, const void *pmid, 
     h->stride[1] = ws->n2;
     h->stride[0] = ws->n1 * ws->n2;
     h->cell = (float)spec->conf_cell_size;
+    int e2 = 0;
+    h->inv = std::frexp(h->cell, &e2) == 0.5f && e2 > -126 && e2 < 126 ? 1.f / h->cell : 0.f;
     h->val = (float)((double)ws->M / (double)ptcl_num);
     h->dcomp = nullptr;
     h->vcomp = nullptr;
     h->win = ws->win;
-    // measured slower on GB300 (the v4 reductions with two zero lanes cost
-    // more than the scalar atomics they replace): opt-in, PMX_WS_VEC
-    h->vec = ws->vec;
+    h->dep = ws->vec ? DEP_V4 : deposit_mode(ws, n);
     h->agg = ws->agg;
     h->pstride = ws->pstride;
     if (ws->xfast) {
