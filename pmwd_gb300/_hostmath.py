@@ -2,8 +2,9 @@
 
 The initial-condition path evaluates a few hundred scalars per call: the
 linear power spectrum on the table of distinct |k| (modes.py:67-117 via
-boltzmann.py:399-455) and the growth factors at a_start (lpt.py:197-210).
-As torch CPU tensors these are ~10^2 dispatched ops (about a millisecond);
+boltzmann.py:399-455) and the growth factors at a_start (lpt.py:197-210); an
+N-body run the drift and kick factors of its steps (nbody.py:12-36).
+As torch CPU tensors these are ~10^2 dispatched ops (one to three milliseconds);
 when nothing needs a gradient they are evaluated here in NumPy with the
 same formulas and the same order of operations as the torch code in
 ``boltzmann`` and ``cosmology``, so both give the same float32 results.
@@ -61,6 +62,67 @@ def E2(a, cosmo):
     Ode = 1 - (Om + Ok)
     de_a = a ** (-3 * (1 + w0 + wa)) * math.exp(-3 * wa * (1 - a))
     return Om * a ** -3 + Ok * a ** -2 + Ode * de_a
+
+
+class _Background:
+    """The growth factors of nbody.py:12-22 at an array of scale factors; the
+    interpolation's intervals and the expansion rate are worked out once."""
+
+    def __init__(self, a, xp, tab, cosmo):
+        self.a, self.tab = a, tab[0]
+        self.i = np.clip(np.searchsorted(xp, a, side='right'), 1, len(xp) - 1)
+        lo = xp[self.i - 1]
+        dx = xp[self.i] - lo
+        self.r = (a - lo) / np.where(dx == 0, 1, dx)
+        self.flat = dx == 0
+        self.below, self.above = a < xp[0], a > xp[-1]
+        self.edges = bool((self.flat | self.below | self.above).any())
+        self.Om, self.Ok = _f(cosmo.Omega_m), _f(cosmo.Omega_k)
+        self.Ode = 1 - (self.Om + self.Ok)
+        w0, wa = _f(cosmo.w_0), _f(cosmo.w_a)
+        self.p, self.q = -3 * (1 + w0 + wa), -3 * wa
+        self.de_a = a ** self.p * np.exp(self.q * (1 - a))
+        self.E2 = self.Om * a ** -3 + self.Ok * a ** -2 + self.Ode * self.de_a
+
+    def growth(self, deriv=0):
+        fp = self.tab[deriv]
+        hi, lo = fp[self.i], fp[self.i - 1]
+        f = lo + self.r * (hi - lo)
+        if self.edges:   # as interp
+            f = np.where(self.flat, hi, f)
+            f = np.where(self.below, fp[0], f)
+            f = np.where(self.above, fp[-1], f)
+        return self.a * f
+
+    def G_D(self):
+        return self.a ** 2 * np.sqrt(self.E2) * self.growth(1)
+
+    def G_K(self):
+        a = self.a
+        H_deriv = 0.5 * (-3 * self.Om * a ** -3 - 2 * self.Ok * a ** -2
+                         + self.Ode * self.de_a * (self.p - self.q * a)) / self.E2
+        return a ** 3 * self.E2 * (self.growth(2) + (2 + H_deriv) * self.growth(1))
+
+
+def op_factors(ops, cosmo, conf):
+    """nbody.op_factors as a float64 NumPy array: the drift_factor or
+    kick_factor (nbody.py:25-36) of every drift and kick, in op order."""
+    if cosmo.growth is None:
+        raise ValueError('Growth table is empty. Call growth_integ or boltzmann first.')
+    xp = np.concatenate((conf.a_lpt.numpy(), conf.a_nbody.numpy()[1:]))   # conf.growth_a
+    tab = cosmo.growth.detach().cpu().numpy()
+    ops = [o for o in ops if len(o) == 4]
+    kick = np.array([o[0].startswith('kick') for o in ops], dtype=bool)
+    args = np.array([o[1:] for o in ops], dtype=np.float64).reshape(-1, 3)
+    num = int(kick.sum())
+    out = np.empty(len(kick))
+    k, d = args[kick], args[~kick]
+    # kicks: the velocities' G_D at both ends, over G_K of the accelerations
+    GD = _Background(np.concatenate((k[:, 2], k[:, 1], d[:, 0])), xp, tab, cosmo).G_D()
+    out[kick] = (GD[:num] - GD[num:2 * num]) / _Background(k[:, 0], xp, tab, cosmo).G_K()
+    D = _Background(np.concatenate((d[:, 2], d[:, 1])), xp, tab, cosmo).growth()
+    out[~kick] = (D[:len(d)] - D[len(d):]) / GD[2 * num:]
+    return out
 
 
 def lpt_factors(cosmo, conf):

@@ -25,7 +25,7 @@ import ctypes
 import numpy as np
 import torch
 
-from . import _lib
+from . import _hostmath, _lib
 from .boltzmann import growth
 from .cosmology import E2, H_deriv
 
@@ -295,8 +295,17 @@ def nbody(ptcl, obsvbl, cosmo, conf, reverse=False):
     Om = cosmo.Omega_m
     if not torch.is_tensor(Om):
         Om = torch.tensor(float(Om), dtype=torch.float64)
-    fwd = op_factors(forward_ops(conf, reverse), cosmo, conf)
-    adj = op_factors(adjoint_ops(conf, reverse), cosmo, conf)
+    fops, aops = forward_ops(conf, reverse), adjoint_ops(conf, reverse)
+    if _hostmath.needs_grad(cosmo):
+        fwd, adj = op_factors(fops, cosmo, conf), op_factors(aops, cosmo, conf)
+    else:
+        # NumPy, and the adjoint's factors only for a run that will have one:
+        # 16 steps took 2.9 ms of torch CPU operations, longer than the steps
+        # themselves on a 128^3 mesh
+        fwd = torch.from_numpy(_hostmath.op_factors(fops, cosmo, conf))
+        adj = torch.zeros(0, dtype=torch.float64)
+        if torch.is_grad_enabled() and (ptcl.disp.requires_grad or ptcl.vel.requires_grad):
+            adj = torch.from_numpy(_hostmath.op_factors(aops, cosmo, conf))
     disp, vel, acc = _NbodyFn.apply(ptcl.disp, ptcl.vel, fwd, adj, Om, ptcl.pmid.contiguous(),
                                     conf, reverse)
     return ptcl.replace(disp=disp, vel=vel, acc=acc), obsvbl
