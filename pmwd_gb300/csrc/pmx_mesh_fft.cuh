@@ -22,10 +22,10 @@
 // At N = 1024 a block of 128 threads holds 4 columns (34 KB), so several
 // blocks share an SM and one's loads overlap another's arithmetic.
 //
-// Measured at 1024^3 (GB300, ms): rows r2c 1.43, cols fwd 1.50, x fwd 4.2,
-// cols inv3 5.35, rows c2r 3 x 1.30; adjoint rows 4.27, cols 5.85, x 4.1,
-// cols inv1 1.88, rows 1.30.  The cuFFT plane transforms and the tiled x pass
-// that they replace: r2c 3.4, x 6.8, c2r 11.1; adjoint 10.1, 8.5, 3.7.
+// Measured at 1024^3 (GB300, ms): rows r2c 1.43, cols fwd 1.51, x fwd 3.88,
+// cols inv 4.80, rows c2r 3 x 1.30; adjoint rows 4.28, cols 5.68, x 3.75, cols
+// inv 1.68, rows 1.30.  The cuFFT plane transforms and the tiled x pass that
+// they replace: r2c 3.4, x 6.8, c2r 11.1; adjoint 10.1, 8.5, 3.7.
 //
 // Layouts.  Strided axes make the memory system, not the arithmetic, the
 // bound: at 1024^3 an x-axis column in a natural (x, ky, kz) array is read in
@@ -61,16 +61,30 @@ template <> struct Fac<512> { static constexpr int R1 = 32, R2 = 16; };
 template <> struct Fac<768> { static constexpr int R1 = 24, R2 = 32; };
 template <> struct Fac<1024> { static constexpr int R1 = 32, R2 = 32; };
 
-template <int N>
-struct ColCfg {
+// Block of T columns of length N: T * R2 threads, one radix-R1 DFT each in the
+// first stage.
+template <int N_, int T_>
+struct TileCfg {
+    static constexpr int N = N_, T = T_;
     static constexpr int R1 = Fac<N>::R1, R2 = Fac<N>::R2;
-    static constexpr int T = 128 / R2 < 4 ? 4 : 128 / R2;   // columns per block
-    static constexpr int TH = T * R2;                       // stage 1: one radix-R1 DFT per thread
+    static constexpr int TH = T * R2;
     // shared exchange buffer: element (k1, b) of column t at k1 * GS + b * T + t;
     // R2 + 1 odd keeps both sides free of bank conflicts
     static constexpr int GS = (R2 + 1) * T;
     static constexpr int BUF = R1 * GS;
 };
+
+// x axis: T consecutive kz of one ky (whole spec blocks of 4 kz).
+template <int N>
+using XCol = TileCfg<N, 128 / Fac<N>::R2 < 4 ? 4 : 128 / Fac<N>::R2>;
+
+// y axis: XP = T / 4 consecutive x-planes times 4 kz, so that a block touches
+// XP * 32 contiguous bytes of a spec block at a time.  Larger XP (256-thread
+// blocks) makes wider pieces but lost to the 128-thread blocks' finer overlap of
+// loads and arithmetic: 5.1 against 4.8 ms for the three inverse transforms at
+// 1024^3, 0.55 against 0.50 at 512^3.
+template <int N>
+using YCol = XCol<N>;
 
 // Twiddle tables of a length-N transform (float2): w^(b k1) at k1 * R2 + b,
 // then the same at b * R1 + k1 (w = exp(-2 pi i / N)).
@@ -100,12 +114,42 @@ __device__ __forceinline__ int64_t spec_at(const MeshGeom &g, int64_t x, int ky,
 }
 
 
+// Table loads in program order.  Left alone, the compiler hoists all of a
+// thread's table loads to the front and spills for their registers: groups of
+// GRP keep the latency covered at GRP values.
+__device__ __forceinline__ float2 ld_tab2(const float2 *p) {
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+constexpr int GRP = 8;
+
+// buf[at(k)] = v[e] * table[idx(k)] (conjugated for INV), k = reg_freq(e); k = 0 has
+// twiddle 1.
+template <int R, bool INV, class At, class Idx>
+__device__ __forceinline__ void twiddle_store(const float2 (&v)[R], float2 *buf,
+                                              const float2 *__restrict__ tw, At &&at, Idx &&idx) {
+    static_for<(R + GRP - 1) / GRP>([&](auto G) {
+        constexpr int e0 = G * GRP, n = R - e0 < GRP ? R - e0 : GRP;
+        float2 w[n];
+        static_for<n>([&](auto I) {
+            constexpr int k = reg_freq<R>(e0 + I);
+            if constexpr (k != 0) w[I] = ld_tab2(tw + idx(k));
+        });
+        static_for<n>([&](auto I) {
+            constexpr int k = reg_freq<R>(e0 + I);
+            float2 x = v[e0 + I];
+            if constexpr (k != 0) x = INV ? cmulc(x, w[I]) : cmul(x, w[I]);
+            buf[at(k)] = x;
+        });
+    });
+}
+
 // Stage 1 of T columns: v holds elements b + a R2 of column t; radix-R1 DFT,
 // twiddles, exchange buffer.
-template <int N, bool INV>
-__device__ __forceinline__ void col_stage1(float2 (&v)[Fac<N>::R1], float2 *buf, int t, int b,
+template <class C, bool INV>
+__device__ __forceinline__ void col_stage1(float2 (&v)[C::R1], float2 *buf, int t, int b,
                                            const float2 *__restrict__ tw) {
-    using C = ColCfg<N>;
     reg_dft<C::R1, INV>(v);
     static_for<C::R1>([&](auto E) {
         constexpr int k1 = reg_freq<C::R1>(E);
@@ -119,10 +163,8 @@ __device__ __forceinline__ void col_stage1(float2 (&v)[Fac<N>::R1], float2 *buf,
 }
 
 // Stage 2 of group (t, k1): u[e] holds frequency k1 + R1 reg_freq(e).
-template <int N, bool INV>
-__device__ __forceinline__ void col_stage2(float2 (&u)[Fac<N>::R2], const float2 *buf, int t,
-                                           int k1) {
-    using C = ColCfg<N>;
+template <class C, bool INV>
+__device__ __forceinline__ void col_stage2(float2 (&u)[C::R2], const float2 *buf, int t, int k1) {
 #pragma unroll
     for (int b = 0; b < C::R2; ++b) u[b] = buf[k1 * C::GS + b * C::T + t];
     reg_dft<C::R2, INV>(u);
@@ -132,11 +174,21 @@ __device__ __forceinline__ void col_stage2(float2 (&u)[Fac<N>::R2], const float2
 // the stores to the later loads in registers, which costs a block per SM.
 __device__ __forceinline__ void parked() { asm volatile("" ::: "memory"); }
 
-// Blocks per SM that `bufs` exchange buffers leave room for, at most 8.
-template <int N>
-constexpr int col_blocks(int bufs) {
-    const int by_smem = 227 * 1024 / (bufs * ColCfg<N>::BUF * 8 + 1024);
-    return by_smem < 1 ? 1 : (by_smem > 8 ? 8 : by_smem);
+// A stride the compiler cannot see through: otherwise the 64-bit offsets of one
+// phase's accesses stay in registers (two for each of 32 elements) for the next
+// phase that uses the same ones.
+__device__ __forceinline__ int64_t fresh(int64_t v) {
+    asm volatile("" : "+l"(v));
+    return v;
+}
+
+// Blocks per SM that `bufs` exchange buffers and `regs` registers per thread
+// leave room for.
+template <class C>
+constexpr int col_blocks(int bufs, int regs) {
+    const int by_smem = 227 * 1024 / (bufs * C::BUF * 8 + 1024), by_regs = 65536 / (regs * C::TH);
+    const int n = by_smem < by_regs ? by_smem : by_regs;
+    return n < 1 ? 1 : n;
 }
 
 template <class K>
@@ -145,8 +197,8 @@ int smem_opt_in(K *fn, size_t bytes) {
     PMX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return PMX_OK;
 }
-template <int N>
-constexpr size_t cols_smem(int bufs) { return (size_t)bufs * ColCfg<N>::BUF * sizeof(float2); }
+template <class C>
+constexpr size_t cols_smem(int bufs) { return (size_t)bufs * C::BUF * sizeof(float2); }
 
 // Calls f(integral_constant<int, N>{}) for the supported length n.
 template <class F>

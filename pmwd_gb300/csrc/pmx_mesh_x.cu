@@ -9,21 +9,36 @@ namespace pmx {
 
 namespace {
 
+// Registers per thread of an x kernel.
+template <int N>
+constexpr int x_regs() { return Fac<N>::R1 >= 24 ? 160 : (Fac<N>::R1 >= 16 ? 96 : 64); }
+
+// The wavenumber tables are read in groups of eight, in program order: left
+// alone the compiler hoists all of a thread's table loads to the front, and
+// their registers with them.
+__device__ __forceinline__ float ld_tab(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 // Inverse first step on a register group in natural order: radix-R2 inverse
 // DFT, conjugate twiddles, back into the group's own place in the buffer.
 template <int N>
 __device__ __forceinline__ void x_inv_step2(const float2 (&w)[Fac<N>::R2], float2 *buf, int t,
                                             int k1, const float2 *__restrict__ twt) {
-    using C = ColCfg<N>;
+    using C = XCol<N>;
     float2 u[C::R2];
     reg_natural<C::R2>(w, u);
     reg_dft<C::R2, true>(u);
-    static_for<C::R2>([&](auto E) {
-        constexpr int b = reg_freq<C::R2>(E);
-        float2 x = u[E];
-        if constexpr (b != 0) x = cmulc(x, __ldg(twt + b * C::R1 + k1));
-        buf[k1 * C::GS + b * C::T + t] = x;
-    });
+    twiddle_store<C::R2, true>(u, buf, twt, [&](int b) { return k1 * C::GS + b * C::T + t; },
+                               [&](int b) { return b * C::R1 + k1; });
+}
+
+// Offset of x = b + A R2 from the column's first block; xbs: 8 x-planes.
+template <int R2, int A>
+__device__ __forceinline__ int64_t x_off(int b, int64_t xbs) {
+    return ((b >> 3) + A * (R2 / 8)) * xbs + (b & 7) * 4;
 }
 
 // Inverse second step: radix-R1 inverse DFTs over k1, stored to column t at
@@ -31,26 +46,24 @@ __device__ __forceinline__ void x_inv_step2(const float2 (&w)[Fac<N>::R2], float
 template <int N>
 __device__ __forceinline__ void x_inv_step1(const float2 *buf, int t, int b, float2 *dst,
                                             int64_t xbs) {
-    using C = ColCfg<N>;
+    using C = XCol<N>;
     float2 v[C::R1];
 #pragma unroll
     for (int k1 = 0; k1 < C::R1; ++k1) v[k1] = buf[k1 * C::GS + b * C::T + t];
     reg_dft<C::R1, true>(v);
-    static_for<C::R1>([&](auto E) {
-        const int x = b + reg_freq<C::R1>(E) * C::R2;
-        dst[(x >> 3) * xbs + (x & 7) * 4] = v[E];
-    });
+    const int64_t xs = fresh(xbs);
+    static_for<C::R1>([&](auto E) { dst[x_off<C::R2, reg_freq<C::R1>(E)>(b, xs)] = v[E]; });
 }
 
 // s0: H in, G_0 out (in place: a block reads its whole tile before it
 // writes); s1: Q out.
 template <int N>
-__global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_fwd(float2 *s0, float2 *s1,
+__global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(2, x_regs<N>())) k_xaxis_fwd(float2 *s0, float2 *s1,
                                                              const float2 *__restrict__ tw,
                                                              const float *__restrict__ kt,
                                                              const __grid_constant__ GreenTab gt,
                                                              MeshGeom g) {
-    using C = ColCfg<N>;
+    using C = XCol<N>;
     constexpr int R1 = C::R1, R2 = C::R2;
     extern __shared__ __align__(16) float2 sm[];
     float2 *A = sm, *B = sm + C::BUF;
@@ -63,12 +76,9 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_fwd(f
     float2 *p0 = s0 + at, *p1 = s1 + at;
     {
         float2 v[R1];
-#pragma unroll
-        for (int a = 0; a < R1; ++a) {
-            const int x = b + a * R2;
-            v[a] = p0[(x >> 3) * xbs + (x & 7) * 4];
-        }
-        col_stage1<N, false>(v, A, t, b, tw_fwd<N>(tw));
+        const int64_t xs = fresh(xbs);
+        static_for<R1>([&](auto I) { v[I] = p0[x_off<R2, I>(b, xs)]; });
+        col_stage1<C, false>(v, A, t, b, tw_fwd<N>(tw));
     }
     __syncthreads();
     const int64_t tot = g.n0 + g.n1 + g.n2h;
@@ -77,11 +87,11 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_fwd(f
     const float cc = gt.c[blockIdx.y];
     for (int k1 = b; k1 < R1; k1 += R2) {
         float2 v[R2];
-        col_stage2<N, false>(v, A, t, k1);
+        col_stage2<C, false>(v, A, t, k1);
         float2 w[R2];
         static_for<R2>([&](auto E) {
             const int ix = k1 + R1 * reg_freq<R2>(E);
-            const float kxi = __ldg(kt + ix), mxi = __ldg(kt + tot + ix);
+            const float kxi = ld_tab(kt + ix), mxi = ld_tab(kt + tot + ix);
             const float k2v = __fadd_rn(__fadd_rn(__fmul_rn(kxi, kxi), ky2), kz2);
             // laplace (k = 0 -> 0); c / k^2 to within 2 ulp
             const float rk = k2v != 0.f ? __fdividef(cc, k2v) : 0.f;
@@ -89,6 +99,7 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_fwd(f
             // P waits in the thread's own group of A while G_0 is transformed
             A[k1 * C::GS + E * C::T + t] = make_float2(pr, pi);
             w[E] = make_float2(__fmul_rn(mxi, pi), -__fmul_rn(mxi, pr));  // -i kx P
+            if constexpr (E % 8 == 7) parked();
         });
         x_inv_step2<N>(w, B, t, k1, tw_tr<N>(tw));
         parked();
@@ -103,12 +114,12 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_fwd(f
 
 // s0: C_0 in, S out (in place); s1: D in.
 template <int N>
-__global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_adj(float2 *s0, const float2 *s1,
+__global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(2, x_regs<N>())) k_xaxis_adj(float2 *s0, const float2 *s1,
                                                              const float2 *__restrict__ tw,
                                                              const float *__restrict__ kt,
                                                              const __grid_constant__ GreenTab gt,
                                                              MeshGeom g) {
-    using C = ColCfg<N>;
+    using C = XCol<N>;
     constexpr int R1 = C::R1, R2 = C::R2;
     extern __shared__ __align__(16) float2 sm[];
     float2 *A = sm, *B = sm + C::BUF;
@@ -123,12 +134,9 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_adj(f
     for (int j = 0; j < 2; ++j) {
         const float2 *p = j ? s1 + at : p0;
         float2 v[R1];
-#pragma unroll
-        for (int a = 0; a < R1; ++a) {
-            const int x = b + a * R2;
-            v[a] = p[(x >> 3) * xbs + (x & 7) * 4];
-        }
-        col_stage1<N, false>(v, sm + j * C::BUF, t, b, tw_fwd<N>(tw));
+        const int64_t xs = fresh(xbs);
+        static_for<R1>([&](auto I) { v[I] = p[x_off<R2, I>(b, xs)]; });
+        col_stage1<C, false>(v, sm + j * C::BUF, t, b, tw_fwd<N>(tw));
     }
     __syncthreads();
     const int64_t tot = g.n0 + g.n1 + g.n2h;
@@ -137,19 +145,20 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_adj(f
     const float cc = gt.c[blockIdx.y];
     for (int k1 = b; k1 < R1; k1 += R2) {
         float2 v[R2];
-        col_stage2<N, false>(v, A, t, k1);
+        col_stage2<C, false>(v, A, t, k1);
         static_for<R2>([&](auto E) { A[k1 * C::GS + E * C::T + t] = v[E]; });
         parked();
-        col_stage2<N, false>(v, B, t, k1);
+        col_stage2<C, false>(v, B, t, k1);
         static_for<R2>([&](auto E) {
             const int ix = k1 + R1 * reg_freq<R2>(E);
-            const float kxi = __ldg(kt + ix), mxi = __ldg(kt + tot + ix);
+            const float kxi = ld_tab(kt + ix), mxi = ld_tab(kt + tot + ix);
             const float k2v = __fadd_rn(__fadd_rn(__fmul_rn(kxi, kxi), ky2), kz2);
             const float2 c0 = A[k1 * C::GS + E * C::T + t];
             const float re = __fadd_rn(-__fmul_rn(mxi, c0.y), v[E].x);
             const float im = __fadd_rn(__fmul_rn(mxi, c0.x), v[E].y);
             const float rk = k2v != 0.f ? __fdividef(cc, k2v) : 0.f;
             v[E] = make_float2(-__fmul_rn(re, rk), -__fmul_rn(im, rk));
+            if constexpr (E % 8 == 7) parked();
         });
         x_inv_step2<N>(v, A, t, k1, tw_tr<N>(tw));
     }
@@ -162,20 +171,20 @@ __global__ void __launch_bounds__(ColCfg<N>::TH, col_blocks<N>(2)) k_xaxis_adj(f
 
 int mesh_xaxis_prepare(int64_t n0) {
     return mesh_axis_dispatch(n0, [&](auto N) -> int {
-        int st = smem_opt_in(k_xaxis_fwd<N>, cols_smem<N>(2));
-        return st ? st : smem_opt_in(k_xaxis_adj<N>, cols_smem<N>(2));
+        int st = smem_opt_in(k_xaxis_fwd<N>, cols_smem<XCol<N>>(2));
+        return st ? st : smem_opt_in(k_xaxis_adj<N>, cols_smem<XCol<N>>(2));
     });
 }
 
 int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, const float2 *tw,
                const float *kt, const GreenTab &gt, cudaStream_t st) {
     return mesh_axis_dispatch(g.n0, [&](auto N) -> int {
-        using C = ColCfg<N>;
+        using C = XCol<N>;
         const dim3 grid((unsigned)(g.n1 * ((4 * g.nzt + C::T - 1) / C::T)), nslot);
         if (adj)
-            k_xaxis_adj<N><<<grid, C::TH, cols_smem<N>(2), st>>>(s0, s1, tw, kt, gt, g);
+            k_xaxis_adj<N><<<grid, C::TH, cols_smem<XCol<N>>(2), st>>>(s0, s1, tw, kt, gt, g);
         else
-            k_xaxis_fwd<N><<<grid, C::TH, cols_smem<N>(2), st>>>(s0, s1, tw, kt, gt, g);
+            k_xaxis_fwd<N><<<grid, C::TH, cols_smem<XCol<N>>(2), st>>>(s0, s1, tw, kt, gt, g);
         PMX_LAUNCH_CHECK("mesh transform, x axis");
         return PMX_OK;
     });
