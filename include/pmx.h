@@ -411,6 +411,60 @@ int pmx_random_bits(uint32_t k0, uint32_t k1, int64_t n, int layout, uint32_t *o
 int pmx_normal(uint32_t k0, uint32_t k1, int64_t n, int layout, float *out, void *stream);
 
 /* --------------------------------------------------------------------------
+ * Lagrangian perturbation theory on a 3-D grid (pmwd/lpt.py:13-76, 136-212):
+ * the stages between the caller's real-to-complex and complex-to-real
+ * transforms, and their transposes.  Spectra are complex64 half spectra
+ * (n0, n1, n2/2+1), contiguous unless strides are given (in complex values:
+ * per axis, then from one spectrum to the next); fields are float32 (n0, n1,
+ * n2).  Transforms are unnormalised; `scale` carries 1 / N where a stage
+ * reads their result, and 1 / cell volume where it reads the modes.
+ * ------------------------------------------------------------------------ */
+
+/* Floats that the tables of a grid take, and the tables: wavenumbers, the
+ * same with the Nyquist entries zeroed, the lattice displacements and pmid of
+ * particles.py:109-154. */
+int pmx_lpt_table_floats(const int64_t grid_shape[3], int64_t *count);
+int pmx_lpt_tables(const int64_t grid_shape[3], const int64_t mesh_shape[3],
+                   double ptcl_spacing, double cell_size, float *tables, void *stream);
+
+/* spec (6, ...) = -k_i k_j pot, pot = -scale modes / k^2, for ij = 00, 11, 22,
+ * 01, 02, 12 (lpt.py:13-37). */
+int pmx_lpt_strain(const int64_t grid_shape[3], const float *tables, const float *modes,
+                   float scale, float *spec, void *stream);
+
+/* Second-order source (lpt.py:40-76) of phi = scale times the six transforms
+ * phi (6, n). */
+int pmx_lpt_source(int64_t n, const float *phi, float scale, float *src, void *stream);
+
+/* spec (3 or 6, ...) = -i k_a pot of the first-order potential -scale modes /
+ * k^2 and, unless src2 is NULL, the second-order one -src2 / k^2. */
+int pmx_lpt_grad(const int64_t grid_shape[3], const float *tables, const float *modes,
+                 float scale, const float *src2, const int64_t *src2_strides, float *spec,
+                 void *stream);
+
+/* pmid, disp and vel (n, 3) of the lattice displaced by scale times the 3 *
+ * orders fields grads (lpt.py:197-210); fac (orders, 2) = D_m, a^2 H dD_m/dlna
+ * in HOST memory, or fac_dev in DEVICE memory. */
+int pmx_lpt_disp(const int64_t grid_shape[3], const float *tables, const float *grads,
+                 float scale, int32_t orders, const float *fac, const float *fac_dev,
+                 int16_t *pmid, float *disp, float *vel, void *stream);
+
+/* Transposes, for a real cotangent of disp and vel.  grads_cot (3 orders, n);
+ * src_cot: the second-order source's, in Fourier space, to be transformed by
+ * an unnormalised complex-to-real transform, from the spectra of the second
+ * order's grads_cot; phi_cot (6, n); modes_cot from the spectra of the first
+ * order's grads_cot and of phi_cot (NULL: first order only). */
+int pmx_lpt_disp_adj(int64_t n, const float *disp_cot, const float *vel_cot, int32_t orders,
+                     const float *fac, float *grads_cot, void *stream);
+int pmx_lpt_src_adj(const int64_t grid_shape[3], const float *tables, const float *spec,
+                    const int64_t *strides, float scale, float *src_cot, void *stream);
+int pmx_lpt_source_adj(int64_t n, const float *phi, float scale, const float *src_cot,
+                       float *phi_cot, void *stream);
+int pmx_lpt_modes_adj(const int64_t grid_shape[3], const float *tables, const float *grads_spec,
+                      const float *strain_spec, const int64_t *strides, float scale,
+                      float *modes_cot, const int64_t *cot_strides, void *stream);
+
+/* --------------------------------------------------------------------------
  * Growth functions (host)
  * ------------------------------------------------------------------------ */
 

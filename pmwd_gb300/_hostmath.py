@@ -128,13 +128,15 @@ def op_factors(ops, cosmo, conf):
 def lpt_factors(cosmo, conf):
     """(lpt_order, 2) float32 array of (D_m, a^2 H dD_m/dlna) at a_start."""
     a = conf.a_start
-    tables = (conf.growth_a.numpy(), cosmo.growth.detach().cpu().numpy())
-    e2 = E2(a, cosmo)
+    xp = np.concatenate((conf.a_lpt.numpy(), conf.a_nbody.numpy()[1:]))   # conf.growth_a
+    tab = cosmo.growth.detach().cpu().numpy()
+    a2H = a ** 2 * math.sqrt(E2(a, cosmo))
+    i = min(max(int(np.searchsorted(xp, a, side='right')), 1), len(xp) - 1)
     rows = []
     for order in range(1, 1 + conf.lpt_order):
-        D = growth(a, cosmo, conf, order=order, tables=tables)
-        dD_dlna = growth(a, cosmo, conf, order=order, deriv=1, tables=tables)
-        rows.append((D, a ** 2 * math.sqrt(e2) * dD_dlna))
+        D, dD = (a ** order * float(interp(a, xp[i - 1:i + 1], tab[order - 1][deriv][i - 1:i + 1]))
+                 for deriv in (0, 1))
+        rows.append((D, a2H * dD))
     return np.asarray(rows, np.float64).astype(np.float32)
 
 

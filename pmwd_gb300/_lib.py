@@ -87,6 +87,20 @@ SIGNATURES = {
                                 c_i32, c_i32, c_d, c_p, c_p, c_p, c_p]),
     'pmx_powspec_bin_zmajor': (c_int, [c_p, c_p, c_i64, ctypes.POINTER(c_i64), c_p, c_p, c_p, c_p,
                                        c_i32, c_i32, c_i32, c_d, c_p, c_p, c_p, c_p]),
+    'pmx_lpt_table_floats': (c_int, [ctypes.POINTER(c_i64), ctypes.POINTER(c_i64)]),
+    'pmx_lpt_tables': (c_int, [ctypes.POINTER(c_i64), ctypes.POINTER(c_i64), c_d, c_d, c_p, c_p]),
+    'pmx_lpt_strain': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, c_f, c_p, c_p]),
+    'pmx_lpt_source': (c_int, [c_i64, c_p, c_f, c_p, c_p]),
+    'pmx_lpt_grad': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, c_f, c_p, ctypes.POINTER(c_i64), c_p,
+                             c_p]),
+    'pmx_lpt_disp': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, c_f, c_i32, ctypes.POINTER(c_f), c_p,
+                             c_p, c_p, c_p, c_p]),
+    'pmx_lpt_disp_adj': (c_int, [c_i64, c_p, c_p, c_i32, ctypes.POINTER(c_f), c_p, c_p]),
+    'pmx_lpt_src_adj': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, ctypes.POINTER(c_i64), c_f, c_p,
+                                c_p]),
+    'pmx_lpt_source_adj': (c_int, [c_i64, c_p, c_f, c_p, c_p, c_p]),
+    'pmx_lpt_modes_adj': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, c_p, ctypes.POINTER(c_i64), c_f,
+                                  c_p, ctypes.POINTER(c_i64), c_p]),
     'pmx_growth_ode': (c_int, [c_p, c_i64, c_p, c_i64, c_d, c_d, c_p, c_p]),
     'pmx_random_bits': (c_int, [ctypes.c_uint32, ctypes.c_uint32, c_i64, c_int, c_p, c_p]),
     'pmx_normal': (c_int, [ctypes.c_uint32, ctypes.c_uint32, c_i64, c_int, c_p, c_p]),

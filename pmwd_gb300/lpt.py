@@ -1,6 +1,13 @@
-"""Lagrangian perturbation theory initial conditions (pmwd/lpt.py:1-212),
-torch on the GPU (cuFFT through torch.fft; autograd gives its VJP)."""
+"""Lagrangian perturbation theory initial conditions (pmwd/lpt.py:1-212) on
+the GPU.
 
+3-D grids on the GPU with a fixed cosmology run the stages between the
+transforms (torch.fft) as libpmx kernels, with a hand-written VJP for the
+modes (``_LptFn``); every other case (cosmology gradients, other dimensions
+and dtypes, CPU tensors) is the same computation in torch operations
+(``_lpt_device``), differentiated by autograd."""
+
+import ctypes
 import math
 import threading
 from collections import OrderedDict
@@ -136,14 +143,133 @@ def _lpt_device(modes, fac, kvec, disp0, vel0, conf):
     return disp, vel
 
 
-# CUDA-graph replay of _lpt_device for calls without gradients on small
-# grids, where launching ~10^3 small kernels one by one would cost more than
-# the transforms themselves.  One graph per (configuration, device); the
-# growth factors are a graph input, so a graph serves every cosmology.
-# Builds and replays run on one library-created stream per device under a
+def _i64(values):
+    return (_lib.c_i64 * len(values))(*values)
+
+
+class _Grid:
+    """Arguments that the libpmx stages of one grid share."""
+
+    def __init__(self, conf, dev):
+        self.shape = tuple(conf.ptcl_grid_shape)
+        self.half = self.shape[:2] + (self.shape[2] // 2 + 1,)
+        self.n = conf.ptcl_num
+        self.c = _i64(self.shape)
+        self.orders = conf.lpt_order
+        self.vol = conf.ptcl_cell_vol
+        self.dev = dev
+        self.stream = _lib.stream_ptr(dev)
+
+    def tables(self, conf):
+        count = _lib.c_i64()
+        _lib.call('pmx_lpt_table_floats', self.c, ctypes.byref(count))
+        tab = torch.empty(count.value, dtype=torch.float32, device=self.dev)
+        _lib.call('pmx_lpt_tables', self.c, _i64(conf.mesh_shape), conf.ptcl_spacing,
+                  conf.cell_size, tab, self.stream)
+        return tab
+
+    def real(self, spec):
+        """Unnormalised complex-to-real transform of each spectrum."""
+        return torch.fft.irfftn(spec, s=self.shape, dim=(-3, -2, -1), norm='forward').contiguous()
+
+    def empty(self, num, dtype=torch.float32):
+        return torch.empty((num,) + (self.half if dtype == torch.complex64 else self.shape),
+                           dtype=dtype, device=self.dev)
+
+
+def _lpt_stages(modes, fac, conf, fac_dev=None):
+    """Forward stages: (pmid, disp, vel, tables, phi); fac (lpt_order, 2) is a
+    float32 NumPy array, or fac_dev a device tensor."""
+    g = _Grid(conf, modes.device)
+    tab = g.tables(conf)
+    phi = src2 = strides = None
+    spec = g.empty(3 * g.orders, torch.complex64)
+    if g.orders > 1:
+        _lib.call('pmx_lpt_strain', g.c, tab, modes, 1 / g.vol, spec, g.stream)
+        phi = g.real(spec)
+        src = torch.empty(g.shape, dtype=torch.float32, device=g.dev)
+        _lib.call('pmx_lpt_source', g.n, phi, 1 / g.n, src, g.stream)
+        src2 = torch.fft.rfftn(src)
+        del src
+        strides = _i64(src2.stride())
+    _lib.call('pmx_lpt_grad', g.c, tab, modes, 1 / g.vol, src2, strides, spec, g.stream)
+    del src2
+    grads = g.real(spec)
+    del spec
+    pmid = torch.empty((g.n, 3), dtype=torch.int16, device=g.dev)
+    disp = torch.empty((g.n, 3), dtype=torch.float32, device=g.dev)
+    vel = torch.empty_like(disp)
+    cf = None if fac_dev is not None else (_lib.c_f * (2 * g.orders))(*fac.reshape(-1).tolist())
+    _lib.call('pmx_lpt_disp', g.c, tab, grads, 1 / g.n, g.orders, cf, fac_dev, pmid, disp, vel,
+              g.stream)
+    return pmid, disp, vel, tab, phi
+
+
+class _LptFn(torch.autograd.Function):
+    """(contiguous modes) -> (pmid, disp, vel), fac and conf fixed."""
+
+    @staticmethod
+    def forward(ctx, modes, fac, conf):
+        pmid, disp, vel, tab, phi = _lpt_stages(modes, fac, conf)
+        if ctx.needs_input_grad[0]:
+            ctx.save_for_backward(modes, tab, phi)
+            ctx.fac, ctx.conf = fac, conf
+        ctx.mark_non_differentiable(pmid)
+        return pmid, disp, vel
+
+    @staticmethod
+    def backward(ctx, _, disp_cot, vel_cot):
+        modes, tab, phi = ctx.saved_tensors
+        conf = ctx.conf
+        g = _Grid(conf, modes.device)
+        zero = None if disp_cot is not None and vel_cot is not None else torch.zeros(
+            (g.n, 3), dtype=torch.float32, device=g.dev)
+        disp_cot = zero if disp_cot is None else disp_cot
+        vel_cot = zero if vel_cot is None else vel_cot
+        if torch.is_grad_enabled():
+            # a gradient of the gradient: through the torch operations
+            grid = Particles.gen_grid(conf, vel=True, device=g.dev)
+            kvec = fftfreq(g.shape, conf.ptcl_spacing, dtype=torch.float32, device=g.dev)
+            disp, vel = _lpt_device(modes, torch.from_numpy(ctx.fac).to(g.dev), kvec, grid.disp.t(),
+                                    grid.vel.t(), conf)
+            return torch.autograd.grad((disp.t(), vel.t()), modes, (disp_cot, vel_cot),
+                                       create_graph=True) + (None, None)
+        cf = (_lib.c_f * (2 * g.orders))(*ctx.fac.reshape(-1).tolist())
+        cot = g.empty(3 * g.orders)
+        _lib.call('pmx_lpt_disp_adj', g.n, disp_cot.contiguous(), vel_cot.contiguous(), g.orders, cf,
+                  cot, g.stream)
+        C = torch.fft.rfftn(cot, dim=(-3, -2, -1))
+        st = _i64(C.stride()[1:] + C.stride()[:1])
+        S = None
+        if g.orders > 1:
+            src = torch.empty(g.half, dtype=torch.complex64, device=g.dev)
+            _lib.call('pmx_lpt_src_adj', g.c, tab, C[3:], st, 1 / g.n, src, g.stream)
+            src = g.real(src)
+            _lib.call('pmx_lpt_source_adj', g.n, phi, 1 / g.n, src, cot, g.stream)
+            del src
+            S = torch.fft.rfftn(cot, dim=(-3, -2, -1))
+            if S.stride() != C.stride():
+                S = torch.empty_strided(C.shape, C.stride(), dtype=C.dtype,
+                                        device=g.dev).copy_(S)
+        del cot
+        # the gradient in the spectra's memory order (dense)
+        order = sorted(range(3), key=lambda a: -C.stride(a + 1))
+        out = torch.empty([g.half[a] for a in order], dtype=torch.complex64, device=g.dev)
+        out = out.permute([order.index(a) for a in range(3)])
+        _lib.call('pmx_lpt_modes_adj', g.c, tab, C, S, st, 1 / (g.n * g.vol), out,
+                  _i64(out.stride()), g.stream)
+        return out, None, None
+
+
+# CUDA-graph replay for calls without gradients on small grids, where
+# launching the stages one by one costs more than running them.  One graph per
+# (configuration, device); the growth factors are a graph input, so a graph
+# serves every cosmology.  Builds and replays run on one library-created stream per device under a
 # lock, so concurrent callers (the serving threads) never share the static
 # buffers in flight and no replay lands in another graph's capture.
-GRAPH_MAX_PTCL = 256 ** 3
+# (128^3: 0.33 ms replayed, 0.52 ms launched one by one; at 256^3 the kernels
+# take 1.9 ms either way and a graph would keep its buffers and copy results)
+GRAPH_MAX_PTCL = 128 ** 3
 _GRAPHS = OrderedDict()
 _GRAPHS_MAX = 8
 _GRAPH_LOCK = threading.Lock()
@@ -166,17 +292,12 @@ class _LptGraph:
                      for _ in range(4)]
         self.ring_ev = [None] * 4
         self.slot = 0
-        grid = Particles.gen_grid(conf, vel=True, device=dev)
-        self.pmid = grid.pmid
-        self.disp0, self.vel0 = grid.disp.t(), grid.vel.t()
-        self.kvec = fftfreq(conf.ptcl_grid_shape, conf.ptcl_spacing, dtype=torch.float32,
-                            device=dev)
         cur = torch.cuda.current_stream(dev)
         self.stream.wait_stream(cur)
         with torch.no_grad():
             with torch.cuda.stream(self.stream):
                 for _ in range(2):   # plans and allocator pools before capture
-                    _lpt_device(self.modes, self.fac, self.kvec, self.disp0, self.vel0, conf)
+                    _lpt_stages(self.modes, None, conf, self.fac)
             self.stream.synchronize()
             # captured on this stream with stream-level syncs only (no device
             # synchronize, which fails while another thread captures), in
@@ -185,8 +306,7 @@ class _LptGraph:
             with torch.cuda.stream(self.stream):
                 self.graph.capture_begin(capture_error_mode='thread_local')
                 try:
-                    self.disp, self.vel = _lpt_device(self.modes, self.fac, self.kvec,
-                                                      self.disp0, self.vel0, conf)
+                    self.out = _lpt_stages(self.modes, None, conf, self.fac)[:3]
                 finally:
                     self.graph.capture_end()
             self.stream.synchronize()
@@ -207,7 +327,7 @@ class _LptGraph:
                 self.ring_ev[i] = ev
                 self.modes.copy_(modes)
                 self.graph.replay()
-                out = (self.pmid.clone(), self.disp.t().contiguous(), self.vel.t().contiguous())
+                out = tuple(t.clone() for t in self.out)
         cur.wait_stream(self.stream)
         for t in out:   # allocated on the graph's stream, used on the caller's
             t.record_stream(cur)
@@ -236,20 +356,21 @@ def _graph_for(conf, modes):
     return g
 
 
-def _wants_graph(modes, cosmo, conf):
-    if not modes.is_cuda or conf.lpt_order < 1 or conf.ptcl_num > GRAPH_MAX_PTCL:
-        return False
-    if modes.dtype != torch.complex64 or tuple(modes.shape) != tuple(
-            conf.ptcl_grid_shape[:-1]) + (conf.ptcl_grid_shape[-1] // 2 + 1,):
-        return False
-    return not _hostmath.needs_grad(modes, cosmo)
+def _fused(modes, cosmo, conf):
+    """Whether the libpmx stages apply: a 3-D complex64 half spectrum on the
+    GPU and no gradient of the cosmology."""
+    return (modes.is_cuda and conf.dim == 3 and conf.lpt_order >= 1
+            and modes.dtype == torch.complex64
+            and tuple(modes.shape) == tuple(conf.ptcl_grid_shape[:-1])
+            + (conf.ptcl_grid_shape[-1] // 2 + 1,)
+            and not _hostmath.needs_grad(cosmo))
 
 
 def lpt(modes, cosmo, conf):
     """LPT displacements and velocities at conf.a_start (lpt.py:136-212).
 
     Returns ``(ptcl, None)`` with particles on the Lagrangian grid.  Calls
-    that need no gradient, on grids up to 256^3, replay a CUDA graph of the
+    that need no gradient, on grids up to 128^3, replay a CUDA graph of the
     device work.
     """
     if conf.dim not in (1, 2, 3):
@@ -261,9 +382,13 @@ def lpt(modes, cosmo, conf):
     dev = modes.device
     if conf.lpt_order == 0:
         return Particles.gen_grid(conf, vel=True, device=dev), None
-    if _wants_graph(modes, cosmo, conf):
-        fac = torch.from_numpy(_hostmath.lpt_factors(cosmo, conf))
-        pmid, disp, vel = _graph_for(conf, modes).run(modes, fac)
+    if _fused(modes, cosmo, conf):
+        fac = _hostmath.lpt_factors(cosmo, conf)
+        if conf.ptcl_num <= GRAPH_MAX_PTCL and not _hostmath.needs_grad(modes):
+            pmid, disp, vel = _graph_for(conf, modes).run(modes, torch.from_numpy(fac))
+        else:
+            with torch.cuda.device(dev):
+                pmid, disp, vel = _LptFn.apply(modes.resolve_conj().contiguous(), fac, conf)
         return Particles(conf, pmid, disp, vel=vel), None
     fac = _growth_factors(cosmo, conf).to(dev)
     kvec = fftfreq(conf.ptcl_grid_shape, conf.ptcl_spacing, dtype=torch.float32, device=dev)
