@@ -330,8 +330,10 @@ __global__ void k_poisson_adj(float2 *ck, int64_t n0, int64_t n1, int64_t n2h, i
 // 512^3).  At one cell per particle the parity alternates from lane to lane, which
 // splits a warp's contiguous reductions (0.72 against 0.59 ms on 384^3):
 // there DEP_JOIN hands a lane's upper value to the next lane when that one's
-// lower cell is the same.  DEP_V4 (opt-in, PMX_WS_VEC): one 16-byte reduction
-// inside an aligned group of four floats, two of them zeros.
+// lower cell is the same, in warps where at least 12 lanes can, and adds as
+// DEP_V2 in those whose particles have left the lattice.  DEP_V4 (opt-in,
+// PMX_WS_VEC): one 16-byte reduction inside an aligned group of four floats, two
+// of them zeros.
 enum Dep { DEP_SCALAR, DEP_V2, DEP_JOIN, DEP_V4 };
 
 struct Hot {
@@ -356,17 +358,8 @@ struct Hot {
     int64_t pstride;
 };
 
-// x / cell as IEEE division gives it: a multiplication where 1 / cell is exact.
 __device__ __forceinline__ float hot_div(const Hot &h, float x) {
-    return h.inv != 0.f ? __fmul_rn(x, h.inv) : __fdiv_rn(x, h.cell);
-}
-
-// i modulo n; positions within one period of the box, the usual ones, take an
-// addition instead of an integer division.
-__device__ __forceinline__ int hot_wrap(int i, int n) {
-    if ((unsigned)i < (unsigned)n) return i;
-    i += i < 0 ? n : -n;
-    return (unsigned)i < (unsigned)n ? i : pymod(i, n);
+    return div_or_mul(x, h.cell, h.inv);
 }
 
 // Neighbours of one axis, as enmesh_axis (pm_util.py:119-149) computes them:
@@ -381,7 +374,7 @@ __device__ __forceinline__ void hot_axis(const Hot &h, int a, int pm, float d, A
     ax.s[0] = d0 > 0.f ? -1.f : -d0;
     ax.s[1] = d1 < 0.f ? 1.f : -d1;
     ax.u = fl + pm;
-    ax.i[0] = hot_wrap(ax.u, h.wrap[a]);
+    ax.i[0] = fast_mod(ax.u, h.wrap[a]);
     ax.i[1] = ax.i[0] + 1 == h.wrap[a] ? 0 : ax.i[0] + 1;
 }
 
@@ -575,7 +568,7 @@ __device__ __forceinline__ int64_t hot_row(const Hot &h, const Axis ax[3], int p
 // particle's eight neighbours; pl[c][b] is the x-plane of neighbour bit b.
 template <int NC>
 __device__ __forceinline__ void hot_add1(const Hot &h, const Axis ax[3], const float (&v)[NC],
-                                         float *const (&pl)[NC][2]) {
+                                         float *const (&pl)[NC][2], int dep) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         const float fxy = __fmul_rn(ax[0].w[p & 1], ax[1].w[p >> 1]);
@@ -584,7 +577,7 @@ __device__ __forceinline__ void hot_add1(const Hot &h, const Axis ax[3], const f
 #pragma unroll
         for (int c = 0; c < NC; ++c)
             zpair_add(pl[c][p & 1], y, ax[2].i[0], ax[2].i[1], __fmul_rn(v[c], fa),
-                      __fmul_rn(v[c], fb), h.dep);
+                      __fmul_rn(v[c], fb), dep);
     }
 }
 
@@ -595,7 +588,7 @@ __device__ __forceinline__ void hot_add(const Hot &h, bool act, const Axis ax[3]
                                         const float (&v)[NC], float *const (&pl)[NC][2]) {
     const int i0 = ax[2].i[0], i1 = ax[2].i[1];
     if (h.dep != DEP_JOIN) {
-        if (act) hot_add1<NC>(h, ax, v, pl);
+        if (act) hot_add1<NC>(h, ax, v, pl, h.dep);
         return;
     }
     // join: the previous lane's upper cells are this lane's lower ones
@@ -605,7 +598,12 @@ __device__ __forceinline__ void hot_add(const Hot &h, bool act, const Axis ax[3]
     const unsigned po = __shfl_up_sync(0xffffffffu, o, 1);
     const int px = __shfl_up_sync(0xffffffffu, x, 1);
     const bool join = act && lane > 0 && px == x && po + 1 == o && i0 != 0;
-    const bool next = (__ballot_sync(0xffffffffu, join) >> lane >> 1) & 1;
+    const unsigned jm = __ballot_sync(0xffffffffu, join);
+    if (__popc(jm) < 12) {
+        if (act) hot_add1<NC>(h, ax, v, pl, (h.stride[1] & 1) == 0 ? DEP_V2 : DEP_SCALAR);
+        return;
+    }
+    const bool next = (jm >> lane >> 1) & 1;
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         const float fxy = __fmul_rn(ax[0].w[p & 1], ax[1].w[p >> 1]);
@@ -632,7 +630,7 @@ __device__ __forceinline__ void hot_add(const Hot &h, bool act, const Axis ax[3]
 __device__ __forceinline__ void hot_deposit1(const Hot &h, const Axis ax[3], float *dens) {
     const float v[1] = {h.val};
     float *const pl[1][2] = {{hot_plane(dens, ax, 0, h.stride[0]), hot_plane(dens, ax, 1, h.stride[0])}};
-    hot_add1<1>(h, ax, v, pl);
+    hot_add1<1>(h, ax, v, pl, h.dep);
 }
 __device__ __forceinline__ void hot_deposit(const Hot &h, bool act, const Axis ax[3], float *dens) {
     const float v[1] = {h.val};
@@ -1674,8 +1672,7 @@ int check_hot(pmx_workspace *ws, const pmx_enmesh_spec *spec, const void *pmid, 
     h->stride[1] = ws->n2;
     h->stride[0] = ws->n1 * ws->n2;
     h->cell = (float)spec->conf_cell_size;
-    int e2 = 0;
-    h->inv = std::frexp(h->cell, &e2) == 0.5f && e2 > -126 && e2 < 126 ? 1.f / h->cell : 0.f;
+    h->inv = exact_inverse(h->cell);
     h->val = (float)((double)ws->M / (double)ptcl_num);
     h->dcomp = nullptr;
     h->vcomp = nullptr;

@@ -59,6 +59,7 @@ struct EmParams {
     int f64;           // 1: non-default (float64) branch, pm_util.py:99-118
     // default branch (pm_util.py:119-137)
     float cellf;       // a1 as float32
+    float cell_inv;    // exact_inverse(cellf)
     int i12[3];        // integer part of offset / a1 (jnp.divmod)
     float d12[3];      // remainder, cast to float32
     // float64 branch
@@ -72,6 +73,8 @@ struct EmParams {
 };
 
 int make_em_params(const pmx_enmesh_spec *spec, EmParams *p);
+// 1 / y if y is a power of two well inside the float range, else 0.
+float exact_inverse(float y);
 
 // 3-D mesh transforms of the Poisson solve by this library's own kernels
 // (pmx_mesh_fft.cuh; pmx_mesh_rows.cu, pmx_mesh_cols.cu, pmx_mesh_x.cu).
@@ -134,13 +137,31 @@ __device__ __forceinline__ int pymod(int x, int m) {
     return r < 0 ? r + m : r;
 }
 
+// i modulo n; positions within one period of the box, the usual ones, take an
+// addition instead of an integer division.
+__device__ __forceinline__ int fast_mod(int i, int n) {
+    if ((unsigned)i < (unsigned)n) return i;
+    i += i < 0 ? n : -n;
+    return (unsigned)i < (unsigned)n ? i : pymod(i, n);
+}
+
+// x / y as IEEE division gives it, by multiplying with inv = 1 / y where that
+// is exact (y a power of two; inv = 0 otherwise).
+__device__ __forceinline__ float div_or_mul(float x, float y, float inv) {
+    return inv != 0.f ? __fmul_rn(x, inv) : __fdiv_rn(x, y);
+}
+
 __device__ __forceinline__ float sgnf(float x) {
     // jnp.sign: -1, 0 (signed), +1
     return x > 0.f ? 1.f : (x < 0.f ? -1.f : x);
 }
 
-// jnp.remainder for doubles (sign of divisor)
+// jnp.remainder for doubles (sign of divisor).  Within one period either way
+// fmod is x or, exactly, x - m; its general loop is what costs at this device's
+// float64 rate.
 __device__ __forceinline__ double pyfmod(double x, double m) {
+    if (x >= 0.0 && x < m) return x;
+    if (x >= m && x < 2.0 * m) return __dsub_rn(x, m);
     double t = fmod(x, m);
     if (t != 0.0 && ((t < 0.0) != (m < 0.0))) t = __dadd_rn(t, m);
     return t;
@@ -148,6 +169,15 @@ __device__ __forceinline__ double pyfmod(double x, double m) {
 
 // jnp.floor_divide for doubles (CPython float_divmod + round half away)
 __device__ __forceinline__ double floordiv(double x, double y) {
+    if (x >= 0.0 && y > 0.0 && x < 1e9 * y) {
+        // the quotient's floor, corrected by its remainder, which is exact in
+        // one fused operation: what fmod and the division below come to
+        double q = floor(__ddiv_rn(x, y));
+        const double r = fma(-q, y, x);
+        if (r < 0.0) q -= 1.0;
+        else if (r >= y) q += 1.0;
+        return q;
+    }
     double mod = fmod(x, y);
     double div = __ddiv_rn(__dsub_rn(x, mod), y);
     if (mod != 0.0 && ((y < 0.0) != (mod < 0.0))) div = __dsub_rn(div, 1.0);
@@ -173,7 +203,7 @@ __device__ __forceinline__ void enmesh_axis(const EmParams &p, int a, int pm, fl
     }
     if (!p.f64) {
         int ip = pm - p.i12[a];
-        float x = __fdiv_rn(__fsub_rn(d, p.d12[a]), p.cellf);
+        float x = div_or_mul(__fsub_rn(d, p.d12[a]), p.cellf, p.cell_inv);
         int fl = (int)floorf(x);
 #pragma unroll
         for (int nb = 0; nb < 2; ++nb) {
@@ -182,7 +212,7 @@ __device__ __forceinline__ void enmesh_axis(const EmParams &p, int a, int pm, fl
             ax.w[nb] = __fsub_rn(1.f, fabsf(d2));
             ax.s[nb] = sgnf(-d2);
             // without wrapping, the reference's int16 sum (two's complement)
-            ax.i[nb] = p.wrap[a] ? pymod(ii + ip, p.wrap[a]) : (int)(short)(ii + ip);
+            ax.i[nb] = p.wrap[a] ? fast_mod(ii + ip, p.wrap[a]) : (int)(short)(ii + ip);
         }
     } else {
         double P = __dsub_rn(__dadd_rn(__dmul_rn((double)pm, p.a1d), (double)d), p.b12[a]);
@@ -192,7 +222,8 @@ __device__ __forceinline__ void enmesh_axis(const EmParams &p, int a, int pm, fl
             if (p.wrap[a]) x = pyfmod(x, p.L[a]);
             double q = floordiv(x, p.a2d);
             double d2 = __dsub_rn(P, __dmul_rn(q, p.a2d));
-            if (p.wrap[a]) d2 = __dsub_rn(d2, __dmul_rn(rint(__ddiv_rn(d2, p.L[a])), p.L[a]));
+            if (p.wrap[a] && fabs(d2) >= 0.25 * p.L[a])   // below, the rounded quotient is 0
+                d2 = __dsub_rn(d2, __dmul_rn(rint(__ddiv_rn(d2, p.L[a])), p.L[a]));
             float d2f = __fdiv_rn((float)d2, p.a2f);
             ax.w[nb] = __fsub_rn(1.f, fabsf(d2f));
             ax.s[nb] = sgnf(-d2f);

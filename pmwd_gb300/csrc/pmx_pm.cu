@@ -5,9 +5,20 @@
 // pmwd/particles.py:212-254.  The Poisson-force hot path uses the fused,
 // specialised kernels in pmx_force.cu.
 //
-// One thread per particle, grid-stride.  Scatter-type updates use float32
-// global reductions (red.global.add.f32 through atomicAdd with the result
-// unused), like the reference's XLA scatter-add.
+// One thread per particle.  Scatter-type updates use float32 global reductions
+// (red.global.add through atomicAdd with the result unused), like the
+// reference's XLA scatter-add.
+//
+// Two sets of kernels.  The default enmesh in 3-D with one or three channels
+// (k_*_cic: any periodic particle set on its own mesh, the usual call) has
+// every neighbour in the mesh, so rows are addressed by 32-bit offsets within
+// an x-plane, both z neighbours are read together and reductions of adjacent
+// cells are merged.  The general kernels cover everything else: other cell
+// sizes (the float64 branch), other dimensions, dropped neighbours, any number
+// of channels.  What bounds the k_*_cic kernels is the L2's reductions and, for
+// clustered sets, its reads.  With the general kernels / with these: scatter and
+// its VJP, 256^3 clustered particles on 256^3, 1.56 / 0.83 ms; gather of three
+// channels and its VJP, 175 x 125 x 225, 0.90 / 0.50 ms.
 
 #include <cmath>
 #include <cstdio>
@@ -56,6 +67,11 @@ static void host_float_divmod(double x, double y, double *div, double *mod) {
     *mod = m;
 }
 
+float exact_inverse(float y) {
+    int e = 0;
+    return std::frexp(y, &e) == 0.5f && e > -126 && e < 126 ? 1.f / y : 0.f;
+}
+
 int make_em_params(const pmx_enmesh_spec *s, EmParams *p) {
     if (!s) return fail(PMX_ERR_ARG, "null enmesh spec");
     if (s->dim < 1 || s->dim > 3) return fail(PMX_ERR_ARG, "dim must be 1, 2 or 3");
@@ -87,6 +103,7 @@ int make_em_params(const pmx_enmesh_spec *s, EmParams *p) {
     p->stride[0] = p->shape[1] * p->shape[2];
     p->f64 = s->cell_size > 0 ? 1 : 0;
     p->cellf = (float)s->conf_cell_size;
+    p->cell_inv = exact_inverse(p->cellf);
     p->a1d = s->conf_cell_size;
     p->a2d = s->cell_size > 0 ? s->cell_size : s->conf_cell_size;
     p->a2f = (float)p->a2d;
@@ -270,6 +287,299 @@ __global__ void k_gather_adj(EmParams p, const int16_t *__restrict__ pmid,
     }
 }
 
+// --------------------------------------------------------------------------
+// default enmesh, 3-D, NC = 1 or 3 channels
+// --------------------------------------------------------------------------
+
+struct Cic {
+    int wrap[3], i12[3];
+    float d12[3], cell, inv, div, div_inv;
+    int64_t s0;      // cells of an x-plane of the mesh array
+    unsigned s1;     // cells of a row
+    bool join;       // about one cell per particle: hand values to the next lane
+    bool pair;       // the added-to array starts on 8 bytes
+};
+
+struct CicAxis {
+    int i[2];
+    float w[2], s[2];
+};
+
+__device__ __forceinline__ void cic_axes(const Cic &p, const int16_t *__restrict__ pmid,
+                                         const float *__restrict__ disp, int64_t q, CicAxis ax[3]) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float x = div_or_mul(__fsub_rn(disp[3 * q + a], p.d12[a]), p.cell, p.inv);
+        const int fl = (int)floorf(x);
+        const float d0 = __fsub_rn(x, (float)fl), d1 = __fsub_rn(x, (float)(fl + 1));
+        ax[a].w[0] = __fsub_rn(1.f, fabsf(d0));
+        ax[a].w[1] = __fsub_rn(1.f, fabsf(d1));
+        ax[a].s[0] = sgnf(-d0);
+        ax[a].s[1] = sgnf(-d1);
+        ax[a].i[0] = fast_mod(fl + (int)pmid[3 * q + a] - p.i12[a], p.wrap[a]);
+        ax[a].i[1] = ax[a].i[0] + 1 == p.wrap[a] ? 0 : ax[a].i[0] + 1;
+    }
+}
+
+// Row r (bit 0: x neighbour, bit 1: y neighbour): its cells' offset from the
+// start of the array is x * s0 + the 32-bit offset.
+__device__ __forceinline__ int64_t cic_plane(const Cic &p, const CicAxis ax[3], int r) {
+    return ax[0].i[r & 1] * p.s0;
+}
+__device__ __forceinline__ unsigned cic_row(const Cic &p, const CicAxis ax[3], int r) {
+    return (unsigned)ax[1].i[r >> 1] * p.s1;
+}
+
+// The NC channels at both z neighbours of a row, m[bit][c].
+template <int NC>
+__device__ __forceinline__ void cic_read(const Cic &p, const CicAxis ax[3], int r,
+                                         const float *__restrict__ mesh, float (&m)[2][NC]) {
+    const float *b = mesh + cic_plane(p, ax, r) * NC;
+    const unsigned y = cic_row(p, ax, r);
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) m[z][c] = __ldg(b + ((y + (unsigned)ax[2].i[z]) * NC + c));
+}
+
+// Adds v[c] (w_x w_y) w_z to the eight neighbours (every lane of a warp calls
+// it).  Two ways to merge reductions, chosen per warp:
+// join: a lane hands its upper z neighbours' values to the next lane if that
+// one's lower cells are the same, the rule among neighbours on the lattice at
+// one cell per particle.  Taken where at least 12 of 32 lanes can.
+// pair (arrays on 8 bytes): adjacent floats of the row at an even offset take
+// one 8-byte reduction: finer meshes and particles that have left the lattice.
+template <int NC>
+__device__ __forceinline__ void cic_add(const Cic &p, bool act, const CicAxis ax[3],
+                                        const float (&v)[NC], float *mesh) {
+    const int i0 = ax[2].i[0], i1 = ax[2].i[1];
+    bool join = false, next = false, joined = false;
+    if (p.join) {
+        const int lane = threadIdx.x & 31;
+        const unsigned o = act ? cic_row(p, ax, 0) + (unsigned)i0 : 0u;
+        const int x = act ? ax[0].i[0] : -1;
+        const unsigned po = __shfl_up_sync(0xffffffffu, o, 1);
+        const int px = __shfl_up_sync(0xffffffffu, x, 1);
+        join = act && lane > 0 && px == x && po + 1 == o && i0 != 0;
+        const unsigned jm = __ballot_sync(0xffffffffu, join);
+        joined = __popc(jm) >= 12;
+        next = (jm >> lane >> 1) & 1;
+    }
+    if (joined) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float fxy = __fmul_rn(ax[0].w[r & 1], ax[1].w[r >> 1]);
+            const float fa = __fmul_rn(fxy, ax[2].w[0]), fb = __fmul_rn(fxy, ax[2].w[1]);
+            float *b = mesh + cic_plane(p, ax, r) * NC;
+            const unsigned y = cic_row(p, ax, r);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                float e = __fmul_rn(v[c], fa);
+                const float u = __fmul_rn(v[c], fb), pu = __shfl_up_sync(0xffffffffu, u, 1);
+                if (join) e += pu;
+                if (act) {
+                    atomicAdd(b + ((y + (unsigned)i0) * NC + c), e);
+                    if (!next) atomicAdd(b + ((y + (unsigned)i1) * NC + c), u);
+                }
+            }
+        }
+        return;
+    }
+    if (!act) return;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const float fxy = __fmul_rn(ax[0].w[r & 1], ax[1].w[r >> 1]);
+        const float fa = __fmul_rn(fxy, ax[2].w[0]), fb = __fmul_rn(fxy, ax[2].w[1]);
+        const int64_t plane = cic_plane(p, ax, r) * NC;
+        float *b = mesh + plane, e[2 * NC];
+        const unsigned y = cic_row(p, ax, r);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            e[c] = __fmul_rn(v[c], fa);
+            e[NC + c] = __fmul_rn(v[c], fb);
+        }
+        const unsigned o0 = (y + (unsigned)i0) * NC, o1 = (y + (unsigned)i1) * NC;
+        if (!p.pair || i1 != i0 + 1) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                atomicAdd(b + (o0 + c), e[c]);
+                atomicAdd(b + (o1 + c), e[NC + c]);
+            }
+        } else if (((o0 + (unsigned)plane) & 1u) == 0) {   // 2 NC floats in NC pairs
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                atomicAdd(reinterpret_cast<float2 *>(b + (o0 + 2 * c)),
+                          make_float2(e[2 * c], e[2 * c + 1]));
+        } else {                                           // a single one at either end
+            atomicAdd(b + o0, e[0]);
+#pragma unroll
+            for (int c = 0; c + 1 < NC; ++c)
+                atomicAdd(reinterpret_cast<float2 *>(b + (o0 + 2 * c + 1)),
+                          make_float2(e[2 * c + 1], e[2 * c + 2]));
+            atomicAdd(b + (o0 + 2 * NC - 1), e[2 * NC - 1]);
+        }
+    }
+}
+
+template <int NC>
+__device__ __forceinline__ void ld_val(const float *__restrict__ val, float scalar, int64_t q,
+                                       float (&v)[NC]) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = val ? val[q * NC + c] : scalar;
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_scatter_cic(Cic p, const int16_t *__restrict__ pmid,
+                                                     const float *__restrict__ disp, int64_t n,
+                                                     const float *__restrict__ val,
+                                                     float val_scalar, float *mesh) {
+    for (int64_t q0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); q0 < n;
+         q0 += (int64_t)gridDim.x * blockDim.x) {   // warp-uniform
+        const int64_t q = q0 + (threadIdx.x & 31);
+        CicAxis ax[3] = {};
+        float v[NC] = {};
+        if (q < n) {
+            cic_axes(p, pmid, disp, q, ax);
+            ld_val<NC>(val, val_scalar, q, v);
+        }
+        cic_add<NC>(p, q < n, ax, v, mesh);
+    }
+}
+
+// Position term sum_k t_k dfrac_k / cell of a row's two values t[bit].
+__device__ __forceinline__ void cic_grad(const CicAxis ax[3], int r, const float t[2], float c[3]) {
+    const int bx = r & 1, by = r >> 1;
+    const float T = fmaf(t[1], ax[2].w[1], t[0] * ax[2].w[0]);
+    const float D = fmaf(t[1], ax[2].s[1], t[0] * ax[2].s[0]);
+    c[0] = fmaf(ax[0].s[bx] * ax[1].w[by], T, c[0]);
+    c[1] = fmaf(ax[0].w[bx] * ax[1].s[by], T, c[1]);
+    c[2] = fmaf(ax[0].w[bx] * ax[1].w[by], D, c[2]);
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_scatter_adj_cic(
+    Cic p, const int16_t *__restrict__ pmid, const float *__restrict__ disp, int64_t n,
+    const float *__restrict__ val, float val_scalar, const float *__restrict__ mesh_cot,
+    float *disp_cot, float *val_cot) {
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        CicAxis ax[3];
+        float v[NC], g[NC] = {}, c[3] = {0.f, 0.f, 0.f};
+        cic_axes(p, pmid, disp, q, ax);
+        ld_val<NC>(val, val_scalar, q, v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float m[2][NC], t[2] = {0.f, 0.f};
+            cic_read<NC>(p, ax, r, mesh_cot, m);
+            const float f = ax[0].w[r & 1] * ax[1].w[r >> 1];
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                t[0] = fmaf(m[0][k], v[k], t[0]);
+                t[1] = fmaf(m[1][k], v[k], t[1]);
+                g[k] = fmaf(f, fmaf(m[1][k], ax[2].w[1], m[0][k] * ax[2].w[0]), g[k]);
+            }
+            cic_grad(ax, r, t, c);
+        }
+        if (val_cot) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k) val_cot[q * NC + k] = g[k];
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) disp_cot[3 * q + a] = div_or_mul(c[a], p.div, p.div_inv);
+    }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_gather_cic(Cic p, const int16_t *__restrict__ pmid,
+                                                    const float *__restrict__ disp, int64_t n,
+                                                    const float *__restrict__ mesh,
+                                                    const float *__restrict__ val,
+                                                    float val_scalar, float *out) {
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        CicAxis ax[3];
+        float v[NC], g[NC] = {};
+        cic_axes(p, pmid, disp, q, ax);
+        ld_val<NC>(val, val_scalar, q, v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float m[2][NC];
+            cic_read<NC>(p, ax, r, mesh, m);
+            const float f = ax[0].w[r & 1] * ax[1].w[r >> 1];
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                g[k] = fmaf(f, fmaf(m[1][k], ax[2].w[1], m[0][k] * ax[2].w[0]), g[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < NC; ++k) out[q * NC + k] = __fadd_rn(v[k], g[k]);
+    }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_gather_adj_cic(Cic p, const int16_t *__restrict__ pmid,
+                                                        const float *__restrict__ disp, int64_t n,
+                                                        const float *__restrict__ mesh,
+                                                        const float *__restrict__ val_cot,
+                                                        float *disp_cot, float *mesh_cot) {
+    for (int64_t q0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); q0 < n;
+         q0 += (int64_t)gridDim.x * blockDim.x) {   // warp-uniform
+        const int64_t q = q0 + (threadIdx.x & 31);
+        CicAxis ax[3] = {};
+        float v[NC] = {};
+        if (q < n) {
+            float c[3] = {0.f, 0.f, 0.f};
+            cic_axes(p, pmid, disp, q, ax);
+            ld_val<NC>(val_cot, 0.f, q, v);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                float m[2][NC], t[2] = {0.f, 0.f};
+                cic_read<NC>(p, ax, r, mesh, m);
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    t[0] = fmaf(m[0][k], v[k], t[0]);
+                    t[1] = fmaf(m[1][k], v[k], t[1]);
+                }
+                cic_grad(ax, r, t, c);
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a) disp_cot[3 * q + a] = div_or_mul(c[a], p.div, p.div_inv);
+        }
+        cic_add<NC>(p, q < n, ax, v, mesh_cot);
+    }
+}
+
+// Whether the k_*_cic kernels cover this enmesh: 3-D, the default branch,
+// periodic, every wrapped neighbour inside the mesh array, 32-bit offsets.
+// mesh is the array that is added to (NULL: only read), n particles.
+static bool cic_params(const EmParams &e, int64_t chan, int64_t n, const float *mesh, Cic *p) {
+    if (e.dim != 3 || e.f64 || (chan != 1 && chan != 3)) return false;
+    for (int a = 0; a < 3; ++a)
+        if (e.wrap[a] <= 0 || e.shape[a] < e.wrap[a]) return false;
+    if (e.stride[0] * chan >= (int64_t)1 << 32) return false;
+    for (int a = 0; a < 3; ++a) {
+        p->wrap[a] = e.wrap[a];
+        p->i12[a] = e.i12[a];
+        p->d12[a] = e.d12[a];
+    }
+    p->cell = e.cellf;
+    p->inv = e.cell_inv;
+    p->div = e.cot_div;
+    p->div_inv = exact_inverse(e.cot_div);
+    p->s0 = e.stride[0];
+    p->s1 = (unsigned)e.stride[1];
+    p->join = (int64_t)e.wrap[0] * e.wrap[1] * e.wrap[2] < 4 * n;
+    p->pair = (uintptr_t)mesh % 8 == 0;
+    return true;
+}
+
+// Blocks of a particle kernel: one particle per thread.  Short blocks are
+// replaced as they end, where a few long ones hold their share of the particles
+// up behind contended reductions.
+static int ptcl_blocks(int64_t n, int threads) {
+    const int64_t g = (n + threads - 1) / threads;
+    return (int)(g < (1 << 30) ? g : 1 << 30);
+}
+
 }  // namespace pmx
 
 using namespace pmx;
@@ -341,8 +651,13 @@ extern "C" int pmx_scatter(const pmx_enmesh_spec *spec, const int16_t *pmid, con
     if (!mesh) return fail(PMX_ERR_ARG, "null mesh");
     if (n == 0) return PMX_OK;
     const int T = 256;
-    k_scatter<<<stride_grid(n, T), T, 0, as_stream(stream)>>>(p, pmid, disp, n, val, val_scalar,
-                                                              channels, mesh);
+    Cic q;
+    if (cic_params(p, channels, n, mesh, &q))
+        (channels == 1 ? k_scatter_cic<1> : k_scatter_cic<3>)
+            <<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(q, pmid, disp, n, val, val_scalar, mesh);
+    else
+        k_scatter<<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(p, pmid, disp, n, val, val_scalar,
+                                                                  channels, mesh);
     PMX_LAUNCH_CHECK("k_scatter");
     return PMX_OK;
 }
@@ -359,8 +674,14 @@ extern "C" int pmx_scatter_adj(const pmx_enmesh_spec *spec, const int16_t *pmid,
     if (!mesh_cot || (n > 0 && !disp_cot)) return fail(PMX_ERR_ARG, "null mesh_cot/disp_cot");
     if (n == 0) return PMX_OK;
     const int T = 256;
-    k_scatter_adj<<<stride_grid(n, T), T, 0, as_stream(stream)>>>(
-        p, pmid, disp, n, val, val_scalar, channels, mesh_cot, disp_cot, val_cot);
+    Cic q;
+    if (cic_params(p, channels, n, nullptr, &q))
+        (channels == 1 ? k_scatter_adj_cic<1> : k_scatter_adj_cic<3>)
+            <<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(q, pmid, disp, n, val, val_scalar,
+                                                             mesh_cot, disp_cot, val_cot);
+    else
+        k_scatter_adj<<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(
+            p, pmid, disp, n, val, val_scalar, channels, mesh_cot, disp_cot, val_cot);
     PMX_LAUNCH_CHECK("k_scatter_adj");
     return PMX_OK;
 }
@@ -375,8 +696,14 @@ extern "C" int pmx_gather(const pmx_enmesh_spec *spec, const int16_t *pmid, cons
     if (!mesh || (n > 0 && !out)) return fail(PMX_ERR_ARG, "null mesh/out");
     if (n == 0) return PMX_OK;
     const int T = 256;
-    k_gather<<<stride_grid(n, T), T, 0, as_stream(stream)>>>(p, pmid, disp, n, mesh, channels,
-                                                             val, val_scalar, out);
+    Cic q;
+    if (cic_params(p, channels, n, nullptr, &q))
+        (channels == 1 ? k_gather_cic<1> : k_gather_cic<3>)
+            <<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(q, pmid, disp, n, mesh, val, val_scalar,
+                                                             out);
+    else
+        k_gather<<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(p, pmid, disp, n, mesh, channels,
+                                                                 val, val_scalar, out);
     PMX_LAUNCH_CHECK("k_gather");
     return PMX_OK;
 }
@@ -393,8 +720,14 @@ extern "C" int pmx_gather_adj(const pmx_enmesh_spec *spec, const int16_t *pmid,
         return fail(PMX_ERR_ARG, "null mesh/mesh_cot/val_cot/disp_cot");
     if (n == 0) return PMX_OK;
     const int T = 256;
-    k_gather_adj<<<stride_grid(n, T), T, 0, as_stream(stream)>>>(
-        p, pmid, disp, n, mesh, channels, val_cot, disp_cot, mesh_cot);
+    Cic q;
+    if (cic_params(p, channels, n, mesh_cot, &q))
+        (channels == 1 ? k_gather_adj_cic<1> : k_gather_adj_cic<3>)
+            <<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(q, pmid, disp, n, mesh, val_cot,
+                                                             disp_cot, mesh_cot);
+    else
+        k_gather_adj<<<ptcl_blocks(n, T), T, 0, as_stream(stream)>>>(
+            p, pmid, disp, n, mesh, channels, val_cot, disp_cot, mesh_cot);
     PMX_LAUNCH_CHECK("k_gather_adj");
     return PMX_OK;
 }

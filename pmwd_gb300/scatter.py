@@ -33,24 +33,29 @@ class _ScatterFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, disp, mesh, val, pmid, conf, offset, cell_size, val_is_default):
         n, dim = pmid.shape
-        chan_shape = tuple(mesh.shape[dim:])
+        if mesh is None:   # a fresh mesh of zeros: nothing to copy
+            vshape = tuple(val.shape[1:]) if torch.is_tensor(val) and val.ndim > 0 else ()
+            out = torch.zeros(tuple(conf.mesh_shape) + vshape, dtype=torch.float32,
+                              device=disp.device)
+        else:
+            out = mesh.to(torch.float32).contiguous().clone()
+        chan_shape = tuple(out.shape[dim:])
         chan = 1
         for c in chan_shape:
             chan *= c
         vt, vs = _val_args(val, n, chan_shape, disp.device)
-        out = mesh.to(torch.float32).contiguous().clone()
-        spec = _spec(conf, dim, mesh.shape[:dim], offset, cell_size)
+        spec = _spec(conf, dim, out.shape[:dim], offset, cell_size)
         _lib.call('pmx_scatter', spec, _lib.ptr(pmid), _lib.ptr(disp), n, _lib.ptr(vt), vs, chan,
                   _lib.ptr(out), _lib.stream_ptr(disp.device))
         ctx.save_for_backward(pmid, disp, vt)
         ctx.meta = (conf, offset, cell_size, vs, chan, chan_shape, dim,
-                    torch.is_tensor(val) and val.ndim == 0)
+                    torch.is_tensor(val) and val.ndim == 0, mesh is None)
         return out
 
     @staticmethod
     def backward(ctx, mesh_cot):
         pmid, disp, vt = ctx.saved_tensors
-        conf, offset, cell_size, vs, chan, chan_shape, dim, val0d = ctx.meta
+        conf, offset, cell_size, vs, chan, chan_shape, dim, val0d, fresh = ctx.meta
         n = pmid.shape[0]
         mesh_cot = mesh_cot.to(torch.float32).contiguous()
         disp_cot = torch.empty_like(disp)
@@ -62,7 +67,7 @@ class _ScatterFn(torch.autograd.Function):
                   _lib.stream_ptr(disp.device))
         if need_val:
             val_cot = val_cot.sum() if val0d else val_cot.reshape((n,) + chan_shape)
-        return disp_cot, mesh_cot, val_cot, None, None, None, None, None
+        return disp_cot, None if fresh else mesh_cot, val_cot, None, None, None, None, None
 
 
 def scatter(ptcl, conf, mesh=None, val=None, offset=0, cell_size=None):
@@ -77,9 +82,5 @@ def scatter(ptcl, conf, mesh=None, val=None, offset=0, cell_size=None):
     default = val is None
     if default:
         val = conf.mesh_size / conf.ptcl_num
-    if mesh is None:
-        vshape = tuple(val.shape[1:]) if torch.is_tensor(val) and val.ndim > 0 else ()
-        mesh = torch.zeros(tuple(conf.mesh_shape) + vshape, dtype=torch.float32,
-                           device=disp.device)
     return _ScatterFn.apply(disp.contiguous(), mesh, val, pmid.contiguous(), conf, offset,
                             cell_size, default)
