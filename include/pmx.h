@@ -387,6 +387,22 @@ int pmx_powspec_bin_zmajor(const float *F, const float *G, int64_t nbatch,
                            int32_t nedges, int32_t right, int32_t nbin, double deconv,
                            double *ksum, double *psum, double *nsum, void *stream);
 
+/* pmx_powspec_bin of any grid in either layout: half_major = 0 as
+ * pmx_powspec_bin, else as pmx_powspec_bin_zmajor.  scratch: 8-byte aligned
+ * device memory of pmx_powspec_scratch_bytes(grid_shape, nedges, nbin,
+ * deconv != 0, ksum != NULL, half_major) bytes (0: bad arguments), in use until
+ * the stream is past this call; NULL: stream-ordered scratch of its own. */
+int64_t pmx_powspec_scratch_bytes(const int64_t grid_shape[3], int32_t nedges,
+                                  int32_t nbin, int32_t deconv, int32_t sums,
+                                  int32_t half_major);
+int pmx_powspec_bin_layout(const float *F, const float *G, int64_t nbatch,
+                           const int64_t grid_shape[3], const double *kx,
+                           const double *ky, const double *kz,
+                           const double *edges, int32_t nedges, int32_t right,
+                           int32_t nbin, double deconv, double *ksum,
+                           double *psum, double *nsum, int32_t half_major,
+                           void *scratch, void *stream);
+
 /* --------------------------------------------------------------------------
  * White noise (pmwd/modes.py:12-49 ``white_noise``)
  * ------------------------------------------------------------------------ */

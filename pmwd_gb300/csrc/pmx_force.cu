@@ -441,18 +441,6 @@ __device__ __forceinline__ float3 kahan_axpy(float3 y, float3 x, float a, float 
     return t;
 }
 
-// (double)x: the exponent rebiased and the mantissa shifted by integer
-// operations for normal numbers.  The float64 unit, which also converts, runs
-// at about two operations per clock and SM here: dot products of six
-// conversions and four operations held up the kick/drift adjoint passes (256^3
-// particles on 256^3: 0.68 against 0.63 ms with these three operations).
-__device__ __forceinline__ double to_f64(float x) {
-    const unsigned u = __float_as_uint(x), e = u & 0x7f800000u;
-    if (e == 0u || e == 0x7f800000u) return (double)x;   // zero, subnormal, inf, NaN
-    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)),
-                            (int)(u << 29));
-}
-
 // s + a . b
 __device__ __forceinline__ double dot3d(float3 a, float3 b, double s) {
     return fma(to_f64(a.x), to_f64(b.x), fma(to_f64(a.y), to_f64(b.y), fma(to_f64(a.z), to_f64(b.z), s)));

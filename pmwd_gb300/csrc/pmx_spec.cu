@@ -7,13 +7,15 @@
 // wavenumber tables in the reference's order ((kx^2 + ky^2) + kz^2), the bin
 // with numpy digitize semantics, P in float64 (|F|^2 from the widened parts,
 // or F conj(G) formed in complex64 and widened, as the reference does), the
-// optional sinc^-deconv window, and accumulates k N, P N and N per bin:
-// warp shuffle sums per distinct bin, then shared-memory float64 sums merged
-// once per block.
+// optional sinc^-deconv window, and accumulates k N, P N and N per bin: sums of
+// each thread's run of cells, then shared-memory float64 sums merged once per
+// block.
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
+#include <climits>
 
 #include "pmx_internal.cuh"
 
@@ -46,9 +48,9 @@ struct SpecArgs {
     int64_t nb, n0, n1, n2h, Mc;
     int nyq_z;                    // 1: the last z index is the Nyquist plane (even n2)
     const double *kx, *ky, *kz;   // cycles per sample (fftfreq / rfftfreq)
-    const double *edges;
-    int ne, right, nbin;
-    double deconv;                // 0: none
+    const long long *keys;        // k_edge_keys
+    int ne, nbin;
+    const double *wx, *wy, *wz;   // sinc^-deconv per axis, or NULL
     double *ksum, *psum, *nsum;   // nbin, 2 nbin (re, im), nbin
 };
 
@@ -58,11 +60,57 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Each warp takes 32 consecutive cells (mostly one or two bins: |k| varies
-// slowly along a row), sums its lanes per distinct bin with shuffles, and
-// one lane adds each bin's sums to the block's shared accumulators (SH) or
-// to global memory.
-template <bool SH>
+// The order of nonnegative doubles is that of their bits.  keys[b] is the
+// smallest s with sqrt(s) beyond edge b (sqrt(s) >= e, or > e with right): |k| is
+// beyond the edge exactly where |k|^2 >= keys[b], rounding of the root included.
+__global__ void k_edge_keys(const double *edges, int ne, int right, long long *keys) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= ne) return;
+    const double e = edges[b];
+    auto beyond = [&](long long s) {
+        const double k = sqrt(__longlong_as_double(s));
+        return right ? k > e : k >= e;
+    };
+    const long long inf = 0x7ff0000000000000ll;
+    long long s = LLONG_MAX;   // e NaN, or its square above every float64
+    if (e < 0.0 || (e == 0.0 && !right)) {
+        s = 0;
+    } else if (e * e < __longlong_as_double(inf)) {
+        s = __double_as_longlong(e * e);
+        // the square and the root round: a few steps either way
+        for (int i = 0; i < 8 && s > 0 && beyond(s - 1); ++i) --s;
+        for (int i = 0; i < 8 && s < inf && !beyond(s); ++i) ++s;
+    }
+    keys[b] = s;
+}
+
+// Root of s >= 0 by Heron steps k + (s - k^2) / (2 k) from the float32 unit's
+// reciprocal root: two steps leave the rounding of the last one.
+__device__ __forceinline__ double root(double s) {
+    const unsigned hi = (unsigned)__double2hiint(s);
+    if (hi < 0x3c900000u || hi >= 0x43000000u) return sqrt(s);   // outside 2^-54 .. 2^49
+    // s truncated to float32, by the exponent and the upper mantissa bits
+    const float f = __uint_as_float(((hi - 0x38000000u) << 3) |
+                                    ((unsigned)__double2loint(s) >> 29));
+    const float r = rsqrtf(f);
+    const double h = to_f64(0.5f * r);
+    double k = to_f64(f * r);
+    k = fma(fma(-k, k, s), h, k);
+    return fma(fma(-k, k, s), h, k);
+}
+
+// A warp takes consecutive rows, (x, y) along kz or with ZM (kz, x) along y, and
+// each lane a contiguous run of their cells: the lane keeps the sums of its
+// current bin in registers, steps through the edges as |k| passes them, and adds
+// its sums to the block's shared accumulators (SH) or to global memory when the
+// bin changes.  The float64 unit is the bound (one to two operations per clock
+// and SM), so x and y run over half their indices only: the up to four cells at
+// +-kx, +-ky have one |k|, root, bin and window.  Bins come from integer
+// comparisons, the windows (three powers of sines per cell before) from tables
+// per axis, and the multiplicity 2 from one doubling per flush.  462^3, log bins:
+// 0.99 ms (5.2 with a binary search, a root and two widened products per cell);
+// 347^3, bins of the fundamental width, window: 0.53 (27).
+template <bool SH, bool ZM>
 __global__ void __launch_bounds__(ST) k_powspec(SpecArgs a) {
     extern __shared__ double sb[];  // SH: 4 doubles per bin (k N, P_re N, P_im N, N)
     if (SH) {
@@ -70,71 +118,99 @@ __global__ void __launch_bounds__(ST) k_powspec(SpecArgs a) {
         __syncthreads();
     }
     const int lane = threadIdx.x & 31;
-    for (int64_t c0 = blockIdx.x * (int64_t)ST + (threadIdx.x & ~31); c0 < a.Mc;
-         c0 += (int64_t)gridDim.x * ST) {  // warp-uniform
-        const int64_t c = c0 + lane;
-        int b = a.nbin;  // "no bin"
-        double kn = 0.0, prn = 0.0, pin = 0.0, N = 0.0;
-        if (c < a.Mc) {
-            const int64_t l = c % a.n2h, r = c / a.n2h;
-            const int64_t j = r % a.n1, i = r / a.n1;
-            const double kxi = a.kx[i], kyj = a.ky[j], kzl = a.kz[l];
-            const double k = sqrt(
-                __dadd_rn(__dadd_rn(__dmul_rn(kxi, kxi), __dmul_rn(kyj, kyj)), __dmul_rn(kzl, kzl)));
-            b = digitize(k, a.edges, a.ne, a.right);
-            if (b < a.nbin) {
-                N = (l == 0 || (a.nyq_z && l == a.n2h - 1)) ? 1.0 : 2.0;
-                double pr = 0.0, pi = 0.0;
+    const int n0 = (int)a.n0, n1 = (int)a.n1, n2h = (int)a.n2h;
+    const int m0 = n0 / 2 + 1, m1 = n1 / 2 + 1, len = ZM ? m1 : n2h;
+    const int64_t rows = (int64_t)m0 * (ZM ? n2h : m1), nw = (int64_t)gridDim.x * (ST / 32);
+    const int run = (len + 31) / 32, c0 = lane * run, c1 = c0 + run < len ? c0 + run : len;
+    const int64_t per = (rows + nw - 1) / nw;
+    const int64_t r0 = ((int64_t)blockIdx.x * (ST / 32) + (threadIdx.x >> 5)) * per;
+    const int64_t r1 = r0 + per < rows ? r0 + per : rows;
+    double sk = 0.0, sp = 0.0, si = 0.0;   // half the sums of k N, P N
+    int cnt = 0, b = -1;
+    long long lo = 0, hi = -1;             // keys of bin b's lower edge and of the next
+    auto flush = [&]() {
+        if (cnt == 0) return;
+        double *k = SH ? sb + 4 * b : a.ksum + b, *p = SH ? sb + 4 * b + 1 : a.psum + 2 * b;
+        atomicAdd(k, sk + sk);
+        atomicAdd(p, sp + sp);
+        if (a.G) atomicAdd(p + 1, si + si);
+        atomicAdd(SH ? sb + 4 * b + 3 : a.nsum + b, (double)cnt);
+        sk = sp = si = 0.0;
+        cnt = 0;
+    };
+    for (int64_t row = r0; row < r1; ++row) {
+        const int jl = (int)(row / m0), i = (int)(row - (int64_t)jl * m0);   // ky or kz; x
+        const int i2 = n0 - i;
+        const bool xx = i > 0 && i2 > i;   // -kx is another cell
+        const double kx = a.kx[i], kr = ZM ? a.kz[jl] : a.ky[jl];
+        const double kx2 = __dmul_rn(kx, kx), kr2 = __dmul_rn(kr, kr);
+        const double kxy = ZM ? kx2 : __dadd_rn(kx2, kr2);
+        const double wr = a.wx ? ZM ? a.wx[i] : a.wx[i] * a.wy[jl] : 1.0;
+        for (int c = c0; c < c1; ++c) {
+            const int j = ZM ? c : jl, l = ZM ? jl : c, j2 = n1 - j;
+            const bool yy = j > 0 && j2 > j;
+            const double kc = (ZM ? a.ky : a.kz)[c];
+            double s = __dadd_rn(kxy, __dmul_rn(kc, kc));   // (kx^2 + ky^2) + kz^2
+            if (ZM) s = __dadd_rn(s, kr2);
+            const long long key = __double_as_longlong(s);
+            if (key >= hi || key < lo) {
+                flush();
+                if (b < 0) {
+                    int e = 0, h = a.ne;   // numpy.digitize
+                    while (e < h) {
+                        const int mid = (e + h) >> 1;
+                        if (a.keys[mid] <= key) e = mid + 1;
+                        else h = mid;
+                    }
+                    b = e;
+                }
+                while (b < a.ne && key >= a.keys[b]) ++b;
+                while (b > 0 && key < a.keys[b - 1]) --b;
+                lo = b > 0 ? a.keys[b - 1] : LLONG_MIN;
+                hi = b < a.ne ? a.keys[b] : LLONG_MAX;
+            }
+            if (b >= a.nbin) continue;
+            double pr = 0.0, pi = 0.0;
+            auto add = [&](int x, int y) {
+                const int64_t at = ZM ? ((int64_t)l * n0 + x) * n1 + y
+                                      : ((int64_t)x * n1 + y) * n2h + l;
                 for (int64_t t = 0; t < a.nb; ++t) {
-                    const float2 f = a.F[t * a.Mc + c];
+                    const float2 f = a.F[t * a.Mc + at];
                     if (a.G) {
-                        const float2 gg = a.G[t * a.Mc + c];
+                        const float2 gg = a.G[t * a.Mc + at];
                         // F * conj(G) in complex64, then widened
-                        pr += (double)__fadd_rn(__fmul_rn(f.x, gg.x), __fmul_rn(f.y, gg.y));
-                        pi += (double)__fsub_rn(__fmul_rn(f.y, gg.x), __fmul_rn(f.x, gg.y));
+                        pr += to_f64(__fadd_rn(__fmul_rn(f.x, gg.x), __fmul_rn(f.y, gg.y)));
+                        pi += to_f64(__fsub_rn(__fmul_rn(f.y, gg.x), __fmul_rn(f.x, gg.y)));
                     } else {
-                        pr += __dadd_rn(__dmul_rn((double)f.x, (double)f.x),
-                                        __dmul_rn((double)f.y, (double)f.y));
+                        const double x = to_f64(f.x), y = to_f64(f.y);
+                        pr = fma(y, y, fma(x, x, pr));
                     }
                 }
-                if (a.deconv != 0.0) {
-                    const double w = pow(sincd(kxi), -a.deconv) * pow(sincd(kyj), -a.deconv) *
-                                     pow(sincd(kzl), -a.deconv);
-                    pr *= w;
-                    pi *= w;
-                }
-                kn = k * N;
-                prn = pr * N;
-                pin = pi * N;
-            } else {
-                b = a.nbin;
+            };
+            add(i, j);
+            if (xx) add(i2, j);
+            if (yy) add(i, j2);
+            if (xx && yy) add(i2, j2);
+            if (a.wx) {
+                const double w = ZM ? (wr * a.wy[c]) * a.wz[jl] : wr * a.wz[c];
+                pr *= w;
+                pi *= w;
             }
-        }
-        // per distinct bin of the warp: shuffle sums, one add
-        unsigned pending = __ballot_sync(0xffffffffu, b < a.nbin);
-        while (pending) {
-            const int src = __ffs(pending) - 1;
-            const int bb = __shfl_sync(0xffffffffu, b, src);
-            const bool mine = b == bb;
-            const double s0 = warp_sum(mine ? kn : 0.0), s1 = warp_sum(mine ? prn : 0.0);
-            const double s2 = a.G ? warp_sum(mine ? pin : 0.0) : 0.0;
-            const double s3 = warp_sum(mine ? N : 0.0);
-            if (lane == src) {
-                if (SH) {
-                    atomicAdd(sb + 4 * bb, s0);
-                    atomicAdd(sb + 4 * bb + 1, s1);
-                    if (a.G) atomicAdd(sb + 4 * bb + 2, s2);
-                    atomicAdd(sb + 4 * bb + 3, s3);
-                } else {
-                    atomicAdd(a.ksum + bb, s0);
-                    atomicAdd(a.psum + 2 * bb, s1);
-                    if (a.G) atomicAdd(a.psum + 2 * bb + 1, s2);
-                    atomicAdd(a.nsum + bb, s3);
-                }
+            const double k = root(s);
+            const int cells = (xx ? 2 : 1) * (yy ? 2 : 1);
+            const bool one = l == 0 || (a.nyq_z && l == n2h - 1);
+            if (one) {
+                pr *= 0.5;
+                pi *= 0.5;
             }
-            pending &= ~__ballot_sync(0xffffffffu, mine);
+            const int N = one ? cells : 2 * cells;
+            sk = fma(k, 0.5 * N, sk);
+            sp += pr;
+            if (a.G) si += pi;
+            cnt += N;
         }
     }
+    flush();
     if (SH) {
         __syncthreads();
         for (int b = threadIdx.x; b < a.nbin; b += ST) {
@@ -169,6 +245,7 @@ struct Pow2Args {
     int h0, h1;                    // n0, n1 (signed index: i' = i <= n/2 ? i : i - n)
     const double *ktab;            // k(m)
     const int *btab;               // bin(m), nbin = none
+    const int *thr;                // k_thresholds, instead of bin(m)
     const float *wx, *wy, *wz;     // sinc^-deconv per axis, or NULL
     int nbin;
     int zm;                        // 1: layout (n2h, n0, n1), y contiguous
@@ -181,6 +258,7 @@ __global__ void k_pow2_tables(int64_t mmax, double D, const double *edges, int n
          m += (int64_t)gridDim.x * blockDim.x) {
         const double k = sqrt((double)m / D);  // exact quotient (D a power of two)
         ktab[m] = k;
+        if (!btab) continue;
         const int b = digitize(k, edges, ne, right);
         btab[m] = b < nbin ? b : nbin;
     }
@@ -350,119 +428,152 @@ __global__ void __launch_bounds__(ST, 6) k_powspec_rows(Pow2Args a) {
     }
 }
 
-// Half-axis-major spectra with n1 a multiple of 32: the warp takes row
-// (kz, x) and lane r walks the contiguous run y in [r n1/32, (r+1) n1/32),
-// keeping the sums of its current bin in registers.  The bins are shells in
-// |k|, so a run changes bin rarely: then the lane adds its sums to the bin
-// array, and at the end of the row the lanes holding the same bin are
-// merged by shuffles and added once.  Every shared-memory add is atomic.
-template <bool CROSS, bool GEOM, bool WIN, bool PRIV>
+// Half-axis-major spectra with n1 a multiple of 32.  A warp takes units of up to
+// 512 consecutive y cells of a row (kz, x), stages them in shared memory with
+// coalesced loads, and lane r walks the run of R = cells / 32 cells from r R,
+// keeping the sums of its current bin in registers until the bin changes, across
+// units too.  The bins are shells in |k|, hence intervals [T[b], T[b+1]) of the
+// integer m: comparing m with the current interval's ends replaces a table
+// lookup per cell.  512^3, log bins, window: 0.32 ms (0.59 with each lane reading
+// its run from global memory, a bin lookup and a float64 addition per cell);
+// reading the spectrum alone takes 0.08, the rest is instructions and the wait
+// for the next unit's loads.
+constexpr int UNIT = 512;
+
+template <bool CROSS, bool GEOM, bool WIN, bool PRIV, bool ONE>
 __global__ void __launch_bounds__(ST, 6) k_powspec_runs(Pow2Args a) {
-    extern __shared__ double sbase[];  // 4 doubles per bin (per warp with PRIV)
-    const int nacc = (PRIV ? ST / 32 : 1) * 4 * a.nbin;
-    for (int i = threadIdx.x; i < nacc; i += ST) sbase[i] = 0.0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    double *sb = PRIV ? sbase + (threadIdx.x >> 5) * 4 * a.nbin : sbase;
+    extern __shared__ double sbase[];  // 4 doubles per bin (per warp with PRIV), then T and the rows
+    const int nbin = a.nbin, nacc = (PRIV ? ST / 32 : 1) * 4 * nbin;
+    int *T = reinterpret_cast<int *>(sbase + nacc);
     const int n2h = (int)a.n2h, n0 = (int)a.n0, n1 = (int)a.n1, h0 = a.h0, h1 = a.h1;
-    const int ax = (int)a.ax, ay = (int)a.ay, az = (int)a.az, nbin = a.nbin;
-    const int R = n1 / 32, nrows = n2h * n0;
-    const int wstride = gridDim.x * (ST / 32);
-    auto add = [&](int b, double pr, double pi, double kn, double nn) {
-        atomicAdd(sb + 4 * b + 1, pr);
-        if (CROSS) atomicAdd(sb + 4 * b + 2, pi);
-        if (GEOM) {
-            atomicAdd(sb + 4 * b, kn);
-            atomicAdd(sb + 4 * b + 3, nn);
-        }
+    const int cells = n1 < UNIT ? n1 : UNIT, R = cells / 32, U = n1 / cells;
+    const int rsh = __ffs(R) - 1, rowlen = cells + 32;   // one pad per run
+    float *rows = reinterpret_cast<float *>(T + ((nbin + 2 + 3) & ~3));
+    for (int i = threadIdx.x; i < nacc; i += ST) sbase[i] = 0.0;
+    for (int i = threadIdx.x; i < nbin + 2; i += ST) T[i] = a.thr[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *sb = PRIV ? sbase + warp * 4 * nbin : sbase;
+    float *Ps = rows + warp * (CROSS ? 2 : 1) * rowlen, *Qs = Ps + rowlen;   // P N: re, im
+    const int ax = (int)a.ax, ay = (int)a.ay, az = (int)a.az;
+    // consecutive units per warp, so that a lane's bin hardly moves between them
+    const int64_t units = (int64_t)n2h * n0 * U, nw = (int64_t)gridDim.x * (ST / 32);
+    const int64_t per = (units + nw - 1) / nw, w = (int64_t)blockIdx.x * (ST / 32) + warp;
+    const int64_t u0 = w * per, u1 = u0 + per < units ? u0 + per : units;
+    int cur = 0, lo = T[0];
+    unsigned width = (unsigned)(T[1] - lo);
+    double ar = 0.0, ai = 0.0, ak = 0.0;
+    int an = 0;
+    // A bin's cells within a run: float32 sums with the rounding errors of their
+    // additions summed beside, some 2^-46 of the sum, in place of a float64
+    // addition per cell (about 30 clocks of the float64 unit per warp).
+    float gr = 0.f, er = 0.f, gi = 0.f, ei = 0.f;
+    auto add2 = [](float &s, float &e, float p) {
+        const float t = __fadd_rn(s, p), q = __fsub_rn(t, s);
+        e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, q)), __fsub_rn(p, q)));
+        s = t;
     };
-    for (int row = blockIdx.x * (ST / 32) + (threadIdx.x >> 5); row < nrows;
-         row += wstride) {  // warp-uniform
-        const int l = row / n0, i = row - l * n0;
-        const int si = i <= h0 / 2 ? i : i - h0;
+    auto fold = [&](const float *P, const float *Q, int n) {   // the last n cells before P, Q
+        if (n == 0) return;
+        // beyond float32: cell by cell
+        if (fabsf(gr) <= FLT_MAX && fabsf(gi) <= FLT_MAX) {
+            ar += to_f64(gr) + to_f64(er);
+            if (CROSS) ai += to_f64(gi) + to_f64(ei);
+        } else {
+            for (int c = -n; c < 0; ++c) {
+                ar += (double)P[c];
+                if (CROSS) ai += (double)Q[c];
+            }
+        }
+        gr = er = gi = ei = 0.f;
+    };
+    auto flush = [&]() {
+        if (cur < nbin) {
+            atomicAdd(sb + 4 * cur + 1, ar);
+            if (CROSS) atomicAdd(sb + 4 * cur + 2, ai);
+            if (GEOM) {
+                atomicAdd(sb + 4 * cur, ak);
+                atomicAdd(sb + 4 * cur + 3, (double)an);
+            }
+        }
+        ar = ai = ak = 0.0;
+        an = 0;
+    };
+    for (int64_t u = u0; u < u1; ++u) {
+        const int row = (int)(u / U), sub = (int)(u - (int64_t)row * U);
+        const int l = row / n0, i = row - l * n0, si = i <= h0 / 2 ? i : i - h0;
         const int mrow = si * si * ax + l * l * az;
         const bool two = !(l == 0 || (a.nyq_z && l == n2h - 1));
-        const int j0 = lane * R;
-        const float2 *Fr = a.F + (int64_t)row * n1 + j0;
-        const float2 *Gr = CROSS ? a.G + (int64_t)row * n1 + j0 : nullptr;
-        int cur = nbin;
-        // a run holds up to n1/32 cells: its sums are float64, so a long
-        // run rounds like the row kernel's per-32-cell float sums
-        double ar = 0.0, ai = 0.0, ak = 0.0, an = 0.0;
-        for (int r = 0; r < R; ++r) {
-            const int j = j0 + r;
-            const int sj = j <= h1 / 2 ? j : j - h1;
-            const int m = mrow + sj * sj * ay;
-            const int b = a.btab[m];
-            if (b != cur) {
-                if (cur < nbin) add(cur, ar, ai, ak, an);
-                cur = b;
-                ar = ai = ak = an = 0.0;
+        const float wxi = WIN ? a.wx[i] : 1.f, wzl = WIN ? a.wz[l] : 1.f;
+        const int64_t base = (int64_t)row * n1 + sub * cells;
+        __syncwarp();   // the previous unit's reads
+#pragma unroll 4
+        for (int c = lane; c < cells; c += 32) {
+            float pr = 0.f, pi = 0.f;
+            const float2 *Fc = a.F + base + c, *Gc = CROSS ? a.G + base + c : nullptr;
+            int64_t t = a.nb;
+            do {
+                const float2 f = *Fc;
+                if (CROSS) {
+                    const float2 gg = *Gc;
+                    pr += __fadd_rn(__fmul_rn(f.x, gg.x), __fmul_rn(f.y, gg.y));
+                    pi += __fsub_rn(__fmul_rn(f.y, gg.x), __fmul_rn(f.x, gg.y));
+                    Gc += a.Mc;
+                } else {
+                    pr += fmaf(f.x, f.x, f.y * f.y);
+                }
+                Fc += a.Mc;
+            } while (!ONE && --t > 0);
+            if (WIN) {  // ((P wx) wy) wz
+                const float wt = (wxi * a.wy[sub * cells + c]) * wzl;
+                pr *= wt;
+                pi *= wt;
             }
-            if (b < nbin) {
-                float pr = 0.f, pi = 0.f;
-                for (int64_t t = 0; t < a.nb; ++t) {
-                    const float2 f = Fr[t * a.Mc + r];
-                    if (CROSS) {
-                        const float2 gg = Gr[t * a.Mc + r];
-                        pr += __fadd_rn(__fmul_rn(f.x, gg.x), __fmul_rn(f.y, gg.y));
-                        pi += __fsub_rn(__fmul_rn(f.y, gg.x), __fmul_rn(f.x, gg.y));
-                    } else {
-                        pr += fmaf(f.x, f.x, f.y * f.y);
-                    }
-                }
-                if (WIN) {  // ((P wx) wy) wz
-                    const float w = (a.wx[i] * a.wy[j]) * a.wz[l];
-                    pr *= w;
-                    pi *= w;
-                }
-                if (two) {
-                    pr += pr;
-                    pi += pi;
-                }
-                ar += pr;
-                ai += pi;
-                if (GEOM) {
-                    const double k = a.ktab[m];
-                    ak += two ? k + k : k;
-                    an += two ? 2.0 : 1.0;
-                }
+            if (two) {
+                pr += pr;
+                pi += pi;
             }
+            Ps[c + (c >> rsh)] = pr;
+            if (CROSS) Qs[c + (c >> rsh)] = pi;
         }
         __syncwarp();
-        // end of row: lanes still holding sums merge per bin
-        const int b = cur;
-        const unsigned peers = __match_any_sync(0xffffffffu, b);
-        const int ndist = __popc(__ballot_sync(0xffffffffu, lane == __ffs(peers) - 1));
-        if (ndist > 4) {
-            if (b < nbin) add(b, ar, ai, ak, an);
-        } else {
-            unsigned pending = __ballot_sync(0xffffffffu, b < nbin);
-            while (pending) {
-                const int src = __ffs(pending) - 1;
-                const int bb = __shfl_sync(0xffffffffu, b, src);
-                const bool mine = b == bb;
-                const double spr = warp_sum(mine ? ar : 0.0);
-                const double spi = CROSS ? warp_sum(mine ? ai : 0.0) : 0.0;
-                double sk = 0.0, sn = 0.0;
-                if (GEOM) {
-                    sk = warp_sum(mine ? ak : 0.0);
-                    sn = warp_sum(mine ? an : 0.0);
-                }
-                if (lane == src) add(bb, spr, spi, sk, sn);
-                pending &= ~__ballot_sync(0xffffffffu, mine);
+        // R divides n1 / 2 (or is 1): |ky| rises or falls along the whole run
+        const float *P = Ps + lane * (R + 1), *Q = Qs + lane * (R + 1);
+        const int j0 = sub * cells + lane * R, up = j0 < h1 / 2 ? 1 : -1, y0 = up > 0 ? j0 : h1 - j0;
+        int m = mrow + y0 * y0 * ay, dm = (2 * up * y0 + 1) * ay, from = 0;
+#pragma unroll 4
+        for (int r = 0; r < R; ++r) {
+            if ((unsigned)(m - lo) >= width) {
+                fold(P + r, Q + r, r - from);
+                from = r;
+                flush();
+                while (m >= T[cur + 1]) ++cur;   // T[nbin + 1] is above every m
+                while (m < T[cur]) --cur;        // and T[0] below
+                lo = T[cur];
+                width = (unsigned)(T[cur + 1] - lo);
             }
+            add2(gr, er, P[r]);
+            if (CROSS) add2(gi, ei, Q[r]);
+            if (GEOM) {
+                const double k = a.ktab[m];
+                ak += two ? k + k : k;
+                an += two ? 2 : 1;
+            }
+            m += dm;
+            dm += 2 * ay;
         }
+        fold(P + R, Q + R, R - from);
     }
+    flush();
     __syncthreads();
-    for (int b = threadIdx.x; b < a.nbin; b += ST) {
+    for (int b = threadIdx.x; b < nbin; b += ST) {
         double acc[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[c] = sbase[4 * b + c];
         if (PRIV)
-            for (int w = 1; w < ST / 32; ++w)
+            for (int w2 = 1; w2 < ST / 32; ++w2)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc[c] += sbase[w * 4 * a.nbin + 4 * b + c];
+                for (int c = 0; c < 4; ++c) acc[c] += sbase[w2 * 4 * nbin + 4 * b + c];
         if (GEOM) {
             atomicAdd(a.ksum + b, acc[0]);
             atomicAdd(a.nsum + b, acc[3]);
@@ -480,18 +591,30 @@ void allow_smem(K *kern, size_t sm) {
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
 }
 
+// Blocks of ST threads that an SM holds.
+template <class K>
+int resident(K *kern, size_t sm) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, ST, sm) != cudaSuccess || n < 1)
+        n = 1;
+    return n;
+}
+
 template <bool CROSS, bool GEOM, bool PRIV>
 void launch_rows_p(const Pow2Args &p, cudaStream_t s) {
-    const size_t sm = (PRIV ? ST / 32 : 1) * 4 * (size_t)p.nbin * sizeof(double);
-    if (p.zm && p.n1 >= 32 && p.n1 % 32 == 0) {   // contiguous runs per lane
-        const int grid = stride_grid(p.n2h * p.n0 * 32, ST, 6);
-        if (p.wx) {
-            allow_smem(k_powspec_runs<CROSS, GEOM, true, PRIV>, sm);
-            k_powspec_runs<CROSS, GEOM, true, PRIV><<<grid, ST, sm, s>>>(p);
-        } else {
-            allow_smem(k_powspec_runs<CROSS, GEOM, false, PRIV>, sm);
-            k_powspec_runs<CROSS, GEOM, false, PRIV><<<grid, ST, sm, s>>>(p);
-        }
+    size_t sm = (PRIV ? ST / 32 : 1) * 4 * (size_t)p.nbin * sizeof(double);
+    if (p.thr) {   // contiguous runs per lane
+        const int64_t cells = p.n1 < UNIT ? p.n1 : UNIT;
+        sm += ((p.nbin + 2 + 3) & ~3) * sizeof(int) +
+              ST / 32 * (CROSS ? 2 : 1) * (cells + 32) * sizeof(float);
+        auto *kern = p.nb == 1 ? p.wx ? k_powspec_runs<CROSS, GEOM, true, PRIV, true>
+                                      : k_powspec_runs<CROSS, GEOM, false, PRIV, true>
+                               : p.wx ? k_powspec_runs<CROSS, GEOM, true, PRIV, false>
+                                      : k_powspec_runs<CROSS, GEOM, false, PRIV, false>;
+        allow_smem(kern, sm);
+        // every warp has the same share: one wave of resident blocks
+        const int grid = stride_grid(p.n2h * p.n0 * (p.n1 / cells) * 32, ST, resident(kern, sm));
+        kern<<<grid, ST, sm, s>>>(p);
         return;
     }
     const int grid = stride_grid(p.n0 * p.n1 * 32, ST, 8);
@@ -512,12 +635,81 @@ void launch_rows(const Pow2Args &p, cudaStream_t s) {
         launch_rows_p<CROSS, GEOM, false>(p, s);
 }
 
-bool is_pow2(int64_t n) { return n > 0 && (n & (n - 1)) == 0; }
+// Power-of-two grids up to 2048, for which |k|^2 has an integer form.
+bool pow2_grid(const int64_t n[3]) {
+    for (int a = 0; a < 3; ++a)
+        if (n[a] < 1 || n[a] > 2048 || (n[a] & (n[a] - 1))) return false;
+    return true;
+}
 
-__global__ void k_sinc_tab(const double *k, int64_t n, double deconv, float *w) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        w[i] = (float)pow(sincd(k[i]), -deconv);
+// sinc^-deconv of all three axes, one after the other.
+struct SincArgs {
+    const double *k[3];
+    int n[3];
+    double deconv;
+};
+template <typename T>
+__global__ void k_sinc_tab(SincArgs s, T *w) {
+    int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= s.n[0] + s.n[1] + s.n[2]) return;
+    const int o = q;
+    int a = 0;
+    for (; a < 2 && q >= s.n[a]; ++a) q -= s.n[a];
+    w[o] = (T)pow(sincd(s.k[a][q]), -s.deconv);
+}
+
+// T[b], b = 1..nbin: the smallest m <= mmax whose |k| falls into bin b or a
+// later one (INT_MAX - 1: none); T[0] and T[nbin + 1] close the list.
+__global__ void k_thresholds(int64_t mmax, double D, const double *edges, int right, int nbin,
+                             int *T) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > nbin + 1) return;
+    int t = b == 0 ? -1 : INT_MAX - 1;
+    if (b >= 1 && b <= nbin) {
+        const double e = edges[b - 1], g = floor(e * e * D) - 2.0;
+        if (e <= 0.0 || g <= (double)mmax) {
+            int64_t m = e <= 0.0 || g < 0.0 ? 0 : (int64_t)g;
+            for (; m <= mmax; ++m) {
+                const double k = sqrt((double)m / D);   // as k_pow2_tables
+                if (right ? e < k : e <= k) {
+                    t = (int)m;
+                    break;
+                }
+            }
+        }
+    }
+    T[b] = t;
+}
+
+// Scratch of one call: k(m), bin(m) or the thresholds and float32 windows of the
+// power-of-two kernels, edge keys and float64 windows of the general one.
+struct Scratch {
+    bool pow2, runs;
+    size_t k, b, w;   // bytes of each part, in this order
+    int64_t mmax;
+    size_t bytes() const { return k + b + w; }
+};
+Scratch scratch_of(const int64_t n[3], int32_t nedges, int32_t nbin, bool deconv, bool geom,
+                   bool zm) {
+    Scratch c{};
+    const int64_t n2h = n[2] / 2 + 1, nwin = deconv ? n[0] + n[1] + n2h : 0;
+    c.pow2 = pow2_grid(n) && nbin <= SMEM_BINS;
+    if (!c.pow2) {
+        c.k = (size_t)nedges * sizeof(long long);
+        c.w = (size_t)nwin * sizeof(double);
+        return c;
+    }
+    const int64_t nmax = std::max(n[0], std::max(n[1], n[2]));
+    for (int a = 0; a < 3; ++a) {
+        const int64_t m = n[a] / 2 * (nmax / n[a]);   // the highest frequency in units of 1 / nmax
+        c.mmax += m * m;
+    }
+    c.runs = zm && n[1] >= 32;
+    // the run kernel takes thresholds for bin(m), and k(m) only where it sums k N
+    c.k = !c.runs || geom ? (size_t)(c.mmax + 1) * sizeof(double) : 0;
+    c.b = (c.runs ? (size_t)nbin + 2 : (size_t)c.mmax + 1) * sizeof(int);
+    c.w = (size_t)nwin * sizeof(float);
+    return c;
 }
 
 }  // namespace
@@ -528,7 +720,8 @@ using namespace pmx;
 static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int64_t grid_shape[3],
                        const double *kx, const double *ky, const double *kz, const double *edges,
                        int32_t nedges, int32_t right, int32_t nbin, double deconv, double *ksum,
-                       double *psum, double *nsum, void *stream, bool zm) {
+                       double *psum, double *nsum, void *stream, bool zm,
+                       void *scratch = nullptr) {
     clear_error();
     if (!F || !grid_shape || !kx || !ky || !kz || !edges || !psum)
         return fail(PMX_ERR_ARG, "null argument");
@@ -549,20 +742,23 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
     a.kx = kx;
     a.ky = ky;
     a.kz = kz;
-    a.edges = edges;
     a.ne = nedges;
-    a.right = right != 0;
+    right = right != 0;
     a.nbin = nbin;
-    a.deconv = deconv;
+    a.wx = a.wy = a.wz = nullptr;
     a.ksum = ksum;
     a.psum = psum;
     a.nsum = nsum;
     cudaStream_t s = as_stream(stream);
-    const int64_t nmax = std::max(grid_shape[0], std::max(grid_shape[1], grid_shape[2]));
-    if (is_pow2(grid_shape[0]) && is_pow2(grid_shape[1]) && is_pow2(grid_shape[2]) && nmax <= 2048 &&
-        nbin <= SMEM_BINS) {
-        // tables of k(m), bin(m) and the per-axis windows: stream-ordered
-        // scratch, freed after the launch (the stream keeps them alive)
+    const int64_t nwin = deconv != 0.0 ? a.n0 + a.n1 + a.n2h : 0;
+    const Scratch sc = scratch_of(grid_shape, nedges, nbin, nwin != 0, ksum != nullptr, zm);
+    if (!sc.pow2 && !ksum)
+        return fail(PMX_ERR_ARG, "ksum/nsum may be NULL only for power-of-two grids <= 2048");
+    // without the caller's: stream-ordered, freed after the launch (the stream
+    // keeps it alive); after a synchronisation that costs some 0.1 ms
+    char *scr = static_cast<char *>(scratch);
+    if (!scr) PMX_CUDA(cudaMallocAsync((void **)&scr, sc.bytes(), s));
+    if (sc.pow2) {
         Pow2Args p;
         p.zm = zm;
         p.F = a.F;
@@ -573,34 +769,32 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
         p.n2h = a.n2h;
         p.Mc = a.Mc;
         p.nyq_z = a.nyq_z;
-        const int64_t D = nmax * nmax;
+        const int64_t nmax = std::max(grid_shape[0], std::max(grid_shape[1], grid_shape[2]));
+        const int64_t D = nmax * nmax, mmax = sc.mmax;
         p.ax = D / (grid_shape[0] * grid_shape[0]);
         p.ay = D / (grid_shape[1] * grid_shape[1]);
         p.az = D / (grid_shape[2] * grid_shape[2]);
         p.h0 = (int)grid_shape[0];
         p.h1 = (int)grid_shape[1];
-        const int64_t i0 = grid_shape[0] / 2, j0 = grid_shape[1] / 2, l0 = a.n2h - 1;
-        const int64_t mmax = i0 * i0 * p.ax + j0 * j0 * p.ay + l0 * l0 * p.az;
         p.nbin = nbin;
         p.ksum = ksum;
         p.psum = psum;
         p.nsum = nsum;
-        char *scr = nullptr;
-        const size_t tb = (size_t)(mmax + 1) * (sizeof(double) + sizeof(int));
-        const size_t wb = deconv != 0.0 ? (size_t)(a.n0 + a.n1 + a.n2h) * sizeof(float) : 0;
-        PMX_CUDA(cudaMallocAsync((void **)&scr, tb + wb, s));
         double *ktab = reinterpret_cast<double *>(scr);
-        int *btab = reinterpret_cast<int *>(scr + (size_t)(mmax + 1) * sizeof(double));
+        int *bt = reinterpret_cast<int *>(scr + sc.k);
         p.ktab = ktab;
-        p.btab = btab;
+        p.btab = sc.runs ? nullptr : bt;
+        p.thr = sc.runs ? bt : nullptr;
         p.wx = p.wy = p.wz = nullptr;
-        k_pow2_tables<<<stride_grid(mmax + 1, 256, 4), 256, 0, s>>>(mmax, (double)D, edges, nedges,
-                                                                     a.right, nbin, ktab, btab);
-        if (wb) {
-            float *w = reinterpret_cast<float *>(scr + tb);
-            k_sinc_tab<<<1, 256, 0, s>>>(kx, a.n0, deconv, w);
-            k_sinc_tab<<<1, 256, 0, s>>>(ky, a.n1, deconv, w + a.n0);
-            k_sinc_tab<<<1, 256, 0, s>>>(kz, a.n2h, deconv, w + a.n0 + a.n1);
+        if (sc.runs)
+            k_thresholds<<<(nbin + 2 + 31) / 32, 32, 0, s>>>(mmax, (double)D, edges, right, nbin, bt);
+        if (sc.k)
+            k_pow2_tables<<<stride_grid(mmax + 1, 256, 4), 256, 0, s>>>(
+                mmax, (double)D, edges, nedges, right, nbin, ktab, sc.runs ? nullptr : bt);
+        if (nwin) {
+            float *w = reinterpret_cast<float *>(scr + sc.k + sc.b);
+            k_sinc_tab<float><<<(int)((nwin + 31) / 32), 32, 0, s>>>(
+                SincArgs{{kx, ky, kz}, {(int)a.n0, (int)a.n1, (int)a.n2h}, deconv}, w);
             p.wx = w;
             p.wy = w + a.n0;
             p.wz = w + a.n0 + a.n1;
@@ -613,19 +807,28 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
             else launch_rows<false, false>(p, s);
         }
         PMX_LAUNCH_CHECK("k_powspec_rows");
-        PMX_CUDA(cudaFreeAsync(scr, s));
+        if (!scratch) PMX_CUDA(cudaFreeAsync(scr, s));
         return PMX_OK;
     }
-    if (zm) return fail(PMX_ERR_SHAPE, "the (n2h, n0, n1) layout needs a power-of-two grid <= 2048");
-    if (!ksum) return fail(PMX_ERR_ARG, "ksum/nsum may be NULL only for power-of-two grids <= 2048");
-    const int grid = stride_grid(a.Mc, ST, 4);
-    if (nbin <= SMEM_BINS) {
-        allow_smem(k_powspec<true>, 4 * nbin * sizeof(double));
-        k_powspec<true><<<grid, ST, 4 * nbin * sizeof(double), s>>>(a);
-    } else {
-        k_powspec<false><<<grid, ST, 0, s>>>(a);
+    long long *keys = reinterpret_cast<long long *>(scr);
+    k_edge_keys<<<(nedges + 63) / 64, 64, 0, s>>>(edges, nedges, right, keys);
+    a.keys = keys;
+    if (nwin) {
+        double *win = reinterpret_cast<double *>(keys + nedges);
+        k_sinc_tab<double><<<(int)((nwin + 31) / 32), 32, 0, s>>>(
+            SincArgs{{kx, ky, kz}, {(int)a.n0, (int)a.n1, (int)a.n2h}, deconv}, win);
+        a.wx = win;
+        a.wy = win + a.n0;
+        a.wz = win + a.n0 + a.n1;
     }
+    const size_t sm = nbin <= SMEM_BINS ? 4 * (size_t)nbin * sizeof(double) : 0;
+    auto *kern = sm ? zm ? k_powspec<true, true> : k_powspec<true, false>
+                    : zm ? k_powspec<false, true> : k_powspec<false, false>;
+    allow_smem(kern, sm);
+    const int grid = stride_grid((a.n0 / 2 + 1) * (zm ? a.n2h : a.n1 / 2 + 1) * 32, ST, resident(kern, sm));
+    kern<<<grid, ST, sm, s>>>(a);
     PMX_LAUNCH_CHECK("k_powspec");
+    if (!scratch) PMX_CUDA(cudaFreeAsync(scr, s));
     return PMX_OK;
 }
 
@@ -643,6 +846,30 @@ extern "C" int pmx_powspec_bin_zmajor(const float *F, const float *G, int64_t nb
                                       const double *ky, const double *kz, const double *edges,
                                       int32_t nedges, int32_t right, int32_t nbin, double deconv,
                                       double *ksum, double *psum, double *nsum, void *stream) {
+    if (grid_shape && (!pow2_grid(grid_shape) || nbin > SMEM_BINS)) {
+        clear_error();
+        return fail(PMX_ERR_SHAPE, "the (n2h, n0, n1) layout needs a power-of-two grid <= 2048");
+    }
     return powspec_bin(F, G, nbatch, grid_shape, kx, ky, kz, edges, nedges, right, nbin, deconv,
                        ksum, psum, nsum, stream, true);
+}
+
+extern "C" int pmx_powspec_bin_layout(const float *F, const float *G, int64_t nbatch,
+                                      const int64_t grid_shape[3], const double *kx,
+                                      const double *ky, const double *kz, const double *edges,
+                                      int32_t nedges, int32_t right, int32_t nbin, double deconv,
+                                      double *ksum, double *psum, double *nsum, int32_t half_major,
+                                      void *scratch, void *stream) {
+    return powspec_bin(F, G, nbatch, grid_shape, kx, ky, kz, edges, nedges, right, nbin, deconv,
+                       ksum, psum, nsum, stream, half_major != 0, scratch);
+}
+
+extern "C" int64_t pmx_powspec_scratch_bytes(const int64_t grid_shape[3], int32_t nedges,
+                                             int32_t nbin, int32_t deconv, int32_t sums,
+                                             int32_t half_major) {
+    if (!grid_shape || nedges < 1 || nbin < 1) return 0;
+    for (int a = 0; a < 3; ++a)
+        if (grid_shape[a] < 1) return 0;
+    return (int64_t)scratch_of(grid_shape, nedges, nbin, deconv != 0, sums != 0, half_major != 0)
+        .bytes();
 }

@@ -54,9 +54,10 @@ def powspec(f, spacing, bins=1j / 3, g=None, deconv=None, cut_zero=True, cut_nyq
     F = fftfwd(f, axes=(-3, -2, -1))
     if F.is_cuda and F.dtype == torch.complex64:
         G = None if g is None else fftfwd(torch.as_tensor(g, device=dev), axes=(-3, -2, -1))
-        kk, PP, NN = _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv)
-        return _finish(kk, PP, NN, edges.to(dev), bcut, cut_zero, spacing, grid_shape, dtype,
-                       g is not None)
+        tabs = _to_device(dev, *fftfreq(grid_shape, None, dtype=torch.float64), edges)
+        e = tabs[-1]
+        kk, PP, NN = _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv, tabs)
+        return _finish(kk, PP, NN, e, bcut, cut_zero, spacing, grid_shape, dtype, g is not None)
     if g is None:
         P = F.real.to(dtype) ** 2 + F.imag.to(dtype) ** 2
     else:
@@ -86,9 +87,18 @@ def powspec(f, spacing, bins=1j / 3, g=None, deconv=None, cut_zero=True, cut_nyq
     return _finish(kk, PP, NN, e, bcut, cut_zero, spacing, grid_shape, dtype, g is not None)
 
 
-def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv):
+def _to_device(dev, *arrays):
+    """float64 arrays, flattened, in one copy that the host does not wait for
+    (it would wait for the transforms too): from pinned memory, which the
+    caching allocator holds until the copy is done."""
+    host = [a.reshape(-1).to(torch.float64) for a in arrays]
+    return torch.cat(host).pin_memory().to(dev, non_blocking=True).split([len(h) for h in host])
+
+
+def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv, tabs=None):
     """One pass of the pmx_powspec_bin kernel over the complex64 spectra:
-    per-bin sums of k N, P N and N in float64."""
+    per-bin sums of k N, P N and N in float64.  tabs: the wavenumbers and edges
+    on the device, where the caller has them."""
     from . import _lib
     dev = F.device
     nb = math.prod(F.shape[:-3])
@@ -98,8 +108,8 @@ def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv):
             raise ValueError(f'shape mismatch: {G.shape} != {F.shape}')
     # torch's CUDA rfftn returns (..., n0, n1, n2h) stored half-axis major,
     # (..., n2h, n0, n1) contiguous: bin it in place instead of transposing
-    zm = (_pow2_grid(grid_shape) and bnum <= 2048
-          and not F.is_contiguous() and F.movedim(-1, -3).is_contiguous()
+    pow2 = _pow2_grid(grid_shape) and bnum <= 2048
+    zm = (not F.is_contiguous() and F.movedim(-1, -3).is_contiguous()
           and (G is None or (G.stride() == F.stride())))
     if zm:
         F = F.movedim(-1, -3)
@@ -107,26 +117,27 @@ def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv):
     else:
         F = F.contiguous()
         G = None if G is None else G.contiguous()
-    kx, ky, kz = (k.reshape(-1).contiguous() for k in
-                  fftfreq(grid_shape, None, dtype=torch.float64, device=dev))
-    e = edges.to(device=dev, dtype=torch.float64).contiguous()
+    kx, ky, kz, e = tabs or _to_device(dev, *fftfreq(grid_shape, None, dtype=torch.float64), edges)
     psum = torch.zeros(bnum, 2, dtype=torch.float64, device=dev)
     # the per-bin sums of k N and N depend on the grid and bins only: for
     # power-of-two grids they are computed on the first call and reused
     key = (dev, grid_shape, tuple(edges.tolist()), bool(right), bnum)
-    cached = _GEOMETRY.get(key) if _pow2_grid(grid_shape) else None
+    cached = _GEOMETRY.get(key) if pow2 else None
     if cached is None:
         ksum = torch.zeros(bnum, dtype=torch.float64, device=dev)
         nsum = torch.zeros(bnum, dtype=torch.float64, device=dev)
     else:
         ksum = nsum = None
     shape = (_lib.c_i64 * 3)(*grid_shape)
-    _lib.call('pmx_powspec_bin_zmajor' if zm else 'pmx_powspec_bin', torch.view_as_real(F),
+    scratch = torch.empty(_lib.load().pmx_powspec_scratch_bytes(
+        shape, len(e), bnum, int(bool(deconv)), int(cached is None), int(zm)),
+        dtype=torch.uint8, device=dev)
+    _lib.call('pmx_powspec_bin_layout', torch.view_as_real(F),
               None if G is None else torch.view_as_real(G),
               nb, shape, kx, ky, kz, e, len(e), int(right), bnum, float(deconv or 0.0), ksum, psum,
-              nsum, _lib.stream_ptr(dev))
+              nsum, int(zm), scratch, _lib.stream_ptr(dev))
     if cached is None:
-        if _pow2_grid(grid_shape):
+        if pow2:
             _GEOMETRY[key] = (ksum, nsum)
     else:
         ksum, nsum = cached[0].clone(), cached[1].clone()

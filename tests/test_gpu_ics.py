@@ -258,3 +258,40 @@ def test_lpt_statistics_match_published(cuda):
     vel_std = float(ptcl.vel.double().std())
     assert abs(disp_std / 0.105 - 1) < 0.05, disp_std
     assert abs(vel_std / 0.007 - 1) < 0.08, vel_std   # printed to one significant digit
+
+
+@pytest.mark.parametrize('shape, bins', [
+    ((5, 7, 3), 1),                # fewer rows than warps, one lane per kz cell
+    ((2, 33, 31, 130), 0.25),      # lanes carry their bin over rows, 3 cells each
+    ((12, 9, 65), 0.02),           # more bins than the shared sums hold
+    ((4, 32, 8), 1j / 3),          # run kernel: one cell per lane
+    ((2, 8, 2048, 4), 0.05),       # a power-of-two grid with too many bins for that kernel
+    ((2, 8, 2048, 4), 1),          # run kernel: 4 units per row, block-shared bins
+    ((8, 128, 8), (0, 0, 0.1, 0.1, 0.3, 2.0)),   # repeated edges, one above every k
+])
+def test_powspec_kernel_edges(cuda, shape, bins):
+    """Auto and cross power with and without the window against the same
+    function in float64 on the CPU.  The kernels form float32 products per
+    cell (window included, some 2^-21 of |F| |G|: 1e-6) and the float32
+    transform is off by up to 1e-6 of the unit rms of these fields in each
+    of the (at most two) channels, times at most (pi/2)^3 = 3.9 with the
+    window: 1e-6 |F| |G| + 1.5e-6 (|F| + |G|) 3.9, and the bins' means are
+    bounded by the same expression of their powers."""
+    from pmwd_gb300.spec_util import powspec
+    rng = np.random.default_rng(9)
+    f = torch.from_numpy(rng.normal(size=shape).astype(np.float32))
+    g = torch.from_numpy(rng.normal(size=shape).astype(np.float32))
+    for kw in ({}, {'deconv': 2}, {'g': g}, {'g': g, 'deconv': 2}):
+        wide = {k: v.double() if k == 'g' else v for k, v in kw.items()}
+        want = powspec(f.double(), 1.0, bins=bins, **wide)
+        dk = {k: v for k, v in kw.items() if k == 'deconv'}
+        pf, pg = (torch.sqrt(powspec(x.double(), 1.0, bins=bins, **dk)[1]) for x in (f, g))
+        if 'g' not in kw:
+            pg = pf
+        got = powspec(f.to(cuda), 1.0, bins=bins,
+                      **{k: v.to(cuda) if k == 'g' else v for k, v in kw.items()})
+        assert got[1].shape == want[1].shape
+        np.testing.assert_array_equal(got[2].cpu().numpy(), want[2].numpy())
+        np.testing.assert_allclose(got[0].cpu().numpy(), want[0].numpy(), rtol=1e-12)
+        off, full = (got[1].cpu() - want[1]).abs(), want[2] > 0
+        assert (off <= 1e-6 * pf * pg + 6e-6 * (pf + pg))[full].all()
