@@ -118,6 +118,7 @@ struct pmx_workspace {
     // they replace cuFFT and the x pass (meshes plane-interleaved as above)
     bool own = false;
     float2 *mtw = nullptr;      // their twiddle tables
+    bool own_plane = false;     // z and y axes in one kernel
     bool win = false;           // warp-window deposits (n2 % 4 == 0)
     int64_t slab = 0;           // x-planes per 2-D cuFFT execution
     float2 *tw = nullptr;       // exp(-2 pi i m / n0)
@@ -1771,7 +1772,8 @@ float green_c(const pmx_workspace *ws, double omega_m) {
 // The Poisson solve by the library's own mesh transforms: dens -> g (adj =
 // false), or mcot -> rcot_of(nslot) (adj = true).  ck holds the half rows; the
 // spectra live in g, which is free until the z axis writes it: the forward
-// c2r after the y axis has read them, the adjoint's rcot where D was.
+// c2r after the y axis has read them, the adjoint's rcot where D was.  With the
+// plane kernels there are no half rows and ck holds the forward spectra.
 int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStream_t st) {
     MeshGeom g;
     g.n0 = ws->n0;
@@ -1781,13 +1783,18 @@ int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStrea
     g.unit = ws->n0 * ws->n1 * ws->n2p;
     GreenTab gt;
     for (int b = 0; b < nslot; ++b) gt.c[b] = c[b];
-    float2 *s0 = reinterpret_cast<float2 *>(ws->g), *s1 = s0 + nslot * g.unit;
+    // the plane kernels write the meshes while other clusters read the spectra
+    const bool plane = ws->own_plane && !adj;
+    float2 *s0 = plane ? ws->ck : reinterpret_cast<float2 *>(ws->g), *s1 = s0 + nslot * g.unit;
     const float2 *tx = ws->mtw, *ty = tx + 2 * ws->n0, *tz = ty + 2 * ws->n1;
     const int64_t planes = nslot * ws->n0;
     int e;
     {
-        Stage sg(ws, adj ? 8 : 2, st, 2);
-        if ((e = mesh_rows(false, adj ? ws->mcot : ws->dens, ws->ck, tz, adj ? 3 * planes : planes,
+        Stage sg(ws, adj ? 8 : 2, st, plane ? 1 : 2);
+        if (plane) {
+            if ((e = mesh_plane(MESH_COLS_FWD, nslot, g, ws->dens, s0, s1, ty, tz, ws->ktab, st)))
+                return e;
+        } else if ((e = mesh_rows(false, adj ? ws->mcot : ws->dens, ws->ck, tz, adj ? 3 * planes : planes,
                            ws->n1, ws->n2, st)) ||
             (e = mesh_cols(adj ? MESH_COLS_ADJ : MESH_COLS_FWD, nslot, g, ws->ck, s0, s1, ty, ws->ktab,
                            st)))
@@ -1797,7 +1804,10 @@ int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStrea
         Stage sg(ws, adj ? 9 : 3, st, 1);
         if ((e = mesh_xaxis(adj, nslot, g, s0, s1, tx, ws->ktab, gt, st))) return e;
     }
-    Stage sg(ws, adj ? 10 : 4, st, 2);
+    Stage sg(ws, adj ? 10 : 4, st, ws->own_plane ? 1 : 2);
+    if (ws->own_plane)
+        return mesh_plane(adj ? MESH_COLS_INV1 : MESH_COLS_INV3, nslot, g,
+                          adj ? ws->rcot_of(nslot) : ws->g, s0, s1, ty, tz, ws->ktab, st);
     if ((e = mesh_cols(adj ? MESH_COLS_INV1 : MESH_COLS_INV3, nslot, g, ws->ck, s0, s1, ty, ws->ktab,
                        st)))
         return e;
@@ -2022,13 +2032,10 @@ void ws_free(pmx_workspace *ws) {
 }
 
 // Whether a workspace of this shape and flags uses the mesh transforms of
-// pmx_mesh_fft.cuh.  They are faster at every supported size (force + VJP at
-// 64^3 62 against 72 us of device time, 1024^3 35.6 against 43.6 ms), but one
-// force takes eight launches instead of six, which shows at 64^3, where the
-// host's launches are the bound (70 against 76 us per force).
+// pmx_mesh_fft.cuh: they are faster at every supported size (a force at 64^3 40
+// against 51 us of device time, force + VJP at 1024^3 33 against 43.6 ms).
 bool own_path(const int64_t s[3], int32_t flags) {
-    return mesh_fft_supported(s[0], s[1], s[2]) && s[0] * s[1] * s[2] > 64 * 64 * 64 &&
-           !(flags & (PMX_WS_CUFFT3D | PMX_WS_PLANE));
+    return mesh_fft_supported(s[0], s[1], s[2]) && !(flags & (PMX_WS_CUFFT3D | PMX_WS_PLANE));
 }
 
 size_t buffers_bytes(const int64_t s[3], int32_t flags, int32_t slots) {
@@ -2183,7 +2190,8 @@ static int ws_create(const int64_t mesh_shape[3], int32_t flags, int32_t slots,
             return fail(PMX_ERR_CUDA, "mesh transform twiddle upload failed");
         }
         if ((st = mesh_rows_prepare(ws->n2)) || (st = mesh_cols_prepare(ws->n1)) ||
-            (st = mesh_xaxis_prepare(ws->n0))) {
+            (st = mesh_xaxis_prepare(ws->n0)) ||
+            (st = mesh_plane_prepare(ws->n1, ws->n2, &ws->own_plane))) {
             ws_free(ws);
             return st;
         }
@@ -2694,7 +2702,7 @@ static int nbody_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int
         const float *f = factors + 3 * i;
         if ((st = force_meshes(ws, h, omega_m, s))) return st;
         if (i + 1 < nsteps) {
-            {
+            if (!ws->own_plane) {   // whose forward kernel leaves dens filled
                 Stage sg(ws, 0, s, 1);
                 k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
                 PMX_LAUNCH_CHECK("k_fill");
@@ -2786,8 +2794,9 @@ static int nbody_adj_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const
         if ((st = force_adj_meshes(ws, omega_m, s))) return st;
         if (i + 1 < nsteps) {
             {
-                Stage sg(ws, 0, s, 2);
-                k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
+                Stage sg(ws, 0, s, ws->own_plane ? 1 : 2);
+                if (!ws->own_plane)
+                    k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
                 k_fill<<<grid_fill(3 * ws->M), 256, 0, s>>>(ws->mcot, 0.f, 3 * ws->M);
                 PMX_LAUNCH_CHECK("k_fill");
             }

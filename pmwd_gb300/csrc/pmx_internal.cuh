@@ -103,6 +103,12 @@ enum { MESH_COLS_FWD, MESH_COLS_ADJ, MESH_COLS_INV1, MESH_COLS_INV3 };
 // y axis of nslot slots: nat <-> spectra (one, or two: spec0 and spec1).
 int mesh_cols(int kind, int nslot, const MeshGeom &g, float2 *nat, float2 *spec0, float2 *spec1,
               const float2 *tw, const float *kt, cudaStream_t st);
+// Both axes of n1 x n1 planes (FWD, INV1, INV3): real planes <-> spectra.  FWD leaves
+// the planes filled with -1, as the next density deposit wants them.
+// prepare: once per workspace; *fits: whether there are kernels for these planes.
+int mesh_plane_prepare(int64_t n1, int64_t n2, bool *fits);
+int mesh_plane(int kind, int nslot, const MeshGeom &g, float *mesh, float2 *spec0, float2 *spec1,
+               const float2 *twy, const float2 *twz, const float *kt, cudaStream_t st);
 int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, const float2 *tw,
                const float *kt, const GreenTab &gt, cudaStream_t st);
 

@@ -15,6 +15,8 @@
 //   k_xaxis_adj (S = IFFT_x(-(c / k^2) [i kx FFT_x(C_0) + FFT_x(D)]));
 //   k_cols_inv; k_rows_c2r.
 // Two spectra instead of three pass through the x axis in either direction.
+// Square planes up to 128 x 128: k_plane_fwd and k_plane_inv do both axes of a plane
+// (pmx_mesh_plane.cu).
 //
 // Every length-N transform is N = R1 * R2: radix-R1 DFTs of R2-strided
 // elements in registers, twiddles, ONE exchange through shared memory,
@@ -85,6 +87,39 @@ using XCol = TileCfg<N, 128 / Fac<N>::R2 < 4 ? 4 : 128 / Fac<N>::R2>;
 // 1024^3, 0.55 against 0.50 at 512^3.
 template <int N>
 using YCol = XCol<N>;
+
+// Half length L = R1 * R2 of a row transform.  R1 / 2 threads share a row:
+// thread 0 holds the groups k1 = 0 and R1 / 2 of the radix-R2 side, thread i
+// the groups i and R1 - i, so that every pair Z[k], Z[L - k] that the
+// real-input split combines meets in one thread's registers.
+template <int L>
+struct RowCfg;
+#define PMX_ROW_CFG(L_, R1_, R2_)                 \
+    template <>                                   \
+    struct RowCfg<L_> {                           \
+        static constexpr int R1 = R1_, R2 = R2_;  \
+        static constexpr int TPR = R1 / 2;        \
+        static constexpr int ROWS = 128 / TPR;    \
+        static constexpr int TH = 128;            \
+        static constexpr int S = R2 + 1;          \
+        /* rows 16, 8 or 4 values apart (mod 16): no bank conflicts between the rows of a half warp */ \
+        static constexpr int RS = R1 * S + (16 + TPR % 16 - R1 * S % 16) % 16; \
+        static constexpr int NZT = (L_ + 4) / 4;  \
+    };
+PMX_ROW_CFG(32, 8, 4)
+PMX_ROW_CFG(48, 8, 6)
+PMX_ROW_CFG(64, 8, 8)
+PMX_ROW_CFG(96, 8, 12)
+PMX_ROW_CFG(128, 16, 8)
+PMX_ROW_CFG(192, 16, 12)
+PMX_ROW_CFG(256, 32, 8)
+PMX_ROW_CFG(384, 32, 12)
+PMX_ROW_CFG(512, 32, 16)
+#undef PMX_ROW_CFG
+
+__device__ __forceinline__ float2 pick(bool c, float2 a, float2 b) {
+    return make_float2(c ? a.x : b.x, c ? a.y : b.y);
+}
 
 // Twiddle tables of a length-N transform (float2): w^(b k1) at k1 * R2 + b,
 // then the same at b * R1 + k1 (w = exp(-2 pi i / N)).

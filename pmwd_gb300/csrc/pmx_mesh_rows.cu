@@ -6,35 +6,6 @@ namespace pmx {
 
 namespace {
 
-// Half length L = R1 * R2 of a row transform.  R1 / 2 threads share a row:
-// thread 0 holds the groups k1 = 0 and R1 / 2 of the radix-R2 side, thread i
-// the groups i and R1 - i, so that every pair Z[k], Z[L - k] that the
-// real-input split combines meets in one thread's registers.
-template <int L>
-struct RowCfg;
-#define PMX_ROW_CFG(L_, R1_, R2_)                 \
-    template <>                                   \
-    struct RowCfg<L_> {                           \
-        static constexpr int R1 = R1_, R2 = R2_;  \
-        static constexpr int TPR = R1 / 2;        \
-        static constexpr int ROWS = 128 / TPR;    \
-        static constexpr int TH = 128;            \
-        static constexpr int S = R2 + 1;          \
-        /* rows 16, 8 or 4 values apart (mod 16): no bank conflicts between the rows of a half warp */ \
-        static constexpr int RS = R1 * S + (16 + TPR % 16 - R1 * S % 16) % 16; \
-        static constexpr int NZT = (L_ + 4) / 4;  \
-    };
-PMX_ROW_CFG(32, 8, 4)
-PMX_ROW_CFG(48, 8, 6)
-PMX_ROW_CFG(64, 8, 8)
-PMX_ROW_CFG(96, 8, 12)
-PMX_ROW_CFG(128, 16, 8)
-PMX_ROW_CFG(192, 16, 12)
-PMX_ROW_CFG(256, 32, 8)
-PMX_ROW_CFG(384, 32, 12)
-PMX_ROW_CFG(512, 32, 16)
-#undef PMX_ROW_CFG
-
 // A group of 8 half rows passes through shared memory, in blocks of 8 rows x 4
 // kz padded to ZB values, on its way to or from global memory, so that it
 // moves in whole 256-byte blocks.  Straight from registers it would move in
@@ -81,10 +52,6 @@ struct RowPairs {
     template <int I>
     __device__ __forceinline__ int k() const { return (2 * I < C::R2 ? k0 : k1) + I * C::R1; }
 };
-
-__device__ __forceinline__ float2 pick(bool c, float2 a, float2 b) {
-    return make_float2(c ? a.x : b.x, c ? a.y : b.y);
-}
 
 // Bound: HBM (one read of the real rows, one write of the half rows): 1.43 ms
 // for 1024 planes of 1024 x 1024, 6.0 TB/s.  The shared-memory pipe comes next

@@ -48,6 +48,13 @@ def test_force_and_vjp_against_cufft(shape):
     assert abs(res[0][2] - res[1][2]) < 1.3e-6 * scale
 
 
+@pytest.mark.parametrize('shape', ((64, 64, 64), (256, 64, 64), (64, 96, 96), (96, 128, 128),
+                                   (128, 192, 192)))
+def test_square_planes(shape):
+    """n x n planes: z and y axes in one kernel up to n = 128, two beyond."""
+    test_force_and_vjp_against_cufft(shape)
+
+
 def test_batched_equals_single():
     """Two slots of one batched call against two single-simulation forces: one x-axis launch
     serves both with its own Green's constant."""
