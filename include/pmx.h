@@ -465,6 +465,16 @@ int pmx_lpt_disp(const int64_t grid_shape[3], const float *tables, const float *
                  float scale, int32_t orders, const float *fac, const float *fac_dev,
                  int16_t *pmid, float *disp, float *vel, void *stream);
 
+/* All of the above in one call, for the grids whose axes the library's own
+ * transforms support (64, 96, 128, 192, 256, 384, 512, 768, 1024): contiguous
+ * modes to pmid, disp and vel.  scratch: 256-byte aligned device memory of
+ * pmx_lpt_solve_floats floats (count 0: no transforms of this shape), in use until
+ * the stream is past this call. */
+int pmx_lpt_solve_floats(const int64_t grid_shape[3], int32_t orders, int64_t *count);
+int pmx_lpt_solve(const int64_t grid_shape[3], const float *tables, const float *modes, float scale,
+                  int32_t orders, const float *fac, float *scratch, int16_t *pmid, float *disp,
+                  float *vel, void *stream);
+
 /* Transposes, for a real cotangent of disp and vel.  grads_cot (3 orders, n);
  * src_cot: the second-order source's, in Fourier space, to be transformed by
  * an unnormalised complex-to-real transform, from the spectra of the second

@@ -90,6 +90,9 @@ SIGNATURES = {
     'pmx_powspec_bin_layout': (c_int, [c_p, c_p, c_i64, ctypes.POINTER(c_i64), c_p, c_p, c_p, c_p,
                                        c_i32, c_i32, c_i32, c_d, c_p, c_p, c_p, c_i32, c_p, c_p]),
     'pmx_powspec_scratch_bytes': (c_i64, [ctypes.POINTER(c_i64), c_i32, c_i32, c_i32, c_i32, c_i32]),
+    'pmx_lpt_solve_floats': (c_int, [ctypes.POINTER(c_i64), c_i32, ctypes.POINTER(c_i64)]),
+    'pmx_lpt_solve': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, c_f, c_i32, ctypes.POINTER(c_f), c_p, c_p,
+                              c_p, c_p, c_p]),
     'pmx_lpt_table_floats': (c_int, [ctypes.POINTER(c_i64), ctypes.POINTER(c_i64)]),
     'pmx_lpt_tables': (c_int, [ctypes.POINTER(c_i64), ctypes.POINTER(c_i64), c_d, c_d, c_p, c_p]),
     'pmx_lpt_strain': (c_int, [ctypes.POINTER(c_i64), c_p, c_p, c_f, c_p, c_p]),

@@ -92,6 +92,13 @@ struct GreenTab {
 bool mesh_fft_supported(int64_t n0, int64_t n1, int64_t n2);
 // Writes the twiddle tables to t (unless NULL); returns their length.
 int64_t mesh_fft_twiddles(int64_t n0, int64_t n1, int64_t n2, float2 *t);
+// The same tables computed on the device (t in device memory).
+int mesh_fft_twiddles_dev(int64_t n0, int64_t n1, int64_t n2, float2 *t, cudaStream_t st);
+// x axis of contiguous modes (n0, n1, n2h), p = scale modes / k^2: spectra X_2, X_1,
+// X_0 (grads false: inverse transforms of kx^2 p, kx p, p) or G_0, Q (grads true: of
+// i kx p, -p), one after the other.
+int mesh_xaxis_modes(bool grads, const MeshGeom &g, const float2 *modes, float scale, float2 *spec,
+                     const float2 *tw, const float *kt, cudaStream_t st);
 int mesh_rows_prepare(int64_t n2);   // once per workspace: shared-memory opt-ins
 int mesh_rows_factors(int64_t n2, int *R1, int *R2);   // of the half length
 int mesh_cols_prepare(int64_t n1);
@@ -99,7 +106,7 @@ int mesh_xaxis_prepare(int64_t n0);
 // z axis of `planes` consecutive planes: real <-> nat.
 int mesh_rows(bool inv, const void *in, void *out, const float2 *tw, int64_t planes, int64_t n1,
               int64_t n2, cudaStream_t st);
-enum { MESH_COLS_FWD, MESH_COLS_ADJ, MESH_COLS_INV1, MESH_COLS_INV3 };
+enum { MESH_COLS_FWD, MESH_COLS_ADJ, MESH_COLS_INV1, MESH_COLS_INV3, MESH_COLS_INV6 };
 // y axis of nslot slots: nat <-> spectra (one, or two: spec0 and spec1).
 int mesh_cols(int kind, int nslot, const MeshGeom &g, float2 *nat, float2 *spec0, float2 *spec1,
               const float2 *tw, const float *kt, cudaStream_t st);

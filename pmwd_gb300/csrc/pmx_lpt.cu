@@ -11,8 +11,16 @@
 // bound).  As separate tensor operations the same stages took about 110 launches
 // and 2.4 of 3.6 ms at 256^3.  Transforms are unnormalised; 1 / N is applied
 // where a stage reads their result.
+//
+// pmx_lpt_solve does all of it with the transforms of pmx_mesh_fft.cuh where they
+// have the shape: ky and kz are constant along x, so the x axis makes three spectra
+// of the modes for the six strains (of kx^2 p, kx p, p) and two for the three
+// gradients, and the spectra between the axes are never written in full.  256^3:
+// 0.95 ms of device time against 1.60 with 3-D cuFFT between the stages.
 
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 #include "pmx_internal.cuh"
 
@@ -123,19 +131,50 @@ __global__ void __launch_bounds__(LT) k_lpt_strain(const float2 *__restrict__ mo
     });
 }
 
+// Fields of a real grid: element r of x-plane x of field c at x xs + c cs + r.
+struct Fields {
+    int64_t xs, cs;
+};
+
 // L = phi_00 phi_22 + phi_00 phi_11 + phi_11 phi_22 - phi_01^2 - phi_02^2 - phi_12^2
-// (lpt.py:40-76), phi = s times the transforms.
+// (lpt.py:40-76), phi = s times the transforms.  A block row per x-plane of pl
+// values, V at a time.
+__device__ __forceinline__ float lpt_source(const float (&p)[6]) {
+    float v = fmaf(p[0], p[1], p[0] * p[2]);
+    v = fmaf(p[1], p[2], v);
+#pragma unroll
+    for (int c = 3; c < 6; ++c) v = fmaf(-p[c], p[c], v);
+    return v;
+}
+template <int V>
 __global__ void __launch_bounds__(LT) k_lpt_source(const float *__restrict__ phi,
-                                                   float *__restrict__ L, int64_t n, float s) {
-    for (int64_t q = blockIdx.x * (int64_t)LT + threadIdx.x; q < n; q += (int64_t)gridDim.x * LT) {
-        float p[6];
+                                                   float *__restrict__ L, int64_t pl, int64_t n0,
+                                                   Fields f, float s) {
+    for (int64_t x = blockIdx.y; x < n0; x += gridDim.y) {
+        const float *ph = phi + x * f.xs;
+        for (int64_t q = (blockIdx.x * (int64_t)LT + threadIdx.x) * V; q < pl;
+             q += (int64_t)gridDim.x * LT * V) {
+            if constexpr (V == 4) {
+                float4 u[6];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) p[c] = s * phi[q + c * n];
-        float v = fmaf(p[0], p[1], p[0] * p[2]);
-        v = fmaf(p[1], p[2], v);
+                for (int c = 0; c < 6; ++c)
+                    u[c] = *reinterpret_cast<const float4 *>(ph + q + c * f.cs);
+                float o[4];
 #pragma unroll
-        for (int c = 3; c < 6; ++c) v = fmaf(-p[c], p[c], v);
-        L[q] = v;
+                for (int i = 0; i < 4; ++i) {
+                    float p[6];
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) p[c] = s * (&u[c].x)[i];
+                    o[i] = lpt_source(p);
+                }
+                *reinterpret_cast<float4 *>(L + x * pl + q) = make_float4(o[0], o[1], o[2], o[3]);
+            } else {
+                float p[6];
+#pragma unroll
+                for (int c = 0; c < 6; ++c) p[c] = s * ph[q + c * f.cs];
+                L[x * pl + q] = lpt_source(p);
+            }
+        }
     }
 }
 
@@ -167,36 +206,85 @@ struct LptFac {
     const float *dev;   // or in device memory (a graph's input)
 };
 
+constexpr int LPT_PB = 2;
+
 // pmid and disp of the lattice plus disp += D_m g_m, vel += a^2 H dD_m/dlna g_m
-// order by order (lpt.py:197-210); g = s times the transforms.
-__global__ void __launch_bounds__(LT) k_lpt_disp(const float *__restrict__ gr, int orders,
+// order by order (lpt.py:197-210); g = s times the transforms, those of order 2 at
+// gr2.  The bound is HBM (54 bytes per particle: 0.13 ms at
+// 256^3), given enough loads in flight: a thread fetches two particles' fields
+// before it uses the first, and the outputs pass through shared memory so that a
+// warp stores whole lines.  0.136 ms; one particle per thread 0.22, with three
+// 12-byte-strided stores each 0.25.
+__global__ void __launch_bounds__(LT) k_lpt_disp(const float *__restrict__ gr,
+                                                 const float *__restrict__ gr2, Fields fl, int orders,
                                                  int16_t *__restrict__ pmid,
                                                  float *__restrict__ disp, float *__restrict__ vel,
                                                  LptGrid g, LptFac f, float s) {
-    const int64_t n = (int64_t)g.n0 * g.n1 * g.n2;
+    constexpr int PB = LPT_PB * LT;   // particles of a block's turn
+    __shared__ __align__(16) float sd[3 * PB], sv[3 * PB];
+    __shared__ __align__(16) int16_t sp[3 * PB];
+    // whole turns are stored in 16-byte pieces (3 PB values of either type are)
+    const bool wide = (((uintptr_t)pmid | (uintptr_t)disp | (uintptr_t)vel) & 15) == 0;
+    const int64_t pl = (int64_t)g.n1 * g.n2, n = g.n0 * pl;
     float fac[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) fac[u] = s * (f.dev ? (u < 2 * orders ? f.dev[u] : 0.f) : f.f[u]);
-    for (int64_t q = blockIdx.x * (int64_t)LT + threadIdx.x; q < n; q += (int64_t)gridDim.x * LT) {
-        const int64_t r = q / g.n2;
-        int c[3];
-        c[2] = (int)(q - r * g.n2);
-        c[0] = (int)(r / g.n1);
-        c[1] = (int)(r - (int64_t)c[0] * g.n1);
+    for (int64_t q0 = blockIdx.x * (int64_t)PB; q0 < n; q0 += (int64_t)gridDim.x * PB) {
+        int c[LPT_PB][3];
+        float x[LPT_PB][2][3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            float d = __ldg(g.lat(a) + c[a]), v = 0.f;
-#pragma unroll
-            for (int o = 0; o < 2; ++o) {
-                if (o >= orders) break;
-                const float x = gr[q + (3 * o + a) * n];
-                d = fmaf(fac[2 * o], x, d);
-                v = fmaf(fac[2 * o + 1], x, v);
+        for (int i = 0; i < LPT_PB; ++i) {   // every load before the first use
+            const int64_t q = q0 + i * LT + threadIdx.x < n ? q0 + i * LT + threadIdx.x : n - 1;
+            if (n <= 0x7fffffff) {   // 32-bit divisions
+                const unsigned u = (unsigned)q / (unsigned)g.n2;
+                c[i][2] = (int)((unsigned)q - u * (unsigned)g.n2);
+                c[i][0] = (int)(u / (unsigned)g.n1);
+                c[i][1] = (int)(u - (unsigned)c[i][0] * (unsigned)g.n1);
+            } else {
+                const int64_t r = q / g.n2;
+                c[i][2] = (int)(q - r * g.n2);
+                c[i][0] = (int)(r / g.n1);
+                c[i][1] = (int)(r - (int64_t)c[i][0] * g.n1);
             }
-            pmid[3 * q + a] = g.pm(a)[c[a]];
-            disp[3 * q + a] = d;
-            vel[3 * q + a] = v;
+            const int64_t at = c[i][0] * fl.xs + ((int64_t)c[i][1] * g.n2 + c[i][2]);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                x[i][0][a] = gr[at + a * fl.cs];
+                x[i][1][a] = orders > 1 ? gr2[at + a * fl.cs] : 0.f;
+            }
         }
+#pragma unroll
+        for (int i = 0; i < LPT_PB; ++i)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int o = 3 * (i * LT + threadIdx.x) + a;
+                float d = fmaf(fac[0], x[i][0][a], __ldg(g.lat(a) + c[i][a]));
+                float v = fac[1] * x[i][0][a];
+                if (orders > 1) {
+                    d = fmaf(fac[2], x[i][1][a], d);
+                    v = fmaf(fac[3], x[i][1][a], v);
+                }
+                sp[o] = g.pm(a)[c[i][a]];
+                sd[o] = d;
+                sv[o] = v;
+            }
+        __syncthreads();
+        const int m = 3 * (int)(n - q0 < PB ? n - q0 : PB);
+        if (wide && m == 3 * PB) {
+            for (int i = threadIdx.x; i < 3 * PB / 4; i += LT) {
+                reinterpret_cast<float4 *>(disp + 3 * q0)[i] = reinterpret_cast<float4 *>(sd)[i];
+                reinterpret_cast<float4 *>(vel + 3 * q0)[i] = reinterpret_cast<float4 *>(sv)[i];
+            }
+            for (int i = threadIdx.x; i < 3 * PB / 8; i += LT)
+                reinterpret_cast<int4 *>(pmid + 3 * q0)[i] = reinterpret_cast<int4 *>(sp)[i];
+        } else {
+            for (int i = threadIdx.x; i < m; i += LT) {
+                pmid[3 * q0 + i] = sp[i];
+                disp[3 * q0 + i] = sd[i];
+                vel[3 * q0 + i] = sv[i];
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -327,6 +415,10 @@ int walk_grid(const Walk &w) {
     return (int)(need < cap ? need : cap);
 }
 int flat_grid(int64_t n) { return stride_grid(n, LT, 64); }
+// one turn per block: a block's stores overlap another one's loads
+int disp_grid(int64_t n) {
+    return (int)std::min<int64_t>((n + LPT_PB * LT - 1) / (LPT_PB * LT), 1 << 30);
+}
 
 int fac_of(const float *fac, int32_t orders, LptFac *f) {
     if (!fac) return fail(PMX_ERR_ARG, "null fac");
@@ -386,7 +478,7 @@ extern "C" int pmx_lpt_strain(const int64_t grid_shape[3], const float *tables, 
 
 extern "C" int pmx_lpt_source(int64_t n, const float *phi, float scale, float *src, void *stream) {
     if (n < 1 || !phi || !src) return fail(PMX_ERR_ARG, "bad lpt source arguments");
-    k_lpt_source<<<flat_grid(n), LT, 0, as_stream(stream)>>>(phi, src, n, scale);
+    k_lpt_source<1><<<flat_grid(n), LT, 0, as_stream(stream)>>>(phi, src, n, 1, Fields{0, n}, scale);
     PMX_LAUNCH_CHECK("k_lpt_source");
     return PMX_OK;
 }
@@ -416,8 +508,96 @@ extern "C" int pmx_lpt_disp(const int64_t grid_shape[3], const float *tables, co
     if (st || (st = fac_of(fac_dev ? none : fac, orders, &f))) return st;
     f.dev = fac_dev;
     if (!grads || !pmid || !disp || !vel) return fail(PMX_ERR_ARG, "null array");
-    k_lpt_disp<<<flat_grid((int64_t)g.n0 * g.n1 * g.n2), LT, 0, as_stream(stream)>>>(
-        grads, orders, pmid, disp, vel, g, f, scale);
+    const int64_t n = (int64_t)g.n0 * g.n1 * g.n2;
+    k_lpt_disp<<<disp_grid(n), LT, 0, as_stream(stream)>>>(
+        grads, grads + 3 * n, Fields{(int64_t)g.n1 * g.n2, n}, orders, pmid, disp, vel, g, f, scale);
+    PMX_LAUNCH_CHECK("k_lpt_disp");
+    return PMX_OK;
+}
+
+// Parts of pmx_lpt_solve's scratch, in floats: twiddles; three spectra; the half
+// rows of up to six fields; six real fields, of which the gradients take the places
+// when the strains are used up; the source.
+struct SolveScratch {
+    MeshGeom g;
+    int64_t M, tw, spec, nat, real, src, total;
+};
+static bool solve_scratch(const LptGrid &g, int32_t orders, SolveScratch *c) {
+    if (!mesh_fft_supported(g.n0, g.n1, g.n2)) return false;
+    c->g.n0 = g.n0;
+    c->g.n1 = g.n1;
+    c->g.n2h = g.n2h;
+    c->g.nzt = (g.n2h + 3) / 4;
+    c->g.unit = (int64_t)g.n0 * g.n1 * 4 * c->g.nzt;
+    c->M = (int64_t)g.n0 * g.n1 * g.n2;
+    const int64_t nf = orders > 1 ? 6 : 3;
+    c->tw = 0;
+    c->spec = (2 * mesh_fft_twiddles(g.n0, g.n1, g.n2, nullptr) + 63) / 64 * 64;
+    c->nat = c->spec + 2 * (orders > 1 ? 3 : 2) * c->g.unit;
+    c->real = c->nat + 2 * nf * c->g.unit;
+    c->src = c->real + nf * c->M;
+    c->total = c->src + (orders > 1 ? c->M : 0);
+    return true;
+}
+
+extern "C" int pmx_lpt_solve_floats(const int64_t grid_shape[3], int32_t orders, int64_t *count) {
+    LptGrid g;
+    float dummy = 0.f;
+    int st = grid_of(grid_shape, &dummy, &g);
+    if (st) return st;
+    if (!count || orders < 1 || orders > 2) return fail(PMX_ERR_ARG, "bad orders or null count");
+    SolveScratch c;
+    *count = solve_scratch(g, orders, &c) ? c.total : 0;
+    return PMX_OK;
+}
+
+extern "C" int pmx_lpt_solve(const int64_t grid_shape[3], const float *tables, const float *modes,
+                             float scale, int32_t orders, const float *fac, float *scratch,
+                             int16_t *pmid, float *disp, float *vel, void *stream) {
+    LptGrid g;
+    LptFac f;
+    SolveScratch c;
+    int e = grid_of(grid_shape, tables, &g);
+    if (e || (e = fac_of(fac, orders, &f))) return e;
+    if (!modes || !scratch || !pmid || !disp || !vel) return fail(PMX_ERR_ARG, "null array");
+    if (!solve_scratch(g, orders, &c)) return fail(PMX_ERR_SHAPE, "no mesh transforms of this shape");
+    cudaStream_t st = as_stream(stream);
+    if ((e = mesh_rows_prepare(g.n2)) || (e = mesh_cols_prepare(g.n1)) || (e = mesh_xaxis_prepare(g.n0)))
+        return e;
+    float2 *tx = reinterpret_cast<float2 *>(scratch), *ty = tx + 2 * g.n0, *tz = ty + 2 * g.n1;
+    float2 *s0 = reinterpret_cast<float2 *>(scratch + c.spec), *s1 = s0 + c.g.unit;
+    float2 *nat = reinterpret_cast<float2 *>(scratch + c.nat);
+    float *real = scratch + c.real, *src = scratch + c.src, *g2 = real + 3 * c.M;
+    const float2 *md = reinterpret_cast<const float2 *>(modes);
+    const int64_t pl = (int64_t)g.n1 * g.n2;
+    const float inv = (float)(1.0 / (double)c.M);
+    if ((e = mesh_fft_twiddles_dev(g.n0, g.n1, g.n2, tx, st))) return e;
+    if (orders > 1) {
+        // six strains: X_2, X_1, X_0 are all that the x axis needs to make of them
+        if ((e = mesh_xaxis_modes(false, c.g, md, scale, s0, tx, tables, st)) ||
+            (e = mesh_cols(MESH_COLS_INV6, 1, c.g, nat, s0, nullptr, ty, tables, st)) ||
+            (e = mesh_rows(true, nat, real, tz, 6 * (int64_t)g.n0, g.n1, g.n2, st)))
+            return e;
+        const int gy = g.n0 < 65535 ? g.n0 : 65535;
+        k_lpt_source<4><<<dim3((unsigned)((pl / 4 + LT - 1) / LT), gy), LT, 0, st>>>(
+            real, src, pl, g.n0, Fields{6 * pl, pl}, inv);
+        PMX_LAUNCH_CHECK("k_lpt_source");
+        // the gradients of the source's potential: a force with c = 1
+        GreenTab gt;
+        gt.c[0] = 1.f;
+        if ((e = mesh_rows(false, src, nat, tz, g.n0, g.n1, g.n2, st)) ||
+            (e = mesh_cols(MESH_COLS_FWD, 1, c.g, nat, s0, s1, ty, tables, st)) ||
+            (e = mesh_xaxis(false, 1, c.g, s0, s1, tx, tables, gt, st)) ||
+            (e = mesh_cols(MESH_COLS_INV3, 1, c.g, nat, s0, s1, ty, tables, st)) ||
+            (e = mesh_rows(true, nat, g2, tz, 3 * (int64_t)g.n0, g.n1, g.n2, st)))
+            return e;
+    }
+    if ((e = mesh_xaxis_modes(true, c.g, md, scale, s0, tx, tables, st)) ||
+        (e = mesh_cols(MESH_COLS_INV3, 1, c.g, nat, s0, s1, ty, tables, st)) ||
+        (e = mesh_rows(true, nat, real, tz, 3 * (int64_t)g.n0, g.n1, g.n2, st)))
+        return e;
+    k_lpt_disp<<<disp_grid(c.M), LT, 0, st>>>(real, g2, Fields{3 * pl, pl}, orders, pmid, disp, vel, g,
+                                              f, inv);
     PMX_LAUNCH_CHECK("k_lpt_disp");
     return PMX_OK;
 }

@@ -143,7 +143,9 @@ k_cols_adj(const float2 *__restrict__ nat,
 }
 
 // Spectra -> nat planes: NC = 1, one spectrum per slot; NC = 3, G_0 (spec0)
-// and Q (spec1) -> planes (slot, x, j) of the three gradients.
+// and Q (spec1) -> planes (slot, x, j) of the three gradients; NC = 6 (one slot),
+// X_2, X_1, X_0 of k_xaxis_modes (spec0) -> planes (x, c) of the second derivatives
+// 00 11 22 01 02 12.
 template <int N, int NC>
 __global__ void __launch_bounds__(YCol<N>::TH, col_blocks<YCol<N>>(1, inv_regs<N>()))
 k_cols_inv(const float2 *__restrict__ spec0,
@@ -161,6 +163,7 @@ k_cols_inv(const float2 *__restrict__ spec0,
     const int64_t tot = g.n0 + g.n1 + g.n2h;
     const float *my = kt + tot + g.n0;
     const float2 *src = (NC == 3 && c.comp ? spec1 : spec0) + slot * g.unit + spec_at(g, x, 0, l);
+    if (NC == 6) src += (c.comp == 0 ? 0 : (c.comp == 3 || c.comp == 4 ? 1 : 2)) * g.unit;
     const int64_t ys = (int64_t)g.nzt * 32;
     float2 v[C::R1];
 #pragma unroll
@@ -176,6 +179,22 @@ k_cols_inv(const float2 *__restrict__ spec0,
         const float m = l < g.n2h ? __ldg(kt + tot + g.n0 + g.n1 + l) : 0.f;
 #pragma unroll
         for (int a = 0; a < C::R1; ++a) v[a] = make_float2(__fmul_rn(m, v[a].y), -__fmul_rn(m, v[a].x));
+    }
+    if constexpr (NC == 6) {
+        const float *ky = kt + g.n0, *kz = ky + g.n1;
+        const float k = l < g.n2h ? __ldg(kz + l) : 0.f, m = l < g.n2h ? __ldg(kz + tot + l) : 0.f;
+        const float fz = c.comp == 2 ? k * k : (c.comp >= 4 ? m : 1.f);
+        if (c.comp == 1 || c.comp == 3 || c.comp == 5) {
+            const float *f = c.comp == 1 ? ky : my;
+#pragma unroll
+            for (int a = 0; a < C::R1; ++a) {
+                const float q = __ldg(f + b + a * C::R2), fy = (c.comp == 1 ? q * q : q) * fz;
+                v[a] = make_float2(v[a].x * fy, v[a].y * fy);
+            }
+        } else {
+#pragma unroll
+            for (int a = 0; a < C::R1; ++a) v[a] = make_float2(v[a].x * fz, v[a].y * fz);
+        }
     }
     col_stage1<C, true>(v, sm, t, b, tw);
     __syncthreads();
@@ -197,6 +216,7 @@ int mesh_cols_prepare(int64_t n1) {
         if ((st = smem_opt_in(k_cols_fwd<N>, cols_smem<YCol<N>>(1))) ||
             (st = smem_opt_in(k_cols_inv<N, 1>, cols_smem<YCol<N>>(1))) ||
             (st = smem_opt_in(k_cols_inv<N, 3>, cols_smem<YCol<N>>(1))) ||
+            (st = smem_opt_in(k_cols_inv<N, 6>, cols_smem<YCol<N>>(1))) ||
             (st = smem_opt_in(k_cols_adj<N>, cols_smem<YCol<N>>(2))))
             return st;
         return PMX_OK;
@@ -219,6 +239,10 @@ int mesh_cols(int kind, int nslot, const MeshGeom &g, float2 *nat, float2 *spec0
             case MESH_COLS_INV1:
                 k_cols_inv<N, 1><<<(unsigned)tiles, C::TH, cols_smem<YCol<N>>(1), st>>>(spec0, nullptr, nat,
                                                                                   tw, kt, g);
+                break;
+            case MESH_COLS_INV6:
+                k_cols_inv<N, 6><<<(unsigned)(6 * tiles), C::TH, cols_smem<YCol<N>>(1), st>>>(
+                    spec0, nullptr, nat, tw, kt, g);
                 break;
             default:
                 k_cols_inv<N, 3><<<(unsigned)(3 * tiles), C::TH, cols_smem<YCol<N>>(1), st>>>(spec0, spec1,

@@ -167,12 +167,109 @@ __global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(2, x_regs<N>(
     x_inv_step1<N>(A, t, b, p0, xbs);
 }
 
+// Modes in their own layout -> x-inverse-transformed spectra, see mesh_xaxis_modes.
+// A tile's p stays in registers where a thread has one group of at most 16 of it;
+// else it is read once per spectrum, after the first time from L1 or L2.  256^3: 83
+// and 68 us for three and two spectra, 113 and 78 with p read each time.
+template <int N>
+constexpr bool modes_keep() { return Fac<N>::R1 <= Fac<N>::R2 && Fac<N>::R2 <= 16; }
+template <int N>
+constexpr int modes_regs() { return modes_keep<N>() || Fac<N>::R1 >= 24 ? 168 : x_regs<N>(); }
+template <int N, bool GRADS>
+__global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(1, modes_regs<N>())) k_xaxis_modes(const float2 *__restrict__ modes,
+                                                             float scale, float2 *spec,
+                                                             const float2 *__restrict__ tw,
+                                                             const float *__restrict__ kt,
+                                                             MeshGeom g) {
+    using C = XCol<N>;
+    constexpr int R1 = C::R1, R2 = C::R2;
+    extern __shared__ __align__(16) float2 sm[];
+    const int nct = (4 * g.nzt + C::T - 1) / C::T;
+    const int t = threadIdx.x % C::T, b = threadIdx.x / C::T;
+    const int ky = blockIdx.x / nct, l = (blockIdx.x % nct) * C::T + t;
+    const bool ok = l < 4 * g.nzt, in = l < g.n2h;
+    const int64_t xbs = g.n1 * g.nzt * 32;                  // 8 x-planes
+    const int64_t at = ((int64_t)ky * g.nzt + (ok ? l >> 2 : 0)) * 32 + (l & 3);
+    const int64_t tot = g.n0 + g.n1 + g.n2h, xs = g.n1 * g.n2h;
+    const float2 *src = modes + (int64_t)ky * g.n2h + l;
+    const float kyj = __ldg(kt + g.n0 + ky), kzl = in ? __ldg(kt + g.n0 + g.n1 + l) : 0.f;
+    const float ky2 = __fmul_rn(kyj, kyj), kz2 = __fmul_rn(kzl, kzl);
+    // p of group k1, in the order of reg_dft
+    auto fetch = [&](float2 (&p)[R2], int k1) {
+        static_for<R2>([&](auto E) {
+            p[E] = in ? src[(k1 + R1 * reg_freq<R2>(E)) * xs] : make_float2(0.f, 0.f);
+        });
+        static_for<R2>([&](auto E) {
+            const float kx = ld_tab(kt + k1 + R1 * reg_freq<R2>(E));
+            const float k2 = __fadd_rn(__fadd_rn(__fmul_rn(kx, kx), ky2), kz2);
+            const float f = k2 != 0.f ? scale * (1.f / k2) : 0.f;   // k = 0 -> 0
+            p[E] = make_float2(p[E].x * f, p[E].y * f);
+        });
+    };
+    constexpr bool KEEP = modes_keep<N>();
+    float2 p[R2];
+    if (KEEP && b < R1) fetch(p, b);
+#pragma unroll 1
+    for (int s = 0; s < (GRADS ? 2 : 3); ++s) {
+        for (int k1 = b; k1 < R1; k1 += R2) {
+            if (!KEEP) fetch(p, k1);
+            float2 w[R2];
+            static_for<R2>([&](auto E) {
+                const int ix = k1 + R1 * reg_freq<R2>(E);
+                const float kx = ld_tab(kt + ix), mx = ld_tab(kt + tot + ix);
+                if (GRADS) {
+                    w[E] = s == 0 ? make_float2(-(mx * p[E].y), mx * p[E].x)
+                                  : make_float2(-p[E].x, -p[E].y);
+                } else {
+                    const float q = s == 0 ? kx * kx : (s == 1 ? mx : 1.f);
+                    w[E] = make_float2(p[E].x * q, p[E].y * q);
+                }
+            });
+            x_inv_step2<N>(w, sm, t, k1, tw_tr<N>(tw));
+        }
+        __syncthreads();
+        if (ok) x_inv_step1<N>(sm, t, b, spec + s * g.unit + at, xbs);
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ float2 twiddle(int j, int n) {   // exp(-2 pi i j / n)
+    double c, s;
+    sincospi(-2.0 * (double)(j % n) / (double)n, &s, &c);
+    return make_float2((float)c, (float)s);
+}
+struct TwAxis {
+    int n, R1, R2;
+};
+__global__ void k_twiddles(TwAxis x, TwAxis y, TwAxis z, float2 *t) {
+    int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const TwAxis ax[3] = {x, y, z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int n = ax[a].n;
+        if (q >= 0 && q < n) {
+            const int k1 = q / ax[a].R2, b = q % ax[a].R2;
+            const float2 w = twiddle(k1 * b, n);
+            t[q] = w;
+            t[n + b * ax[a].R1 + k1] = w;
+        }
+        q -= n;
+        t += 2 * n;
+    }
+    if (q >= 0 && q <= z.n) t[q] = twiddle(q, 2 * z.n);
+}
+
 }  // namespace
 
 int mesh_xaxis_prepare(int64_t n0) {
     return mesh_axis_dispatch(n0, [&](auto N) -> int {
-        int st = smem_opt_in(k_xaxis_fwd<N>, cols_smem<XCol<N>>(2));
-        return st ? st : smem_opt_in(k_xaxis_adj<N>, cols_smem<XCol<N>>(2));
+        int st;
+        if ((st = smem_opt_in(k_xaxis_fwd<N>, cols_smem<XCol<N>>(2))) ||
+            (st = smem_opt_in(k_xaxis_adj<N>, cols_smem<XCol<N>>(2))) ||
+            (st = smem_opt_in(k_xaxis_modes<N, false>, cols_smem<XCol<N>>(1))) ||
+            (st = smem_opt_in(k_xaxis_modes<N, true>, cols_smem<XCol<N>>(1))))
+            return st;
+        return PMX_OK;
     });
 }
 
@@ -188,6 +285,37 @@ int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, c
         PMX_LAUNCH_CHECK("mesh transform, x axis");
         return PMX_OK;
     });
+}
+
+int mesh_xaxis_modes(bool grads, const MeshGeom &g, const float2 *modes, float scale, float2 *spec,
+                     const float2 *tw, const float *kt, cudaStream_t st) {
+    return mesh_axis_dispatch(g.n0, [&](auto N) -> int {
+        using C = XCol<N>;
+        const unsigned grid = (unsigned)(g.n1 * ((4 * g.nzt + C::T - 1) / C::T));
+        const size_t smem = cols_smem<XCol<N>>(1);
+        if (grads)
+            k_xaxis_modes<N, true><<<grid, C::TH, smem, st>>>(modes, scale, spec, tw, kt, g);
+        else
+            k_xaxis_modes<N, false><<<grid, C::TH, smem, st>>>(modes, scale, spec, tw, kt, g);
+        PMX_LAUNCH_CHECK("mesh transform of modes, x axis");
+        return PMX_OK;
+    });
+}
+
+int mesh_fft_twiddles_dev(int64_t n0, int64_t n1, int64_t n2, float2 *t, cudaStream_t st) {
+    TwAxis ax[3];
+    const int64_t n[3] = {n0, n1, n2 / 2};
+    for (int a = 0; a < 3; ++a) {
+        ax[a].n = (int)n[a];
+        if (a < 2)
+            mesh_axis_r(n[a], [&](int R1, int R2) { ax[a].R1 = R1; ax[a].R2 = R2; });
+        else if (int e = mesh_rows_factors(n2, &ax[a].R1, &ax[a].R2))
+            return e;
+    }
+    const int tot = (int)(n0 + n1 + 2 * n[2] + 1);
+    k_twiddles<<<(tot + 63) / 64, 64, 0, st>>>(ax[0], ax[1], ax[2], t);
+    PMX_LAUNCH_CHECK("k_twiddles");
+    return PMX_OK;
 }
 
 // Tables in tw: the x axis' 2 n0 entries, the y axis' 2 n1, then the z axis'

@@ -113,3 +113,20 @@ def test_second_derivative():
                      pg.lpt(m, cosmo, conf)[0]))
     want = second(modes.to(torch.complex128).requires_grad_(), lambda m: _reference(m, fac, conf))
     assert _rel(got, want) < 2e-5
+
+
+@pytest.mark.parametrize('order', [1, 2])
+@pytest.mark.parametrize('grid', [(192, 128, 96), (64, 256, 192), (384, 96, 64), (96, 64, 512)])
+def test_own_transforms_against_float64(grid, order):
+    """Grids above the graphs' limit whose axes the library transforms itself.  Up to 22
+    levels instead of 17: TOL sqrt(22 / 17) = 2.3e-6."""
+    import pmwd_gb300 as pg
+    from pmwd_gb300 import _hostmath
+    conf, cosmo, modes, _ = _setup(grid, order)
+    lattice = pg.Particles.gen_grid(conf)
+    ptcl, _ = pg.lpt(modes, cosmo, conf)
+    disp, vel = _reference(modes.to(torch.complex128), _hostmath.lpt_factors(cosmo, conf), conf)
+    assert torch.equal(ptcl.pmid, lattice.pmid)
+    assert _rel(ptcl.vel, vel) < 2.3e-6
+    assert _rel(ptcl.disp - lattice.disp, disp) < 2.3e-6 + 2e-7 * float(
+        (lattice.disp.norm() + disp.norm()) / disp.norm())
