@@ -1357,31 +1357,30 @@ __global__ void __launch_bounds__(PT) k_sa_ka(Hot h, const int16_t *__restrict__
 // Sums the per-block partials in a fixed order: dots[s] = sum of slot s for
 // s < nslots (dots may be NULL), and *om_out = om_scale * sum of slot 2
 // (om_out may be NULL).  Slot 2 holds nblk2 partials (the gather VJP's
-// grid), the other slots nblk; slot s starts at part + s * pstride.
+// grid), the other slots nblk; slot s starts at part + s * pstride.  A block per
+// slot: three slots one after the other took 25 us of an adjoint step of 128^3
+// particles, side by side 10.
 __global__ void k_finish(const double *part, int64_t pstride, int nblk, int nblk2, double *dots,
                          int nslots, double *om_out, double om_scale) {
     __shared__ double sh[32];
-    int last = nslots > 3 ? nslots : 3;
-    for (int s = 0; s < last; ++s) {
-        bool want = (dots && s < nslots) || (om_out && s == 2);
-        if (!want) continue;
-        const int nb = s == 2 ? nblk2 : nblk;
-        const double *p = part + s * pstride;
-        // eight independent partial sums per thread of the 1024 (a fixed
-        // order), so the loads of a large grid's partials overlap
-        double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        int b = threadIdx.x;
-        for (; b + 7 * 1024 < nb; b += 8 * 1024) {
+    const int s = blockIdx.x;
+    if (!((dots && s < nslots) || (om_out && s == 2))) return;
+    const int nb = s == 2 ? nblk2 : nblk;
+    const double *p = part + s * pstride;
+    // eight independent partial sums per thread of the 1024 (a fixed
+    // order), so the loads of a large grid's partials overlap
+    double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    int b = threadIdx.x;
+    for (; b + 7 * 1024 < nb; b += 8 * 1024) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] += p[b + u * 1024];
-        }
-        for (; b < nb; b += 1024) a[0] += p[b];
-        double v = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-        double t = block_sum<1024>(v, sh);
-        if (threadIdx.x == 0) {
-            if (dots && s < nslots) dots[s] = t;
-            if (om_out && s == 2) *om_out = om_scale * t;
-        }
+        for (int u = 0; u < 8; ++u) a[u] += p[b + u * 1024];
+    }
+    for (; b < nb; b += 1024) a[0] += p[b];
+    double v = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+    double t = block_sum<1024>(v, sh);
+    if (threadIdx.x == 0) {
+        if (dots && s < nslots) dots[s] = t;
+        if (om_out && s == 2) *om_out = om_scale * t;
     }
 }
 
@@ -1490,17 +1489,16 @@ struct FinishTab {
 __global__ void k_finish_b(const double *part, int64_t pstride, int nblk,
                            const __grid_constant__ FinishTab t, int ndots) {
     __shared__ double sh[32];
-    const double *pp = part + blockIdx.x * NSLOT * pstride;
+    const int s = blockIdx.y;
+    if (s >= ndots && s != 2) return;
+    const double *p = part + (blockIdx.x * NSLOT + s) * pstride;
     double *dots = t.dots[blockIdx.x];
-    for (int s = 0; s < 3; ++s) {
-        if (s >= ndots && s != 2) continue;
-        double v = 0.0;
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += pp[s * pstride + b];
-        double tt = block_sum<1024>(v, sh);
-        if (threadIdx.x == 0) {
-            if (s < ndots) dots[s] = tt;
-            if (s == 2) dots[3] = t.oms[blockIdx.x] * tt;
-        }
+    double v = 0.0;
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += p[b];
+    double tt = block_sum<1024>(v, sh);
+    if (threadIdx.x == 0) {
+        if (s < ndots) dots[s] = tt;
+        if (s == 2) dots[3] = t.oms[blockIdx.x] * tt;
     }
 }
 
@@ -2408,7 +2406,7 @@ extern "C" int pmx_force_vjp(pmx_workspace *ws, const pmx_enmesh_spec *spec, con
         } else {
             {
                 Stage sg(ws, 12, s, 1);
-                k_finish<<<1, 1024, 0, s>>>(ws->part, ws->pstride, G, G, nullptr, 0, omega_m_cot,
+                k_finish<<<3, 1024, 0, s>>>(ws->part, ws->pstride, G, G, nullptr, 0, omega_m_cot,
                                             om_scale(omega_m));
                 PMX_LAUNCH_CHECK("k_finish");
             }
@@ -2613,7 +2611,7 @@ static int nbody_adj_step(pmx_workspace *ws, const pmx_enmesh_spec *spec, const 
     }
     {
         Stage sg(ws, 12, s, 1);
-        k_finish<<<1, 1024, 0, s>>>(ws->part, ws->pstride, G2, G, dots, 3, dots + 3,
+        k_finish<<<3, 1024, 0, s>>>(ws->part, ws->pstride, G2, G, dots, 3, dots + 3,
                                     om_scale(omega_m));
         PMX_LAUNCH_CHECK("k_finish");
     }
@@ -2786,7 +2784,7 @@ static int nbody_adj_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const
         }
         {
             Stage sg(ws, 12, s, 1);
-            k_finish<<<1, 1024, 0, s>>>(ws->part, ws->pstride, nb01, G, dots + 4 * i, 3,
+            k_finish<<<3, 1024, 0, s>>>(ws->part, ws->pstride, nb01, G, dots + 4 * i, 3,
                                         dots + 4 * i + 3,
                                         om_scale(omega_m));
             PMX_LAUNCH_CHECK("k_finish");
@@ -2992,7 +2990,7 @@ extern "C" int pmx_nbody_adj_steps_batch(pmx_workspace *ws, const pmx_enmesh_spe
         FinishTab ft = bc.fin;
         for (int b = 0; b < bc.nb; ++b) ft.dots[b] = bc.fin.dots[b] + 4 * row;
         Stage sg(ws, 12, s, 1);
-        k_finish_b<<<bc.nb, 1024, 0, s>>>(ws->part, ws->pstride, bc.G, ft, ndots);
+        k_finish_b<<<dim3(bc.nb, 3), 1024, 0, s>>>(ws->part, ws->pstride, bc.G, ft, ndots);
         PMX_LAUNCH_CHECK("k_finish_b");
         return PMX_OK;
     };
