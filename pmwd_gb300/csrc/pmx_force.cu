@@ -20,6 +20,7 @@
 #include <cudaTypedefs.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -247,38 +248,69 @@ __global__ void k_ktab(float *kt, int n0, int n1, int n2, double period, float n
     }
 }
 
+// The Fourier kernels of the 3-D cuFFT path.  A thread takes POIS cells 256 apart
+// and loads all of them before it uses one: these meshes live in L2 and the kernels
+// are bound by latency, not bytes.  180 x 150 x 120: 10.5 us forward and 12.2 adjoint;
+// a warp per row with one cell in flight per lane and 64-bit divisions 15.6 and 16.6.
+constexpr int POIS = 4;
+
+// Cell e of the half spectrum: wavenumbers and their gradient counterparts.
+struct Cell {
+    float k2, mx, my, mz;
+};
+__device__ __forceinline__ Cell fourier_cell(int64_t e, int64_t n0, int64_t n1, int64_t n2h,
+                                             bool small, const float *__restrict__ kt) {
+    int64_t i, j, l;
+    if (small) {   // 32-bit divisions
+        const unsigned r = (unsigned)e / (unsigned)n2h, x = r / (unsigned)n1;
+        l = (unsigned)e - r * (unsigned)n2h;
+        i = x;
+        j = r - x * (unsigned)n1;
+    } else {
+        const int64_t r = e / n2h;
+        l = e - r * n2h;
+        i = r / n1;
+        j = r - i * n1;
+    }
+    const float *ky = kt + n0, *kz = ky + n1, *m = kz + n2h;
+    const float kxi = __ldg(kt + i), kyj = __ldg(ky + j), kzl = __ldg(kz + l);
+    const float kxy = __fadd_rn(__fmul_rn(kxi, kxi), __fmul_rn(kyj, kyj));
+    Cell c;
+    c.k2 = __fadd_rn(kxy, __fmul_rn(kzl, kzl));
+    c.mx = __ldg(m + i);
+    c.my = __ldg(m + n0 + j);
+    c.mz = __ldg(m + n0 + n1 + l);
+    return c;
+}
+
 // Forward Fourier kernel, fused laplace + neg_grad for the three axes
 // (gravity.py:9-16, 37-44, 58-62): reads the r2c spectrum of the overdensity
 // and writes -i k_j * (-(F c)/k^2) for j = 0,1,2 (k = 0 -> 0), c = 1.5
 // Omega_m / N folding in the real-space scale and irfftn's 1/N.
-// One warp per (i, j) row of n2h complex values.
-__global__ void k_poisson_fwd(float2 *ck, int64_t n0, int64_t n1, int64_t n2h, int64_t Mc,
-                              const float *__restrict__ kt, float c) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const float *kx = kt, *ky = kt + n0, *kz = kt + n0 + n1;
-    const int64_t tot = n0 + n1 + n2h;
-    const float *mx = kt + tot, *my = kt + tot + n0, *mz = kt + tot + n0 + n1;
-    for (int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
-         row < n0 * n1; row += warps) {
-        int64_t i = row / n1, j = row - i * n1;
-        float kxi = __ldg(kx + i), kyj = __ldg(ky + j);
-        float mxi = __ldg(mx + i), myj = __ldg(my + j);
-        float kxy = __fadd_rn(__fmul_rn(kxi, kxi), __fmul_rn(kyj, kyj));
-        float2 *r0 = ck + row * n2h;
-        for (int64_t l = lane; l < n2h; l += 32) {
-            float kzl = __ldg(kz + l), mzl = __ldg(mz + l);
-            float k2 = __fadd_rn(kxy, __fmul_rn(kzl, kzl));
-            float2 F = r0[l];
+__global__ void __launch_bounds__(256) k_poisson_fwd(float2 *ck, int64_t n0, int64_t n1, int64_t n2h,
+                                                     int64_t Mc, const float *__restrict__ kt,
+                                                     float c) {
+    const bool small = Mc <= 0xffffffffll;
+    for (int64_t e0 = blockIdx.x * (int64_t)(256 * POIS) + threadIdx.x; e0 < Mc;
+         e0 += (int64_t)gridDim.x * 256 * POIS) {
+        float2 F[POIS];
+#pragma unroll
+        for (int u = 0; u < POIS; ++u)
+            F[u] = e0 + u * 256 < Mc ? ck[e0 + u * 256] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < POIS; ++u) {
+            const int64_t e = e0 + u * 256;
+            if (e >= Mc) break;
+            const Cell q = fourier_cell(e, n0, n1, n2h, small, kt);
             float pr = 0.f, pi = 0.f;
-            if (k2 != 0.f) {
-                pr = -__fdiv_rn(__fmul_rn(F.x, c), k2);
-                pi = -__fdiv_rn(__fmul_rn(F.y, c), k2);
+            if (q.k2 != 0.f) {
+                pr = -__fdiv_rn(__fmul_rn(F[u].x, c), q.k2);
+                pi = -__fdiv_rn(__fmul_rn(F[u].y, c), q.k2);
             }
             // (-i k)(pr + i pi) = (k pi, -k pr)
-            r0[l] = make_float2(__fmul_rn(mxi, pi), -__fmul_rn(mxi, pr));
-            r0[Mc + l] = make_float2(__fmul_rn(myj, pi), -__fmul_rn(myj, pr));
-            r0[2 * Mc + l] = make_float2(__fmul_rn(mzl, pi), -__fmul_rn(mzl, pr));
+            ck[e] = make_float2(__fmul_rn(q.mx, pi), -__fmul_rn(q.mx, pr));
+            ck[Mc + e] = make_float2(__fmul_rn(q.my, pi), -__fmul_rn(q.my, pr));
+            ck[2 * Mc + e] = make_float2(__fmul_rn(q.mz, pi), -__fmul_rn(q.mz, pr));
         }
     }
 }
@@ -287,35 +319,34 @@ __global__ void k_poisson_fwd(float2 *ck, int64_t n0, int64_t n1, int64_t n2h, i
 // irfftn o (-i k_j)(-1/k^2) o rfftn is irfftn o (+i k_j)(-1/k^2) o rfftn;
 // summed over the three axes: S = -(c/k^2) sum_j i k_j G_j, written over
 // the first spectrum.
-__global__ void k_poisson_adj(float2 *ck, int64_t n0, int64_t n1, int64_t n2h, int64_t Mc,
-                              const float *__restrict__ kt, float c) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const float *kx = kt, *ky = kt + n0, *kz = kt + n0 + n1;
-    const int64_t tot = n0 + n1 + n2h;
-    const float *mx = kt + tot, *my = kt + tot + n0, *mz = kt + tot + n0 + n1;
-    for (int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
-         row < n0 * n1; row += warps) {
-        int64_t i = row / n1, j = row - i * n1;
-        float kxi = __ldg(kx + i), kyj = __ldg(ky + j);
-        float mxi = __ldg(mx + i), myj = __ldg(my + j);
-        float kxy = __fadd_rn(__fmul_rn(kxi, kxi), __fmul_rn(kyj, kyj));
-        float2 *r0 = ck + row * n2h;
-        for (int64_t l = lane; l < n2h; l += 32) {
-            float kzl = __ldg(kz + l), mzl = __ldg(mz + l);
-            float k2 = __fadd_rn(kxy, __fmul_rn(kzl, kzl));
-            float2 G0 = r0[l], G1 = r0[Mc + l], G2 = r0[2 * Mc + l];
+__global__ void __launch_bounds__(256) k_poisson_adj(float2 *ck, int64_t n0, int64_t n1, int64_t n2h,
+                                                     int64_t Mc, const float *__restrict__ kt,
+                                                     float c) {
+    const bool small = Mc <= 0xffffffffll;
+    for (int64_t e0 = blockIdx.x * (int64_t)(256 * POIS) + threadIdx.x; e0 < Mc;
+         e0 += (int64_t)gridDim.x * 256 * POIS) {
+        float2 G[POIS][3];
+#pragma unroll
+        for (int u = 0; u < POIS; ++u)
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                G[u][a] = e0 + u * 256 < Mc ? ck[a * Mc + e0 + u * 256] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < POIS; ++u) {
+            const int64_t e = e0 + u * 256;
+            if (e >= Mc) break;
+            const Cell q = fourier_cell(e, n0, n1, n2h, small, kt);
             // i k (a + i b) = (-k b, k a)
-            float re = -__fadd_rn(__fadd_rn(__fmul_rn(mxi, G0.y), __fmul_rn(myj, G1.y)),
-                                  __fmul_rn(mzl, G2.y));
-            float im = __fadd_rn(__fadd_rn(__fmul_rn(mxi, G0.x), __fmul_rn(myj, G1.x)),
-                                 __fmul_rn(mzl, G2.x));
+            const float re = -__fadd_rn(__fadd_rn(__fmul_rn(q.mx, G[u][0].y), __fmul_rn(q.my, G[u][1].y)),
+                                        __fmul_rn(q.mz, G[u][2].y));
+            const float im = __fadd_rn(__fadd_rn(__fmul_rn(q.mx, G[u][0].x), __fmul_rn(q.my, G[u][1].x)),
+                                       __fmul_rn(q.mz, G[u][2].x));
             float sr = 0.f, si = 0.f;
-            if (k2 != 0.f) {
-                sr = -__fdiv_rn(__fmul_rn(re, c), k2);
-                si = -__fdiv_rn(__fmul_rn(im, c), k2);
+            if (q.k2 != 0.f) {
+                sr = -__fdiv_rn(__fmul_rn(re, c), q.k2);
+                si = -__fdiv_rn(__fmul_rn(im, c), q.k2);
             }
-            r0[l] = make_float2(sr, si);
+            ck[e] = make_float2(sr, si);
         }
     }
 }
@@ -1691,10 +1722,7 @@ int ensure_ktab(pmx_workspace *ws, double cell, cudaStream_t st) {
 }
 
 int poisson_grid(pmx_workspace *ws) {
-    int64_t rows = ws->n0 * ws->n1;
-    int64_t blocks = (rows + 7) / 8;  // 8 warps per block
-    int64_t cap = (int64_t)device_sms() * 16;
-    return (int)(blocks < cap ? blocks : cap);
+    return (int)std::min<int64_t>((ws->Mc + 256 * POIS - 1) / (256 * POIS), 1 << 30);
 }
 
 // Issues the slab loop of transform `kind` on stream s0: slab i (S x-planes
