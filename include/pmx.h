@@ -124,17 +124,20 @@ int pmx_gather_adj(const pmx_enmesh_spec *spec, const int16_t *pmid,
 typedef struct pmx_workspace pmx_workspace;
 
 #define PMX_WS_ADJOINT 1   /* also allocate buffers for the force VJP */
-#define PMX_WS_CUFFT3D 2   /* use 3-D cuFFT plans even where the fused x pass
-                              applies (n0 a power of two in 64..1024);
-                              for comparisons and tests */
+#define PMX_WS_CUFFT3D 2   /* use 3-D cuFFT plans even where the library's own
+                              transforms (every axis 64, 96, 128, 192, 256,
+                              384, 512, 768 or 1024) or the fused x pass (n0
+                              a power of two in 64..1024) apply; for
+                              comparisons and tests */
 #define PMX_WS_WINDOW 4    /* deposit through per-warp shared-memory windows
                               flushed with 16-byte vector reductions instead
                               of one global atomic per contribution (opt-in:
                               slower for lattice-ordered particles on GB300) */
-#define PMX_WS_PLANE 8     /* with the fused x pass, do the (y, z) plane
-                              transforms with the cluster plane kernels
-                              instead of slab-wise 2-D cuFFT (square
-                              power-of-two planes 64..1024) */
+#define PMX_WS_PLANE 8     /* the fused x pass in place of the library's own
+                              transforms, with the (y, z) plane transforms
+                              by the cluster plane kernels instead of
+                              slab-wise 2-D cuFFT (square power-of-two planes
+                              64..1024) */
 #define PMX_WS_VEC 16      /* deposit z-neighbour pairs that share an aligned
                               group of four floats with one 16-byte vector
                               reduction (n2 % 4 == 0; opt-in: slower on
@@ -168,9 +171,9 @@ int pmx_workspace_bytes(const int64_t mesh_shape[3], int32_t flags,
                         size_t *bytes);
 
 /* Creates the workspace on the current device: mesh and spectrum buffers,
- * cuFFT plans (r2c, batched c2r, and for PMX_WS_ADJOINT batched r2c and
- * c2r) with caller-visible work areas.  This is the only call that
- * allocates device memory. */
+ * twiddle tables or cuFFT plans (r2c, batched c2r, and for PMX_WS_ADJOINT
+ * batched r2c and c2r) with caller-visible work areas.  This is the only call
+ * of the workspace that allocates device memory. */
 int pmx_workspace_create(const int64_t mesh_shape[3], int32_t flags,
                          pmx_workspace **ws);
 int pmx_workspace_destroy(pmx_workspace *ws);
@@ -328,7 +331,7 @@ typedef struct pmx_sim {
 
 /* A workspace whose buffers hold `slots` simulations (1..16) of the same
  * mesh shape; pmx_workspace_create is the case slots = 1.  Batched calls
- * need the fused x-pass path (n0 a power of two in 64..1024) and the plain
+ * need the own transforms or the fused x pass (n0 a power of two) and the plain
  * deposits (no PMX_WS_WINDOW). */
 int pmx_workspace_create_batch(const int64_t mesh_shape[3], int32_t flags,
                                int32_t slots, pmx_workspace **ws);

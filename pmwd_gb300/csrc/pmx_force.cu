@@ -8,9 +8,12 @@
 //
 // Device layout of a workspace (float32 unless noted):
 //   dens  M           CIC density (initialised to -1, so it holds the overdensity)
-//   ck    3 * Mc      complex64 half spectra (r2c output; the Fourier kernel
-//                     writes the three gradient spectra over it)
-//   g     3 * M       real acceleration meshes (planar, one per axis)
+//   ck    3 * Mc      complex64: half rows of the own transforms (with the plane
+//                     kernels their spectra); on the cuFFT paths the half spectra
+//                     (the Fourier kernel writes the three gradients over them)
+//   g     3 * M       real acceleration meshes, plane-interleaved (x, 3, n1, n2)
+//                     (planar on the 3-D cuFFT path); the own transforms keep
+//                     their spectra here until the z axis writes it
 //   mcot  3 * M       cotangents of g (adjoint workspaces only)
 //   ktab  2*(n0+n1+n2h) angular wavenumbers, plain and Nyquist-masked
 //   part  4 * pstride float64 per-block partial sums of the dot products

@@ -90,9 +90,15 @@ def powspec(f, spacing, bins=1j / 3, g=None, deconv=None, cut_zero=True, cut_nyq
 def _to_device(dev, *arrays):
     """float64 arrays, flattened, in one copy that the host does not wait for
     (it would wait for the transforms too): from pinned memory, which the
-    caching allocator holds until the copy is done."""
+    caching allocator holds until the copy is done.  A capture would keep the
+    copy longer than that: there the plain copy refuses, as any upload does."""
     host = [a.reshape(-1).to(torch.float64) for a in arrays]
-    return torch.cat(host).pin_memory().to(dev, non_blocking=True).split([len(h) for h in host])
+    packed = torch.cat(host)
+    if torch.cuda.is_current_stream_capturing():
+        packed = packed.to(dev)
+    else:
+        packed = packed.pin_memory().to(dev, non_blocking=True)
+    return packed.split([len(h) for h in host])
 
 
 def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv, tabs=None):
