@@ -1297,7 +1297,9 @@ template <bool AGG = false>
 __global__ void __launch_bounds__(PT) k_gk_kds(Hot h, const int16_t *__restrict__ pmid, float *disp,
                                                float *vel, int64_t n, const float *__restrict__ g,
                                                float K2, float K1n, float Dn, float *dens) {
+    after_previous();
     gk_kds_body<AGG>(h, pmid, disp, vel, n, g, K2, K1n, Dn, dens);
+    next_may_start();
 }
 
 // k_sadj<true> of adjoint step i, then k_ka<true> of adjoint step i+1: the
@@ -1831,7 +1833,7 @@ int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStrea
     }
     {
         Stage sg(ws, adj ? 9 : 3, st, 1);
-        if ((e = mesh_xaxis(adj, nslot, g, s0, s1, tx, ws->ktab, gt, st))) return e;
+        if ((e = mesh_xaxis(adj, nslot, g, s0, s1, tx, ws->ktab, gt, st, plane))) return e;
     }
     Stage sg(ws, adj ? 10 : 4, st, ws->own_plane ? 1 : 2);
     if (ws->own_plane)
@@ -2741,7 +2743,8 @@ static int nbody_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int
                 k_gk_kds<true><<<G, PT, 0, s>>>(h, pmid, disp, vel, n, ws->g, f[2], f[3], f[4],
                                                 ws->dens);
             else
-                k_gk_kds<<<G, PT, 0, s>>>(h, pmid, disp, vel, n, ws->g, f[2], f[3], f[4], ws->dens);
+                PMX_CUDA(launch_after(ws->own_plane, k_gk_kds<false>, G, PT, 0, s, h, pmid, disp, vel, n,
+                                      ws->g, f[2], f[3], f[4], ws->dens));
             PMX_LAUNCH_CHECK("k_gk_kds");
         } else {
             Stage sg(ws, 5, s, 1);
