@@ -457,7 +457,9 @@ __global__ void __launch_bounds__(ST, 6) k_powspec_runs(Pow2Args a) {
     float *Ps = rows + warp * (CROSS ? 2 : 1) * rowlen, *Qs = Ps + rowlen;   // P N: re, im
     const int ax = (int)a.ax, ay = (int)a.ay, az = (int)a.az;
     // consecutive units per warp, so that a lane's bin hardly moves between them
-    const int64_t units = (int64_t)n2h * n0 * U, nw = (int64_t)gridDim.x * (ST / 32);
+    // (of rows longer than a unit, first all their first units, and so on)
+    const int nrows = n2h * n0;
+    const int64_t units = (int64_t)nrows * U, nw = (int64_t)gridDim.x * (ST / 32);
     const int64_t per = (units + nw - 1) / nw, w = (int64_t)blockIdx.x * (ST / 32) + warp;
     const int64_t u0 = w * per, u1 = u0 + per < units ? u0 + per : units;
     int cur = 0, lo = T[0];
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(ST, 6) k_powspec_runs(Pow2Args a) {
         an = 0;
     };
     for (int64_t u = u0; u < u1; ++u) {
-        const int row = (int)(u / U), sub = (int)(u - (int64_t)row * U);
+        const int sub = (int)(u / nrows), row = (int)(u - (int64_t)sub * nrows);
         const int l = row / n0, i = row - l * n0, si = i <= h0 / 2 ? i : i - h0;
         const int mrow = si * si * ax + l * l * az;
         const bool two = !(l == 0 || (a.nyq_z && l == n2h - 1));
