@@ -216,6 +216,7 @@ namespace pmx {
 // ---------------------------------------------------------------------------
 
 __global__ void k_fill(float *p, float v, int64_t n) {
+    after_previous();
     int64_t n4 = n >> 2;
     float4 v4 = make_float4(v, v, v, v);
     float4 *p4 = reinterpret_cast<float4 *>(p);
@@ -901,6 +902,7 @@ template <bool KD, bool WIN, bool KAHAN, bool AGG = false>
 __global__ void __launch_bounds__(PT) k_kds(Hot h, const int16_t *__restrict__ pmid, float *disp,
                                             float *vel, const float *__restrict__ acc, int64_t n,
                                             float K1, float D, float *dens) {
+    after_previous();
     kds_body<KD, WIN, KAHAN, AGG>(h, pmid, disp, vel, acc, n, K1, D, dens);
 }
 
@@ -1045,6 +1047,7 @@ __global__ void __launch_bounds__(PT) k_gather3(Hot h, const int16_t *__restrict
                                                 const float *__restrict__ disp, float *vel,
                                                 float *acc, int64_t n, int64_t M,
                                                 const float *__restrict__ g, float K2) {
+    after_previous();
     gather3_body<KICK, KAHAN>(h, pmid, disp, vel, acc, n, M, g, K2);
 }
 
@@ -1125,6 +1128,7 @@ __global__ void __launch_bounds__(PT) k_ka(Hot h, const int16_t *__restrict__ pm
                                            float *disp_cot, float *vel_cot,
                                            const float *__restrict__ alpha, int64_t n, float K1,
                                            float D, float *dens, double *part) {
+    after_previous();
     ka_body<KD, WIN, KAHAN, AGG>(h, pmid, disp, vel, acc, disp_cot, vel_cot, alpha, n, K1, D, dens,
                                  part);
 }
@@ -1203,6 +1207,7 @@ __global__ void __launch_bounds__(PT, 4) k_g3adj(Hot h, const int16_t *__restric
                                               float *alpha, int64_t n, int64_t M,
                                               const float *__restrict__ g, float *mcot,
                                               double *part) {
+    after_previous();
     g3adj_body<WIN, AGG>(h, pmid, disp, vel_cot, acc, alpha, n, M, g, mcot, part);
 }
 
@@ -1237,6 +1242,7 @@ __global__ void __launch_bounds__(PT) k_sadj(Hot h, const int16_t *__restrict__ 
                                              const float *__restrict__ acc, float *disp_cot,
                                              float *alpha, int64_t n,
                                              const float *__restrict__ rho_cot, float K2) {
+    after_previous();
     sadj_body<KICK, KAHAN>(h, pmid, disp, vel, acc, disp_cot, alpha, n, rho_cot, K2);
 }
 
@@ -1299,7 +1305,6 @@ __global__ void __launch_bounds__(PT) k_gk_kds(Hot h, const int16_t *__restrict_
                                                float K2, float K1n, float Dn, float *dens) {
     after_previous();
     gk_kds_body<AGG>(h, pmid, disp, vel, n, g, K2, K1n, Dn, dens);
-    next_may_start();
 }
 
 // k_sadj<true> of adjoint step i, then k_ka<true> of adjoint step i+1: the
@@ -1386,6 +1391,7 @@ __global__ void __launch_bounds__(PT) k_sa_ka(Hot h, const int16_t *__restrict__
                                               int64_t n, const float *__restrict__ rho_cot,
                                               float K2, float K1n, float Dn, float *dens,
                                               double *part) {
+    after_previous();
     sa_ka_body<AGG>(h, pmid, disp, vel, acc, disp_cot, vel_cot, alpha, n, rho_cot, K2, K1n, Dn,
                     dens, part);
 }
@@ -1398,6 +1404,7 @@ __global__ void __launch_bounds__(PT) k_sa_ka(Hot h, const int16_t *__restrict__
 // particles, side by side 10.
 __global__ void k_finish(const double *part, int64_t pstride, int nblk, int nblk2, double *dots,
                          int nslots, double *om_out, double om_scale) {
+    after_previous();
     __shared__ double sh[32];
     const int s = blockIdx.x;
     if (!((dots && s < nslots) || (om_out && s == 2))) return;
@@ -1833,7 +1840,7 @@ int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStrea
     }
     {
         Stage sg(ws, adj ? 9 : 3, st, 1);
-        if ((e = mesh_xaxis(adj, nslot, g, s0, s1, tx, ws->ktab, gt, st, plane))) return e;
+        if ((e = mesh_xaxis(adj, nslot, g, s0, s1, tx, ws->ktab, gt, st))) return e;
     }
     Stage sg(ws, adj ? 10 : 4, st, ws->own_plane ? 1 : 2);
     if (ws->own_plane)
@@ -2353,7 +2360,7 @@ extern "C" int pmx_force(pmx_workspace *ws, const pmx_enmesh_spec *spec, const i
     if ((st = ensure_ktab(ws, spec->conf_cell_size, s))) return st;
     {
         Stage sg(ws, 0, s, 1);
-        k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f, ws->M));
         PMX_LAUNCH_CHECK("k_fill");
     }
     if (n > 0) {
@@ -2373,8 +2380,8 @@ extern "C" int pmx_force(pmx_workspace *ws, const pmx_enmesh_spec *spec, const i
                 k_gather3_tma<false><<<ptcl_grid(ws, n), PT, TMA_SMEM, s>>>(
                     h, ws->tmap, pmid, disp, nullptr, acc, n, ws->g, 0.f, ws->err);
             else
-                k_gather3<false, false><<<ptcl_grid(ws, n), PT, 0, s>>>(h, pmid, disp, nullptr,
-                                                                    acc, n, ws->M, ws->g, 0.f);
+                PMX_CUDA(launch_after(k_gather3<false, false>, ptcl_grid(ws, n), PT, 0, s, h,
+                                      pmid, disp, nullptr, acc, n, ws->M, ws->g, 0.f));
             PMX_LAUNCH_CHECK("k_gather3");
         }
     }
@@ -2394,8 +2401,9 @@ extern "C" int pmx_force_vjp(pmx_workspace *ws, const pmx_enmesh_spec *spec, con
     if ((st = ensure_ktab(ws, spec->conf_cell_size, s))) return st;
     {
         Stage sg(ws, 0, s, 2);
-        k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
-        k_fill<<<grid_fill(3 * ws->M), 256, 0, s>>>(ws->mcot, 0.f, 3 * ws->M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f, ws->M));
+        PMX_CUDA(launch_after(k_fill, grid_fill(3 * ws->M), 256, 0, s, ws->mcot, 0.f,
+                              3 * ws->M));
         PMX_LAUNCH_CHECK("k_fill");
     }
     const int G = ptcl_grid(ws, n);
@@ -2416,11 +2424,11 @@ extern "C" int pmx_force_vjp(pmx_workspace *ws, const pmx_enmesh_spec *spec, con
                 k_g3adj<true><<<G, PT, WIN3_SMEM, s>>>(h, pmid, disp, acc_cot, acc, disp_cot, n, ws->M,
                                                        ws->g, ws->mcot, ws->part);
             else if (h.agg)
-                k_g3adj<false, true><<<G, PT, 0, s>>>(h, pmid, disp, acc_cot, acc, disp_cot, n, ws->M,
-                                                      ws->g, ws->mcot, ws->part);
+                PMX_CUDA(launch_after(k_g3adj<false, true>, G, PT, 0, s, h, pmid, disp,
+                                      acc_cot, acc, disp_cot, n, ws->M, ws->g, ws->mcot, ws->part));
             else
-                k_g3adj<false><<<G, PT, 0, s>>>(h, pmid, disp, acc_cot, acc, disp_cot, n, ws->M, ws->g,
-                                                ws->mcot, ws->part);
+                PMX_CUDA(launch_after(k_g3adj<false>, G, PT, 0, s, h, pmid, disp, acc_cot,
+                                      acc, disp_cot, n, ws->M, ws->g, ws->mcot, ws->part));
             PMX_LAUNCH_CHECK("k_g3adj");
         }
     }
@@ -2428,8 +2436,8 @@ extern "C" int pmx_force_vjp(pmx_workspace *ws, const pmx_enmesh_spec *spec, con
     if (n > 0) {
         {
             Stage sg(ws, 11, s, 1);
-            k_sadj<false, false><<<G, PT, 0, s>>>(h, pmid, disp, nullptr, nullptr, nullptr, disp_cot,
-                                                  n, ws->rcot_of(1), 0.f);
+            PMX_CUDA(launch_after(k_sadj<false, false>, G, PT, 0, s, h, pmid, disp, nullptr,
+                                  nullptr, nullptr, disp_cot, n, ws->rcot_of(1), 0.f));
             PMX_LAUNCH_CHECK("k_sadj");
         }
     }
@@ -2439,8 +2447,8 @@ extern "C" int pmx_force_vjp(pmx_workspace *ws, const pmx_enmesh_spec *spec, con
         } else {
             {
                 Stage sg(ws, 12, s, 1);
-                k_finish<<<3, 1024, 0, s>>>(ws->part, ws->pstride, G, G, nullptr, 0, omega_m_cot,
-                                            om_scale(omega_m));
+                PMX_CUDA(launch_after(k_finish, 3, 1024, 0, s, ws->part, ws->pstride, G, G,
+                                      nullptr, 0, omega_m_cot, om_scale(omega_m)));
                 PMX_LAUNCH_CHECK("k_finish");
             }
         }
@@ -2552,7 +2560,7 @@ static int nbody_step(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int1
     if ((st = ensure_ktab(ws, spec->conf_cell_size, s))) return st;
     {
         Stage sg(ws, 0, s, 1);
-        k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f, ws->M));
         PMX_LAUNCH_CHECK("k_fill");
     }
     const int G = ptcl_grid(ws, n);
@@ -2569,14 +2577,14 @@ static int nbody_step(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int1
         {
             Stage sg(ws, 5, s, 1);
             if (h.vcomp)
-                k_gather3<true, true><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, n, ws->M, ws->g,
-                                                       factors[2]);
+                PMX_CUDA(launch_after(k_gather3<true, true>, G, PT, 0, s, h, pmid, disp, vel,
+                                      acc, n, ws->M, ws->g, factors[2]));
             else if (ws->tma)
                 k_gather3_tma<true><<<G, PT, TMA_SMEM, s>>>(h, ws->tmap, pmid, disp, vel, acc, n,
                                                             ws->g, factors[2], ws->err);
             else
-                k_gather3<true, false><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, n, ws->M, ws->g,
-                                                        factors[2]);
+                PMX_CUDA(launch_after(k_gather3<true, false>, G, PT, 0, s, h, pmid, disp, vel,
+                                      acc, n, ws->M, ws->g, factors[2]));
             PMX_LAUNCH_CHECK("k_gather3");
         }
     }
@@ -2601,8 +2609,9 @@ static int nbody_adj_step(pmx_workspace *ws, const pmx_enmesh_spec *spec, const 
     if ((st = ensure_ktab(ws, spec->conf_cell_size, s))) return st;
     {
         Stage sg(ws, 0, s, 2);
-        k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
-        k_fill<<<grid_fill(3 * ws->M), 256, 0, s>>>(ws->mcot, 0.f, 3 * ws->M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f, ws->M));
+        PMX_CUDA(launch_after(k_fill, grid_fill(3 * ws->M), 256, 0, s, ws->mcot, 0.f,
+                              3 * ws->M));
         PMX_LAUNCH_CHECK("k_fill");
     }
     if (n == 0) {
@@ -2624,28 +2633,28 @@ static int nbody_adj_step(pmx_workspace *ws, const pmx_enmesh_spec *spec, const 
             k_g3adj<true><<<G, PT, WIN3_SMEM, s>>>(h, pmid, disp, vel_cot, acc, acc_cot, n, ws->M,
                                                    ws->g, ws->mcot, ws->part);
         else if (h.agg)
-            k_g3adj<false, true><<<G, PT, 0, s>>>(h, pmid, disp, vel_cot, acc, acc_cot, n, ws->M,
-                                                  ws->g, ws->mcot, ws->part);
+            PMX_CUDA(launch_after(k_g3adj<false, true>, G, PT, 0, s, h, pmid, disp, vel_cot,
+                                  acc, acc_cot, n, ws->M, ws->g, ws->mcot, ws->part));
         else
-            k_g3adj<false><<<G, PT, 0, s>>>(h, pmid, disp, vel_cot, acc, acc_cot, n, ws->M, ws->g,
-                                            ws->mcot, ws->part);
+            PMX_CUDA(launch_after(k_g3adj<false>, G, PT, 0, s, h, pmid, disp, vel_cot, acc,
+                                  acc_cot, n, ws->M, ws->g, ws->mcot, ws->part));
         PMX_LAUNCH_CHECK("k_g3adj");
     }
     if ((st = force_adj_meshes(ws, omega_m, s))) return st;
     {
         Stage sg(ws, 11, s, 1);
         if (h.vcomp)
-            k_sadj<true, true><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot, acc_cot, n,
-                                                ws->rcot_of(1), factors[2]);
+            PMX_CUDA(launch_after(k_sadj<true, true>, G, PT, 0, s, h, pmid, disp, vel, acc,
+                                  disp_cot, acc_cot, n, ws->rcot_of(1), factors[2]));
         else
-            k_sadj<true, false><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot, acc_cot, n,
-                                                 ws->rcot_of(1), factors[2]);
+            PMX_CUDA(launch_after(k_sadj<true, false>, G, PT, 0, s, h, pmid, disp, vel, acc,
+                                  disp_cot, acc_cot, n, ws->rcot_of(1), factors[2]));
         PMX_LAUNCH_CHECK("k_sadj");
     }
     {
         Stage sg(ws, 12, s, 1);
-        k_finish<<<3, 1024, 0, s>>>(ws->part, ws->pstride, G2, G, dots, 3, dots + 3,
-                                    om_scale(omega_m));
+        PMX_CUDA(launch_after(k_finish, 3, 1024, 0, s, ws->part, ws->pstride, G2, G, dots, 3,
+                              dots + 3, om_scale(omega_m)));
         PMX_LAUNCH_CHECK("k_finish");
     }
     return PMX_OK;
@@ -2716,17 +2725,17 @@ static int nbody_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int
     const int G = ptcl_grid(ws, n);
     {
         Stage sg(ws, 0, s, 1);
-        k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f, ws->M));
         PMX_LAUNCH_CHECK("k_fill");
     }
     {
         Stage sg(ws, 1, s, 1);
         if (h.agg)
-            k_kds<true, false, false, true><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, n, factors[0],
-                                                             factors[1], ws->dens);
+            PMX_CUDA(launch_after(k_kds<true, false, false, true>, G, PT, 0, s, h, pmid, disp,
+                                  vel, acc, n, factors[0], factors[1], ws->dens));
         else
-            k_kds<true, false, false><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, n, factors[0],
-                                                         factors[1], ws->dens);
+            PMX_CUDA(launch_after(k_kds<true, false, false>, G, PT, 0, s, h, pmid, disp, vel,
+                                  acc, n, factors[0], factors[1], ws->dens));
         PMX_LAUNCH_CHECK("k_kds");
     }
     for (int32_t i = 0; i < nsteps; ++i) {
@@ -2735,15 +2744,16 @@ static int nbody_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int
         if (i + 1 < nsteps) {
             if (!ws->own_plane) {   // whose forward kernel leaves dens filled
                 Stage sg(ws, 0, s, 1);
-                k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
+                PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f,
+                                      ws->M));
                 PMX_LAUNCH_CHECK("k_fill");
             }
             Stage sg(ws, 13, s, 1);
             if (h.agg)
-                k_gk_kds<true><<<G, PT, 0, s>>>(h, pmid, disp, vel, n, ws->g, f[2], f[3], f[4],
-                                                ws->dens);
+                PMX_CUDA(launch_after(k_gk_kds<true>, G, PT, 0, s, h, pmid, disp, vel, n,
+                                      ws->g, f[2], f[3], f[4], ws->dens));
             else
-                PMX_CUDA(launch_after(ws->own_plane, k_gk_kds<false>, G, PT, 0, s, h, pmid, disp, vel, n,
+                PMX_CUDA(launch_after(k_gk_kds<false>, G, PT, 0, s, h, pmid, disp, vel, n,
                                       ws->g, f[2], f[3], f[4], ws->dens));
             PMX_LAUNCH_CHECK("k_gk_kds");
         } else {
@@ -2752,8 +2762,8 @@ static int nbody_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const int
                 k_gather3_tma<true><<<G, PT, TMA_SMEM, s>>>(h, ws->tmap, pmid, disp, vel, acc, n,
                                                             ws->g, f[2], ws->err);
             else
-                k_gather3<true, false><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, n, ws->M, ws->g,
-                                                        f[2]);
+                PMX_CUDA(launch_after(k_gather3<true, false>, G, PT, 0, s, h, pmid, disp, vel,
+                                      acc, n, ws->M, ws->g, f[2]));
             PMX_LAUNCH_CHECK("k_gather3");
         }
     }
@@ -2787,20 +2797,21 @@ static int nbody_adj_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const
     int nb01 = G2;  // blocks of the kernel that last wrote dot slots 0 and 1
     {
         Stage sg(ws, 0, s, 2);
-        k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
-        k_fill<<<grid_fill(3 * ws->M), 256, 0, s>>>(ws->mcot, 0.f, 3 * ws->M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f, ws->M));
+        PMX_CUDA(launch_after(k_fill, grid_fill(3 * ws->M), 256, 0, s, ws->mcot, 0.f,
+                              3 * ws->M));
         PMX_LAUNCH_CHECK("k_fill");
     }
     {
         Stage sg(ws, 6, s, 1);
         if (h.agg)
-            k_ka<true, false, false, true><<<G2, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot,
-                                                             vel_cot, acc_cot, n, factors[0],
-                                                             factors[1], ws->dens, ws->part);
+            PMX_CUDA(launch_after(k_ka<true, false, false, true>, G2, PT, 0, s, h, pmid, disp,
+                                  vel, acc, disp_cot, vel_cot, acc_cot, n, factors[0], factors[1],
+                                  ws->dens, ws->part));
         else
-            k_ka<true, false, false><<<G2, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot, vel_cot,
-                                                         acc_cot, n, factors[0], factors[1],
-                                                         ws->dens, ws->part);
+            PMX_CUDA(launch_after(k_ka<true, false, false>, G2, PT, 0, s, h, pmid, disp, vel,
+                                  acc, disp_cot, vel_cot, acc_cot, n, factors[0], factors[1],
+                                  ws->dens, ws->part));
         PMX_LAUNCH_CHECK("k_ka");
     }
     for (int32_t i = 0; i < nsteps; ++i) {
@@ -2809,18 +2820,17 @@ static int nbody_adj_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const
         {
             Stage sg(ws, 7, s, 1);
             if (h.agg)
-                k_g3adj<false, true><<<G, PT, 0, s>>>(h, pmid, disp, vel_cot, acc, acc_cot, n, ws->M,
-                                                      ws->g, ws->mcot, ws->part);
+                PMX_CUDA(launch_after(k_g3adj<false, true>, G, PT, 0, s, h, pmid, disp,
+                                      vel_cot, acc, acc_cot, n, ws->M, ws->g, ws->mcot, ws->part));
             else
-                k_g3adj<false><<<G, PT, 0, s>>>(h, pmid, disp, vel_cot, acc, acc_cot, n, ws->M,
-                                                ws->g, ws->mcot, ws->part);
+                PMX_CUDA(launch_after(k_g3adj<false>, G, PT, 0, s, h, pmid, disp, vel_cot,
+                                      acc, acc_cot, n, ws->M, ws->g, ws->mcot, ws->part));
             PMX_LAUNCH_CHECK("k_g3adj");
         }
         {
             Stage sg(ws, 12, s, 1);
-            k_finish<<<3, 1024, 0, s>>>(ws->part, ws->pstride, nb01, G, dots + 4 * i, 3,
-                                        dots + 4 * i + 3,
-                                        om_scale(omega_m));
+            PMX_CUDA(launch_after(k_finish, 3, 1024, 0, s, ws->part, ws->pstride, nb01, G,
+                                  dots + 4 * i, 3, dots + 4 * i + 3, om_scale(omega_m)));
             PMX_LAUNCH_CHECK("k_finish");
         }
         if ((st = force_adj_meshes(ws, omega_m, s))) return st;
@@ -2828,25 +2838,27 @@ static int nbody_adj_steps(pmx_workspace *ws, const pmx_enmesh_spec *spec, const
             {
                 Stage sg(ws, 0, s, ws->own_plane ? 1 : 2);
                 if (!ws->own_plane)
-                    k_fill<<<grid_fill(ws->M), 256, 0, s>>>(ws->dens, -1.f, ws->M);
-                k_fill<<<grid_fill(3 * ws->M), 256, 0, s>>>(ws->mcot, 0.f, 3 * ws->M);
+                    PMX_CUDA(launch_after(k_fill, grid_fill(ws->M), 256, 0, s, ws->dens, -1.f,
+                                          ws->M));
+                PMX_CUDA(launch_after(k_fill, grid_fill(3 * ws->M), 256, 0, s, ws->mcot, 0.f,
+                                      3 * ws->M));
                 PMX_LAUNCH_CHECK("k_fill");
             }
             Stage sg(ws, 14, s, 1);
             if (h.agg)
-                k_sa_ka<true><<<G2, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot, vel_cot,
-                                                   acc_cot, n, ws->rcot_of(1), f[2], f[3], f[4],
-                                                   ws->dens, ws->part);
+                PMX_CUDA(launch_after(k_sa_ka<true>, G2, PT, 0, s, h, pmid, disp, vel, acc,
+                                      disp_cot, vel_cot, acc_cot, n, ws->rcot_of(1), f[2], f[3],
+                                      f[4], ws->dens, ws->part));
             else
-                k_sa_ka<<<G2, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot, vel_cot, acc_cot,
-                                             n, ws->rcot_of(1), f[2], f[3], f[4], ws->dens,
-                                             ws->part);
+                PMX_CUDA(launch_after(k_sa_ka<false>, G2, PT, 0, s, h, pmid, disp, vel, acc,
+                                      disp_cot, vel_cot, acc_cot, n, ws->rcot_of(1), f[2], f[3],
+                                      f[4], ws->dens, ws->part));
             PMX_LAUNCH_CHECK("k_sa_ka");
             nb01 = G2;
         } else {
             Stage sg(ws, 11, s, 1);
-            k_sadj<true, false><<<G, PT, 0, s>>>(h, pmid, disp, vel, acc, disp_cot, acc_cot, n,
-                                                 ws->rcot_of(1), f[2]);
+            PMX_CUDA(launch_after(k_sadj<true, false>, G, PT, 0, s, h, pmid, disp, vel, acc,
+                                  disp_cot, acc_cot, n, ws->rcot_of(1), f[2]));
             PMX_LAUNCH_CHECK("k_sadj");
         }
     }
@@ -2954,7 +2966,7 @@ extern "C" int pmx_nbody_steps_batch(pmx_workspace *ws, const pmx_enmesh_spec *s
     const dim3 grid(bc.G, bc.nb);
     auto fill_dens = [&]() -> int {
         Stage sg(ws, 0, s, 1);
-        k_fill<<<grid_fill(nb * M), 256, 0, s>>>(ws->dens, -1.f, nb * M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(nb * M), 256, 0, s, ws->dens, -1.f, nb * M));
         PMX_LAUNCH_CHECK("k_fill");
         return PMX_OK;
     };
@@ -3015,8 +3027,9 @@ extern "C" int pmx_nbody_adj_steps_batch(pmx_workspace *ws, const pmx_enmesh_spe
     float *rcot = ws->rcot_of(bc.nb);
     auto fills = [&]() -> int {
         Stage sg(ws, 0, s, 2);
-        k_fill<<<grid_fill(nb * M), 256, 0, s>>>(ws->dens, -1.f, nb * M);
-        k_fill<<<grid_fill(3 * nb * M), 256, 0, s>>>(ws->mcot, 0.f, 3 * nb * M);
+        PMX_CUDA(launch_after(k_fill, grid_fill(nb * M), 256, 0, s, ws->dens, -1.f, nb * M));
+        PMX_CUDA(launch_after(k_fill, grid_fill(3 * nb * M), 256, 0, s, ws->mcot, 0.f,
+                              3 * nb * M));
         PMX_LAUNCH_CHECK("k_fill");
         return PMX_OK;
     };

@@ -117,7 +117,7 @@ int mesh_plane_prepare(int64_t n1, int64_t n2, bool *fits);
 int mesh_plane(int kind, int nslot, const MeshGeom &g, float *mesh, float2 *spec0, float2 *spec1,
                const float2 *twy, const float2 *twz, const float *kt, cudaStream_t st);
 int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, const float2 *tw,
-               const float *kt, const GreenTab &gt, cudaStream_t st, bool overlap = false);
+               const float *kt, const GreenTab &gt, cudaStream_t st);
 
 // Fused x-axis pass of the Poisson solve (pmx_fft.cu).  Forward (adj =
 // false): in = FFT_yz(rho) (n0, n1, n2h), out = the three gradient spectra
@@ -310,18 +310,16 @@ __device__ __forceinline__ double to_f64(float x) {
                             (int)(u << 29));
 }
 
-// Programmatic dependent launch: a kernel launched by launch_after starts while the
-// stream's previous kernel ends; it waits in after_previous() until that one's
-// memory operations are visible, before it touches global memory.  Every kernel of such
-// a chain waits, so each sees all earlier ones.  next_may_start() is called where a
-// block has nothing left to do; without these launches both are no-ops.
+// Programmatic dependent launch: a kernel launched by launch_after is set up while
+// the stream's previous kernel ends; it waits in after_previous() until that one is
+// done and its memory operations are visible, before it touches global memory.
+// Every kernel of such a chain waits, so each sees all earlier ones.  It saves the
+// 1 to 2 us between two kernels.  Without such a launch after_previous() returns at
+// once.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void next_may_start() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 template <class... K, class... A>
-cudaError_t launch_after(bool overlap, void (*fn)(K...), dim3 grid, int block, size_t smem,
-                         cudaStream_t st, A... args) {
+cudaError_t launch_after(void (*fn)(K...), dim3 grid, int block, size_t smem, cudaStream_t st,
+                         A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
@@ -331,7 +329,7 @@ cudaError_t launch_after(bool overlap, void (*fn)(K...), dim3 grid, int block, s
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = overlap ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, fn, K(args)...);
 }
 

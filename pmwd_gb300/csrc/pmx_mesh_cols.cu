@@ -61,6 +61,7 @@ k_cols_fwd(const float2 *__restrict__ nat,
     const int t = threadIdx.x % C::T, b = threadIdx.x / C::T;
     const int xi = t >> 2, l = c.zt * 4 + (t & 3);
     const float2 *src = nat + (c.p + xi) * (g.n1 * 4 * g.nzt) + c.zt * 32 + (t & 3);
+    after_previous();
     float2 v[C::R1];
     static_for<C::R1>([&](auto A) { v[A] = src[nat_row<A * C::R2>(g.nzt, b)]; });
     col_stage1<C, false>(v, sm, t, b, tw);
@@ -93,6 +94,7 @@ k_cols_adj(const float2 *__restrict__ nat,
     const int64_t ps = g.n1 * 4 * g.nzt;
     const float2 *src = nat + (c.p + xi) * 3 * ps + c.zt * 32 + (t & 3);
     const int64_t x = c.p % g.n0 + xi, slot = c.p / g.n0;
+    after_previous();
     float2 v[C::R1];
     if (c.comp == 0) {
         static_for<C::R1>([&](auto A) { v[A] = src[nat_row<A * C::R2>(g.nzt, b)]; });
@@ -165,6 +167,7 @@ k_cols_inv(const float2 *__restrict__ spec0,
     const float2 *src = (NC == 3 && c.comp ? spec1 : spec0) + slot * g.unit + spec_at(g, x, 0, l);
     if (NC == 6) src += (c.comp == 0 ? 0 : (c.comp == 3 || c.comp == 4 ? 1 : 2)) * g.unit;
     const int64_t ys = (int64_t)g.nzt * 32;
+    after_previous();
     float2 v[C::R1];
 #pragma unroll
     for (int a = 0; a < C::R1; ++a) v[a] = src[(b + a * C::R2) * ys];
@@ -230,23 +233,24 @@ int mesh_cols(int kind, int nslot, const MeshGeom &g, float2 *nat, float2 *spec0
         const int64_t tiles = nslot * g.n0 / (C::T / 4) * g.nzt;
         switch (kind) {
             case MESH_COLS_FWD:
-                k_cols_fwd<N><<<(unsigned)tiles, C::TH, cols_smem<YCol<N>>(1), st>>>(nat, spec0, tw, g);
+                PMX_CUDA(launch_after(k_cols_fwd<N>, (unsigned)tiles, C::TH, cols_smem<YCol<N>>(1),
+                                      st, nat, spec0, tw, g));
                 break;
             case MESH_COLS_ADJ:
-                k_cols_adj<N><<<(unsigned)(2 * tiles), C::TH, cols_smem<YCol<N>>(2), st>>>(nat, spec0, spec1,
-                                                                                     tw, kt, g);
+                PMX_CUDA(launch_after(k_cols_adj<N>, (unsigned)(2 * tiles), C::TH,
+                                      cols_smem<YCol<N>>(2), st, nat, spec0, spec1, tw, kt, g));
                 break;
             case MESH_COLS_INV1:
-                k_cols_inv<N, 1><<<(unsigned)tiles, C::TH, cols_smem<YCol<N>>(1), st>>>(spec0, nullptr, nat,
-                                                                                  tw, kt, g);
+                PMX_CUDA(launch_after(k_cols_inv<N, 1>, (unsigned)tiles, C::TH,
+                                      cols_smem<YCol<N>>(1), st, spec0, nullptr, nat, tw, kt, g));
                 break;
             case MESH_COLS_INV6:
-                k_cols_inv<N, 6><<<(unsigned)(6 * tiles), C::TH, cols_smem<YCol<N>>(1), st>>>(
-                    spec0, nullptr, nat, tw, kt, g);
+                PMX_CUDA(launch_after(k_cols_inv<N, 6>, (unsigned)(6 * tiles), C::TH,
+                                      cols_smem<YCol<N>>(1), st, spec0, nullptr, nat, tw, kt, g));
                 break;
             default:
-                k_cols_inv<N, 3><<<(unsigned)(3 * tiles), C::TH, cols_smem<YCol<N>>(1), st>>>(spec0, spec1,
-                                                                                        nat, tw, kt, g);
+                PMX_CUDA(launch_after(k_cols_inv<N, 3>, (unsigned)(3 * tiles), C::TH,
+                                      cols_smem<YCol<N>>(1), st, spec0, spec1, nat, tw, kt, g));
         }
         PMX_LAUNCH_CHECK("mesh transform, y axis");
         return PMX_OK;

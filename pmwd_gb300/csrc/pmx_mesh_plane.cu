@@ -257,7 +257,6 @@ k_plane_fwd(float *in, float fill, float2 *__restrict__ spec, const float2 *__re
         e[0] = make_float4(0.5f * (a.y + m.y), -0.5f * (a.x - m.x), 0.f, 0.f);
         e[1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    next_may_start();
 }
 
 // Spectra -> real planes: NC = 1, one spectrum per slot; NC = 3, G_0 (spec0) and Q
@@ -328,7 +327,6 @@ k_plane_inv(const float2 *__restrict__ spec0, const float2 *__restrict__ spec1,
     const int y = threadIdx.x / R::TPR, lane = threadIdx.x % R::TPR;
     row_inv<L>(sm + y * R::RS, reinterpret_cast<float2 *>(out) + (id * N + y) * L, lane, twz,
                twz + 2 * L);
-    next_may_start();
 }
 
 template <class F>
@@ -362,13 +360,13 @@ int mesh_plane(int kind, int nslot, const MeshGeom &g, float *mesh, float2 *spec
         using P = PlaneCfg<N>;
         const unsigned planes = (unsigned)(nslot * g.n0);
         if (kind == MESH_COLS_FWD)
-            PMX_CUDA(launch_after(true, k_plane_fwd<N>, planes, P::TH, P::SMEM, st, mesh, -1.f, spec0, twy,
-                                  twz, g));
+            PMX_CUDA(launch_after(k_plane_fwd<N>, planes, P::TH, P::SMEM, st, mesh, -1.f, spec0,
+                                  twy, twz, g));
         else if (kind == MESH_COLS_INV1)
-            PMX_CUDA(launch_after(true, k_plane_inv<N, 1>, planes, P::TH, P::SMEM, st, spec0, nullptr,
+            PMX_CUDA(launch_after(k_plane_inv<N, 1>, planes, P::TH, P::SMEM, st, spec0, nullptr,
                                   mesh, twy, twz, kt, g));
         else
-            PMX_CUDA(launch_after(true, k_plane_inv<N, 3>, 3 * planes, P::TH, P::SMEM, st, spec0, spec1,
+            PMX_CUDA(launch_after(k_plane_inv<N, 3>, 3 * planes, P::TH, P::SMEM, st, spec0, spec1,
                                   mesh, twy, twz, kt, g));
         PMX_LAUNCH_CHECK("mesh transform, z and y axes");
         return PMX_OK;

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(RowCfg<L>::TH) k_rows_r2c(const float *__restr
     const float2 *src = reinterpret_cast<const float2 *>(in) + (row0 + r) * L;
     constexpr int IT = (R2 + TPR - 1) / TPR;
     float2 v[IT][R1];
+    after_previous();
 #pragma unroll
     for (int i = 0; i < IT; ++i)   // every load before the first use
         if (R2 % TPR == 0 || i * TPR + lane < R2) {
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(RowCfg<L>::TH) k_rows_c2r(const float2 *__rest
     const RowPairs<L> pr(lane);
     float2 u0[R2], u1[R2];
     const float2 *in = nat + row0 * (4 * C::NZT);
+    after_previous();
     for (int i = threadIdx.x; i < C::ROWS * 2 * C::NZT; i += C::TH)
         cp_async16(sm + (i >> 4) * ZB + (i & 15) * 2, in + 2 * i);
     cp_async_wait();
@@ -246,11 +248,11 @@ int mesh_rows(bool inv, const void *in, void *out, const float2 *tw, int64_t pla
         using C = RowCfg<L>;
         const unsigned grid = (unsigned)(planes * n1 / C::ROWS);
         if (inv)
-            k_rows_c2r<L><<<grid, C::TH, rows_smem<L>(), st>>>((const float2 *)in, (float *)out,
-                                                                   tw, tw + 2 * L);
+            PMX_CUDA(launch_after(k_rows_c2r<L>, grid, C::TH, rows_smem<L>(), st,
+                                  (const float2 *)in, (float *)out, tw, tw + 2 * L));
         else
-            k_rows_r2c<L><<<grid, C::TH, rows_smem<L>(), st>>>((const float *)in, (float2 *)out,
-                                                                    tw, tw + 2 * L);
+            PMX_CUDA(launch_after(k_rows_r2c<L>, grid, C::TH, rows_smem<L>(), st, (const float *)in,
+                                  (float2 *)out, tw, tw + 2 * L));
         PMX_LAUNCH_CHECK("mesh transform, z axis");
         return PMX_OK;
     });

@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(2, x_regs<N>(
     if (!ok) return;
     x_inv_step1<N>(B, t, b, p0, xbs);
     x_inv_step1<N>(A, t, b, p1, xbs);
-    next_may_start();
 }
 
 // s0: C_0 in, S out (in place); s1: D in.
@@ -132,6 +131,7 @@ __global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(2, x_regs<N>(
     const int64_t xbs = g.n1 * g.nzt * 32;
     const int64_t at = blockIdx.y * g.unit + ((int64_t)ky * g.nzt + (ok ? l >> 2 : 0)) * 32 + (l & 3);
     float2 *p0 = s0 + at;
+    after_previous();
 #pragma unroll 1
     for (int j = 0; j < 2; ++j) {
         const float2 *p = j ? s1 + at : p0;
@@ -276,15 +276,16 @@ int mesh_xaxis_prepare(int64_t n0) {
 }
 
 int mesh_xaxis(bool adj, int nslot, const MeshGeom &g, float2 *s0, float2 *s1, const float2 *tw,
-               const float *kt, const GreenTab &gt, cudaStream_t st, bool overlap) {
+               const float *kt, const GreenTab &gt, cudaStream_t st) {
     return mesh_axis_dispatch(g.n0, [&](auto N) -> int {
         using C = XCol<N>;
         const dim3 grid((unsigned)(g.n1 * ((4 * g.nzt + C::T - 1) / C::T)), nslot);
         if (adj)
-            k_xaxis_adj<N><<<grid, C::TH, cols_smem<XCol<N>>(2), st>>>(s0, s1, tw, kt, gt, g);
+            PMX_CUDA(launch_after(k_xaxis_adj<N>, grid, C::TH, cols_smem<XCol<N>>(2), st, s0, s1,
+                                  tw, kt, gt, g));
         else
-            PMX_CUDA(launch_after(overlap, k_xaxis_fwd<N>, grid, C::TH, cols_smem<XCol<N>>(2), st, s0,
-                                  s1, tw, kt, gt, g));
+            PMX_CUDA(launch_after(k_xaxis_fwd<N>, grid, C::TH, cols_smem<XCol<N>>(2), st, s0, s1,
+                                  tw, kt, gt, g));
         PMX_LAUNCH_CHECK("mesh transform, x axis");
         return PMX_OK;
     });
