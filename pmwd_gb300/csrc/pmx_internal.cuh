@@ -315,7 +315,9 @@ __device__ __forceinline__ double to_f64(float x) {
 // done and its memory operations are visible, before it touches global memory.
 // Every kernel of such a chain waits, so each sees all earlier ones.  It saves the
 // 1 to 2 us between two kernels.  Without such a launch after_previous() returns at
-// once.
+// once.  The next kernel is set up as blocks exit: allowed from a block's start on
+// (griddepcontrol.launch_dependents), its waiting blocks take the room of the large
+// meshes' kernels (8 steps of 256^3 particles on 512^3: 57.9 ms against 28.5).
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... K, class... A>
 cudaError_t launch_after(void (*fn)(K...), dim3 grid, int block, size_t smem, cudaStream_t st,
