@@ -89,3 +89,42 @@ def test_batched_equals_single():
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert _rel(a, b) < 1e-6   # the order of the float32 deposits differs
+
+
+@pytest.mark.parametrize('shape', ((64, 64, 64), (128, 192, 192)))
+def test_captured_steps_replay(shape):
+    """Multi-step calls under stream capture, between copies: the kernels' programmatic
+    launches become graph edges.  The deposits' order differs, as between two runs."""
+    import pmwd_gb300 as pg
+    from pmwd_gb300 import _lib
+    conf = pg.Configuration(1.0, tuple(n // 2 for n in shape), mesh_shape=2)
+    gen = torch.Generator(device='cuda')
+    gen.manual_seed(5)
+    p = pg.Particles.gen_grid(conf)
+    start = p.disp + 0.3 * torch.randn(p.disp.shape, generator=gen, device='cuda')
+    disp, vel, acc = start.clone(), torch.zeros_like(start), torch.zeros_like(start)
+    spec = _lib.make_spec(3, conf.mesh_shape, conf.mesh_shape, conf.cell_size)
+    ws = _lib.Workspace(conf.mesh_shape)
+    fac = (_lib.c_f * 9)(*(0.01, 0.02, 0.01) * 3)
+    out = torch.empty_like(start)
+
+    def run():
+        disp.copy_(start)
+        vel.zero_()
+        acc.zero_()
+        _lib.call('pmx_force', ws.handle, spec, p.pmid, disp, len(p), conf.ptcl_num, 0.3, acc,
+                  _lib.stream_ptr())
+        _lib.call('pmx_nbody_steps', ws.handle, spec, p.pmid, disp, vel, acc, len(p),
+                  conf.ptcl_num, 3, fac, 0.3, _lib.stream_ptr())
+        out.copy_(vel)
+
+    run()
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run()
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert _rel(out, want) < 1e-6   # the order of the float32 deposits differs
