@@ -294,6 +294,7 @@ __device__ __forceinline__ Cell fourier_cell(int64_t e, int64_t n0, int64_t n1, 
 __global__ void __launch_bounds__(256) k_poisson_fwd(float2 *ck, int64_t n0, int64_t n1, int64_t n2h,
                                                      int64_t Mc, const float *__restrict__ kt,
                                                      float c) {
+    after_previous();
     const bool small = Mc <= 0xffffffffll;
     for (int64_t e0 = blockIdx.x * (int64_t)(256 * POIS) + threadIdx.x; e0 < Mc;
          e0 += (int64_t)gridDim.x * 256 * POIS) {
@@ -326,6 +327,7 @@ __global__ void __launch_bounds__(256) k_poisson_fwd(float2 *ck, int64_t n0, int
 __global__ void __launch_bounds__(256) k_poisson_adj(float2 *ck, int64_t n0, int64_t n1, int64_t n2h,
                                                      int64_t Mc, const float *__restrict__ kt,
                                                      float c) {
+    after_previous();
     const bool small = Mc <= 0xffffffffll;
     for (int64_t e0 = blockIdx.x * (int64_t)(256 * POIS) + threadIdx.x; e0 < Mc;
          e0 += (int64_t)gridDim.x * 256 * POIS) {
@@ -1901,8 +1903,8 @@ int force_meshes_b(pmx_workspace *ws, int nslot, const float *c, cudaStream_t st
     }
     {
         Stage sg(ws, 3, st, 1);
-        k_poisson_fwd<<<poisson_grid(ws), 256, 0, st>>>(ws->ck, ws->n0, ws->n1, ws->n2h, ws->Mc,
-                                                         ws->ktab, c0);
+        PMX_CUDA(launch_after(k_poisson_fwd, poisson_grid(ws), 256, 0, st, ws->ck, ws->n0, ws->n1,
+                              ws->n2h, ws->Mc, ws->ktab, c0));
         PMX_LAUNCH_CHECK("k_poisson_fwd");
     }
     {
@@ -1962,8 +1964,8 @@ int force_adj_meshes_b(pmx_workspace *ws, int nslot, const float *c, cudaStream_
     }
     {
         Stage sg(ws, 9, st, 1);
-        k_poisson_adj<<<poisson_grid(ws), 256, 0, st>>>(ws->ck, ws->n0, ws->n1, ws->n2h, ws->Mc,
-                                                         ws->ktab, c0);
+        PMX_CUDA(launch_after(k_poisson_adj, poisson_grid(ws), 256, 0, st, ws->ck, ws->n0, ws->n1,
+                              ws->n2h, ws->Mc, ws->ktab, c0));
         PMX_LAUNCH_CHECK("k_poisson_adj");
     }
     {

@@ -150,6 +150,7 @@ template <int V>
 __global__ void __launch_bounds__(LT) k_lpt_source(const float *__restrict__ phi,
                                                    float *__restrict__ L, int64_t pl, int64_t n0,
                                                    Fields f, float s) {
+    after_previous();
     for (int64_t x = blockIdx.y; x < n0; x += gridDim.y) {
         const float *ph = phi + x * f.xs;
         for (int64_t q = (blockIdx.x * (int64_t)LT + threadIdx.x) * V; q < pl;
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(LT) k_lpt_disp(const float *__restrict__ gr,
                                                  int16_t *__restrict__ pmid,
                                                  float *__restrict__ disp, float *__restrict__ vel,
                                                  LptGrid g, LptFac f, float s) {
+    after_previous();
     constexpr int PB = LPT_PB * LT;   // particles of a block's turn
     __shared__ __align__(16) float sd[3 * PB], sv[3 * PB];
     __shared__ __align__(16) int16_t sp[3 * PB];
@@ -579,8 +581,8 @@ extern "C" int pmx_lpt_solve(const int64_t grid_shape[3], const float *tables, c
             (e = mesh_rows(true, nat, real, tz, 6 * (int64_t)g.n0, g.n1, g.n2, st)))
             return e;
         const int gy = g.n0 < 65535 ? g.n0 : 65535;
-        k_lpt_source<4><<<dim3((unsigned)((pl / 4 + LT - 1) / LT), gy), LT, 0, st>>>(
-            real, src, pl, g.n0, Fields{6 * pl, pl}, inv);
+        PMX_CUDA(launch_after(k_lpt_source<4>, dim3((unsigned)((pl / 4 + LT - 1) / LT), gy), LT, 0, st,
+                              real, src, pl, g.n0, Fields{6 * pl, pl}, inv));
         PMX_LAUNCH_CHECK("k_lpt_source");
         // the gradients of the source's potential: a force with c = 1
         GreenTab gt;
@@ -596,8 +598,8 @@ extern "C" int pmx_lpt_solve(const int64_t grid_shape[3], const float *tables, c
         (e = mesh_cols(MESH_COLS_INV3, 1, c.g, nat, s0, s1, ty, tables, st)) ||
         (e = mesh_rows(true, nat, real, tz, 3 * (int64_t)g.n0, g.n1, g.n2, st)))
         return e;
-    k_lpt_disp<<<disp_grid(c.M), LT, 0, st>>>(real, g2, Fields{3 * pl, pl}, orders, pmid, disp, vel, g,
-                                              f, inv);
+    PMX_CUDA(launch_after(k_lpt_disp, disp_grid(c.M), LT, 0, st, real, g2, Fields{3 * pl, pl}, orders,
+                          pmid, disp, vel, g, f, inv));
     PMX_LAUNCH_CHECK("k_lpt_disp");
     return PMX_OK;
 }

@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(1, modes_regs
     const bool ok = l < 4 * g.nzt, in = l < g.n2h;
     const int64_t xbs = g.n1 * g.nzt * 32;                  // 8 x-planes
     const int64_t at = ((int64_t)ky * g.nzt + (ok ? l >> 2 : 0)) * 32 + (l & 3);
+    after_previous();
     const int64_t tot = g.n0 + g.n1 + g.n2h, xs = g.n1 * g.n2h;
     const float2 *src = modes + (int64_t)ky * g.n2h + l;
     const float kyj = __ldg(kt + g.n0 + ky), kzl = in ? __ldg(kt + g.n0 + g.n1 + l) : 0.f;
@@ -298,9 +299,11 @@ int mesh_xaxis_modes(bool grads, const MeshGeom &g, const float2 *modes, float s
         const unsigned grid = (unsigned)(g.n1 * ((4 * g.nzt + C::T - 1) / C::T));
         const size_t smem = cols_smem<XCol<N>>(1);
         if (grads)
-            k_xaxis_modes<N, true><<<grid, C::TH, smem, st>>>(modes, scale, spec, tw, kt, g);
+            PMX_CUDA(launch_after(k_xaxis_modes<N, true>, grid, C::TH, smem, st, modes, scale, spec, tw,
+                                  kt, g));
         else
-            k_xaxis_modes<N, false><<<grid, C::TH, smem, st>>>(modes, scale, spec, tw, kt, g);
+            PMX_CUDA(launch_after(k_xaxis_modes<N, false>, grid, C::TH, smem, st, modes, scale, spec, tw,
+                                  kt, g));
         PMX_LAUNCH_CHECK("mesh transform of modes, x axis");
         return PMX_OK;
     });
