@@ -1,6 +1,8 @@
 """Power spectrum estimator (pmwd/spec_util.py:1-147), torch on the GPU."""
 
 import math
+import threading
+from collections import OrderedDict
 
 import torch
 
@@ -128,7 +130,8 @@ def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv, tabs=None):
     # the per-bin sums of k N and N depend on the grid and bins only: for
     # power-of-two grids they are computed on the first call and reused
     key = (dev, grid_shape, tuple(edges.tolist()), bool(right), bnum)
-    cached = _GEOMETRY.get(key) if pow2 else None
+    stream = torch.cuda.current_stream(dev)
+    cached = _GEOMETRY.get(key, stream) if pow2 else None
     if cached is None:
         ksum = torch.zeros(bnum, dtype=torch.float64, device=dev)
         nsum = torch.zeros(bnum, dtype=torch.float64, device=dev)
@@ -142,16 +145,52 @@ def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv, tabs=None):
               None if G is None else torch.view_as_real(G),
               nb, shape, kx, ky, kz, e, len(e), int(right), bnum, float(deconv or 0.0), ksum, psum,
               nsum, int(zm), scratch, _lib.stream_ptr(dev))
-    if cached is None:
-        if pow2:
-            _GEOMETRY[key] = (ksum, nsum)
-    else:
-        ksum, nsum = cached[0].clone(), cached[1].clone()
+    if cached is not None:
+        ksum, nsum = cached
+    elif pow2:
+        _GEOMETRY.put(key, (ksum, nsum), stream)
     PP = psum[:, 0] if G is None else torch.complex(psum[:, 0], psum[:, 1])
     return ksum, PP, nsum
 
 
-_GEOMETRY = {}
+class _GeometryCache:
+    """Per-bin sums of k N and N of the last grids and bins (a few hundred
+    bytes to 32 KB an entry, the oldest given back beyond ``size``).  What goes
+    in and out are copies, so a caller's changes stay its own; an event says
+    when a copy's stream has written it, and any other stream waits for that
+    before it reads."""
+
+    def __init__(self, size=64):
+        self.size = size
+        self.entries = OrderedDict()
+        self.lock = threading.Lock()
+
+    def get(self, key, stream):
+        with self.lock:
+            entry = self.entries.get(key)
+            if entry is None:
+                return None
+            self.entries.move_to_end(key)
+        sums, written = entry
+        stream.wait_event(written)
+        for t in sums:   # not reused, once given back, before this stream's read
+            t.record_stream(stream)
+        return tuple(t.clone() for t in sums)
+
+    def put(self, key, sums, stream):
+        entry = tuple(t.clone() for t in sums), stream.record_event()
+        with self.lock:
+            self.entries[key] = entry
+            self.entries.move_to_end(key)
+            while len(self.entries) > self.size:
+                self.entries.popitem(last=False)
+
+    def clear(self):
+        with self.lock:
+            self.entries.clear()
+
+
+_GEOMETRY = _GeometryCache()
 
 
 def _pow2_grid(grid_shape):
