@@ -390,7 +390,7 @@ int pmx_powspec_bin_zmajor(const float *F, const float *G, int64_t nbatch,
                            int32_t nedges, int32_t right, int32_t nbin, double deconv,
                            double *ksum, double *psum, double *nsum, void *stream);
 
-/* pmx_powspec_bin of any grid in either layout: half_major = 0 as
+/* pmx_powspec_bin of any grid in either layout (spectra on 8 bytes): half_major = 0 as
  * pmx_powspec_bin, else as pmx_powspec_bin_zmajor.  scratch: 8-byte aligned
  * device memory of pmx_powspec_scratch_bytes(grid_shape, nedges, nbin,
  * deconv != 0, ksum != NULL, half_major) bytes (0: bad arguments), in use until
@@ -435,7 +435,8 @@ int pmx_normal(uint32_t k0, uint32_t k1, int64_t n, int layout, float *out, void
  * transforms, and their transposes.  Spectra are complex64 half spectra
  * (n0, n1, n2/2+1), contiguous unless strides are given (in complex values:
  * per axis, then from one spectrum to the next); fields are float32 (n0, n1,
- * n2).  Transforms are unnormalised; `scale` carries 1 / N where a stage
+ * n2).  Spectra and modes are on 8 bytes (PMX_ERR_ALIGN otherwise).
+ * Transforms are unnormalised; `scale` carries 1 / N where a stage
  * reads their result, and 1 / cell volume where it reads the modes.
  * ------------------------------------------------------------------------ */
 
@@ -470,9 +471,9 @@ int pmx_lpt_disp(const int64_t grid_shape[3], const float *tables, const float *
 
 /* All of the above in one call, for the grids whose axes the library's own
  * transforms support (64, 96, 128, 192, 256, 384, 512, 768, 1024): contiguous
- * modes to pmid, disp and vel.  scratch: 256-byte aligned device memory of
- * pmx_lpt_solve_floats floats (count 0: no transforms of this shape), in use until
- * the stream is past this call. */
+ * modes to pmid, disp and vel.  scratch: 16-byte aligned device memory (256 for
+ * whole lines) of pmx_lpt_solve_floats floats (count 0: no transforms of this
+ * shape), in use until the stream is past this call. */
 int pmx_lpt_solve_floats(const int64_t grid_shape[3], int32_t orders, int64_t *count);
 int pmx_lpt_solve(const int64_t grid_shape[3], const float *tables, const float *modes, float scale,
                   int32_t orders, const float *fac, float *scratch, int16_t *pmid, float *disp,

@@ -72,6 +72,13 @@ struct EmParams {
     float cot_div;
 };
 
+// Whether every pointer is on `bytes` bytes (NULL is): what kernels that read pairs or
+// 16 bytes at a time need of the caller's arrays.
+template <class... P>
+bool aligned(size_t bytes, const P *...p) {
+    return ((reinterpret_cast<uintptr_t>(p) % bytes == 0) && ...);
+}
+
 int make_em_params(const pmx_enmesh_spec *spec, EmParams *p);
 // 1 / y if y is a power of two well inside the float range, else 0.
 float exact_inverse(float y);

@@ -26,6 +26,9 @@
 
 using namespace pmx;
 
+#define PMX_ALIGNED(bytes, ...) \
+    if (!aligned(bytes, __VA_ARGS__)) return fail(PMX_ERR_ALIGN, "arrays must be on " #bytes " bytes")
+
 namespace {
 
 constexpr int LT = 256;
@@ -472,6 +475,7 @@ extern "C" int pmx_lpt_strain(const int64_t grid_shape[3], const float *tables, 
     int st = grid_of(grid_shape, tables, &g);
     if (st || (st = walk_of(g, nullptr, &w))) return st;
     if (!modes || !spec) return fail(PMX_ERR_ARG, "null modes/spec");
+    PMX_ALIGNED(8, modes, spec);
     k_lpt_strain<<<walk_grid(w), LT, 0, as_stream(stream)>>>((const float2 *)modes, (float2 *)spec, g,
                                                              w, scale);
     PMX_LAUNCH_CHECK("k_lpt_strain");
@@ -493,6 +497,7 @@ extern "C" int pmx_lpt_grad(const int64_t grid_shape[3], const float *tables, co
     int st = grid_of(grid_shape, tables, &g);
     if (st || (st = walk_of(g, nullptr, &w))) return st;
     if (!modes || !spec || (src2 && !src2_strides)) return fail(PMX_ERR_ARG, "null modes/spec/strides");
+    PMX_ALIGNED(8, modes, src2, spec);
     k_lpt_grad<<<walk_grid(w), LT, 0, as_stream(stream)>>>(
         (const float2 *)modes, (const float2 *)src2, src2 ? src2_strides[0] : 0,
         src2 ? src2_strides[1] : 0, src2 ? src2_strides[2] : 0, (float2 *)spec, g, w, scale);
@@ -562,6 +567,8 @@ extern "C" int pmx_lpt_solve(const int64_t grid_shape[3], const float *tables, c
     int e = grid_of(grid_shape, tables, &g);
     if (e || (e = fac_of(fac, orders, &f))) return e;
     if (!modes || !scratch || !pmid || !disp || !vel) return fail(PMX_ERR_ARG, "null array");
+    PMX_ALIGNED(8, modes);
+    PMX_ALIGNED(16, scratch);
     if (!solve_scratch(g, orders, &c)) return fail(PMX_ERR_SHAPE, "no mesh transforms of this shape");
     cudaStream_t st = as_stream(stream);
     if ((e = mesh_rows_prepare(g.n2)) || (e = mesh_cols_prepare(g.n1)) || (e = mesh_xaxis_prepare(g.n0)))
@@ -623,6 +630,7 @@ extern "C" int pmx_lpt_src_adj(const int64_t grid_shape[3], const float *tables,
     int st = grid_of(grid_shape, tables, &g);
     if (st || (st = walk_of(g, strides, &w))) return st;
     if (!spec || !src_cot) return fail(PMX_ERR_ARG, "null array");
+    PMX_ALIGNED(8, spec, src_cot);
     k_lpt_src_adj<<<walk_grid(w), LT, 0, as_stream(stream)>>>((const float2 *)spec, (float2 *)src_cot,
                                                               g, w, scale);
     PMX_LAUNCH_CHECK("k_lpt_src_adj");
@@ -646,6 +654,7 @@ extern "C" int pmx_lpt_modes_adj(const int64_t grid_shape[3], const float *table
     int st = grid_of(grid_shape, tables, &g);
     if (st || (st = walk_of(g, strides, &w))) return st;
     if (!grads_spec || !modes_cot || !cot_strides) return fail(PMX_ERR_ARG, "null array");
+    PMX_ALIGNED(8, grads_spec, strain_spec, modes_cot);
     k_lpt_modes_adj<<<walk_grid(w), LT, 0, as_stream(stream)>>>(
         (const float2 *)grads_spec, (const float2 *)strain_spec, (float2 *)modes_cot, cot_strides[0],
         cot_strides[1], cot_strides[2], g, w, scale);

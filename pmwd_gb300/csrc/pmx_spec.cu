@@ -727,6 +727,8 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
     clear_error();
     if (!F || !grid_shape || !kx || !ky || !kz || !edges || !psum)
         return fail(PMX_ERR_ARG, "null argument");
+    if (!aligned(8, F, G) || !aligned(8, static_cast<char *>(scratch)))
+        return fail(PMX_ERR_ALIGN, "spectra and scratch must be on 8 bytes");
     if (!ksum != !nsum) return fail(PMX_ERR_ARG, "ksum and nsum are both given or both NULL");
     if (nbatch < 1 || nedges < 1 || nbin < 1 || nbin > nedges)
         return fail(PMX_ERR_ARG, "need nbatch >= 1 and 1 <= nbin <= nedges");
