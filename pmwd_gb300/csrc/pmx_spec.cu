@@ -714,6 +714,22 @@ Scratch scratch_of(const int64_t n[3], int32_t nedges, int32_t nbin, bool deconv
     return c;
 }
 
+// Scratch of a call whose caller brings none: stream-ordered (after a synchronisation
+// that costs some 0.1 ms), given back behind the launches, also when one fails.
+struct OwnScratch {
+    cudaStream_t s;
+    char *p = nullptr;
+    int release() {
+        char *q = p;
+        p = nullptr;
+        if (q) PMX_CUDA(cudaFreeAsync(q, s));
+        return PMX_OK;
+    }
+    ~OwnScratch() {
+        if (p) cudaFreeAsync(p, s);
+    }
+};
+
 }  // namespace
 }  // namespace pmx
 
@@ -758,10 +774,12 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
     const Scratch sc = scratch_of(grid_shape, nedges, nbin, nwin != 0, ksum != nullptr, zm);
     if (!sc.pow2 && !ksum)
         return fail(PMX_ERR_ARG, "ksum/nsum may be NULL only for power-of-two grids <= 2048");
-    // without the caller's: stream-ordered, freed after the launch (the stream
-    // keeps it alive); after a synchronisation that costs some 0.1 ms
+    OwnScratch own{s};
     char *scr = static_cast<char *>(scratch);
-    if (!scr) PMX_CUDA(cudaMallocAsync((void **)&scr, sc.bytes(), s));
+    if (!scr) {
+        PMX_CUDA(cudaMallocAsync((void **)&own.p, sc.bytes(), s));
+        scr = own.p;
+    }
     if (sc.pow2) {
         Pow2Args p;
         p.zm = zm;
@@ -811,8 +829,7 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
             else launch_rows<false, false>(p, s);
         }
         PMX_LAUNCH_CHECK("k_powspec_rows");
-        if (!scratch) PMX_CUDA(cudaFreeAsync(scr, s));
-        return PMX_OK;
+        return own.release();
     }
     long long *keys = reinterpret_cast<long long *>(scr);
     k_edge_keys<<<(nedges + 63) / 64, 64, 0, s>>>(edges, nedges, right, keys);
@@ -832,8 +849,7 @@ static int powspec_bin(const float *F, const float *G, int64_t nbatch, const int
     const int grid = stride_grid((a.n0 / 2 + 1) * (zm ? a.n2h : a.n1 / 2 + 1) * 32, ST, resident(kern, sm));
     kern<<<grid, ST, sm, s>>>(a);
     PMX_LAUNCH_CHECK("k_powspec");
-    if (!scratch) PMX_CUDA(cudaFreeAsync(scr, s));
-    return PMX_OK;
+    return own.release();
 }
 
 extern "C" int pmx_powspec_bin(const float *F, const float *G, int64_t nbatch,
