@@ -18,7 +18,7 @@ import torch
 from . import _hostmath, _lib
 from .boltzmann import growth
 from .cosmology import E2
-from .gravity import laplace, neg_grad
+from .gravity import _laplace, laplace, neg_grad
 from .particles import Particles
 from .pm_util import fftfreq, fftfwd, fftinv
 
@@ -119,7 +119,12 @@ def _growth_factors(cosmo, conf):
     return torch.stack(rows).to(torch.float32)
 
 
-def _lpt_device(modes, fac, kvec, disp0, vel0, conf):
+def _laplace_ops(kvec, src):
+    """laplace in torch operations alone, which every transform of them follows."""
+    return _laplace(src, sum(k ** 2 for k in kvec))
+
+
+def _lpt_device(modes, fac, kvec, disp0, vel0, conf, laplace=laplace):
     """The device work of lpt (lpt.py:136-212) for lpt_order >= 1: the
     potentials, the 2nd-order source, and every displacement field of every
     order from one batched inverse FFT; fac (lpt_order, 2) float32 on the
@@ -205,6 +210,16 @@ def _lpt_stages(modes, fac, conf, fac_dev=None):
     return pmid, disp, vel, tab, phi
 
 
+def _has_storage(t):
+    """Whether the library can read t: a batched cotangent (is_grads_batched, a
+    vectorised jacobian, vmap over backward calls) has no memory of its own."""
+    try:
+        t.data_ptr()
+    except RuntimeError:
+        return False
+    return True
+
+
 def _lpt_solve(modes, fac, conf):
     """(pmid, disp, vel) by one library call with its own transforms, or None
     where it has none of this shape."""
@@ -250,14 +265,17 @@ class _LptFn(torch.autograd.Function):
             (g.n, 3), dtype=torch.float32, device=g.dev)
         disp_cot = zero if disp_cot is None else disp_cot
         vel_cot = zero if vel_cot is None else vel_cot
-        if torch.is_grad_enabled():
-            # a gradient of the gradient: through the torch operations
-            grid = Particles.gen_grid(conf, vel=True, device=g.dev)
-            kvec = fftfreq(g.shape, conf.ptcl_spacing, dtype=torch.float32, device=g.dev)
-            disp, vel = _lpt_device(modes, torch.from_numpy(ctx.fac).to(g.dev), kvec, grid.disp.t(),
-                                    grid.vel.t(), conf)
-            return torch.autograd.grad((disp.t(), vel.t()), modes, (disp_cot, vel_cot),
-                                       create_graph=True) + (None, None)
+        create = torch.is_grad_enabled()
+        if create or not (_has_storage(disp_cot) and _has_storage(vel_cot)):
+            # a gradient of the gradient, or many gradients at once: through the
+            # torch operations
+            with torch.enable_grad():
+                grid = Particles.gen_grid(conf, vel=True, device=g.dev)
+                kvec = fftfreq(g.shape, conf.ptcl_spacing, dtype=torch.float32, device=g.dev)
+                disp, vel = _lpt_device(modes, torch.from_numpy(ctx.fac).to(g.dev), kvec,
+                                        grid.disp.t(), grid.vel.t(), conf, _laplace_ops)
+                return torch.autograd.grad((disp.t(), vel.t()), modes, (disp_cot, vel_cot),
+                                           create_graph=create) + (None, None)
         cf = (_lib.c_f * (2 * g.orders))(*ctx.fac.reshape(-1).tolist())
         cot = g.empty(3 * g.orders)
         _lib.call('pmx_lpt_disp_adj', g.n, disp_cot.contiguous(), vel_cot.contiguous(), g.orders, cf,

@@ -1,0 +1,56 @@
+"""Forms in which torch asks lpt for the modes' gradient besides one plain backward call."""
+
+import pytest
+import torch
+
+import pmwd_gb300 as pg
+
+pytestmark = pytest.mark.gpu
+
+# float32 transforms in another order: as the stages' own gradient test
+GTOL = 4e-6
+
+
+def _setup(cuda, order=2, grid=(6, 9, 8)):
+    conf = pg.Configuration(1.7, grid, mesh_shape=1, lpt_order=order)
+    cosmo = pg.boltzmann(pg.SimpleLCDM(conf), conf, transfer=False, varlin=False)
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    modes = (30 * torch.fft.rfftn(torch.randn(grid, generator=gen, device=cuda))).contiguous()
+    cots = torch.randn((3, conf.ptcl_num, 3), generator=gen, device=cuda)
+    return conf, cosmo, modes, cots
+
+
+def _close(a, b):
+    assert a.shape == b.shape
+    assert float((a - b).norm() / b.norm()) < GTOL
+
+
+@pytest.mark.parametrize('order', [1, 2])
+@pytest.mark.parametrize('create', [False, True])
+def test_batched_cotangents(cuda, order, create):
+    conf, cosmo, modes, cots = _setup(cuda, order)
+    m = modes.requires_grad_()
+    p, _ = pg.lpt(m, cosmo, conf)
+    want = torch.stack([torch.autograd.grad((p.disp, p.vel), m, (c, 2 * c), retain_graph=True)[0]
+                        for c in cots])
+    (got,) = torch.autograd.grad((p.disp, p.vel), m, (cots, 2 * cots), is_grads_batched=True,
+                                 retain_graph=True, create_graph=create)
+    _close(got.detach(), want)
+    got = torch.vmap(lambda c: torch.autograd.grad((p.disp, p.vel), m, (c, 2 * c), retain_graph=True,
+                                                   create_graph=create)[0])(cots)
+    _close(got.detach(), want)
+    # one of the outputs alone
+    want = torch.stack([torch.autograd.grad(p.vel, m, c, retain_graph=True)[0] for c in cots])
+    (got,) = torch.autograd.grad(p.vel, m, cots, is_grads_batched=True)
+    _close(got, want)
+
+
+def test_vectorised_jacobian(cuda):
+    conf, cosmo, modes, _ = _setup(cuda, grid=(4, 3, 2))
+
+    def f(x):
+        return pg.lpt(torch.view_as_complex(x), cosmo, conf)[0].disp
+
+    x = torch.view_as_real(modes).clone()
+    _close(torch.autograd.functional.jacobian(f, x, vectorize=True),
+           torch.autograd.functional.jacobian(f, x))
