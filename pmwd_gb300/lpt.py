@@ -278,8 +278,8 @@ class _LptFn(torch.autograd.Function):
                                            create_graph=create) + (None, None)
         cf = (_lib.c_f * (2 * g.orders))(*ctx.fac.reshape(-1).tolist())
         cot = g.empty(3 * g.orders)
-        _lib.call('pmx_lpt_disp_adj', g.n, disp_cot.contiguous(), vel_cot.contiguous(), g.orders, cf,
-                  cot, g.stream)
+        _lib.call('pmx_lpt_disp_adj', g.n, disp_cot.resolve_neg().contiguous(),
+                  vel_cot.resolve_neg().contiguous(), g.orders, cf, cot, g.stream)
         C = torch.fft.rfftn(cot, dim=(-3, -2, -1))
         st = _i64(C.stride()[1:] + C.stride()[:1])
         S = None
@@ -430,7 +430,8 @@ def lpt(modes, cosmo, conf):
             pmid, disp, vel = _graph_for(conf, modes).run(modes, torch.from_numpy(fac))
         else:
             with torch.cuda.device(dev):
-                pmid, disp, vel = _LptFn.apply(modes.resolve_conj().contiguous(), fac, conf)
+                pmid, disp, vel = _LptFn.apply(modes.resolve_conj().resolve_neg().contiguous(), fac,
+                                                conf)
         return Particles(conf, pmid, disp, vel=vel), None
     fac = _growth_factors(cosmo, conf).to(dev)
     kvec = fftfreq(conf.ptcl_grid_shape, conf.ptcl_spacing, dtype=torch.float32, device=dev)

@@ -54,3 +54,20 @@ def test_vectorised_jacobian(cuda):
     x = torch.view_as_real(modes).clone()
     _close(torch.autograd.functional.jacobian(f, x, vectorize=True),
            torch.autograd.functional.jacobian(f, x))
+
+
+@pytest.mark.parametrize('grad', [False, True])
+def test_negative_views(cuda, grad):
+    """Modes and cotangents whose sign is still to be applied (torch's negative bit)."""
+    conf, cosmo, modes, cots = _setup(cuda)
+    view = torch._neg_view(modes)
+    assert view.is_neg() and view.is_contiguous()
+    got = pg.lpt(view.detach().requires_grad_(grad), cosmo, conf)[0]
+    want = pg.lpt((-modes).requires_grad_(grad), cosmo, conf)[0]
+    assert torch.equal(got.vel, want.vel)
+    if grad:
+        m = modes.clone().requires_grad_()
+        out = pg.lpt(m, cosmo, conf)[0].disp
+        (got,) = torch.autograd.grad(out, m, torch._neg_view(cots[0]), retain_graph=True)
+        (want,) = torch.autograd.grad(out, m, -cots[0])
+        assert torch.equal(got, want)
