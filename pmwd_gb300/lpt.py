@@ -251,16 +251,19 @@ class _LptFn(torch.autograd.Function):
         else:
             pmid, disp, vel = out
         if ctx.needs_input_grad[0]:
-            ctx.save_for_backward(modes, tab, phi)
+            # the VJP needs tab and phi only; the modes, which their owner may change
+            # before it runs, serve the torch operations in backward
+            ctx.save_for_backward(tab, phi)
+            ctx.modes, ctx.version = modes, modes._version
             ctx.fac, ctx.conf = fac, conf
         ctx.mark_non_differentiable(pmid)
         return pmid, disp, vel
 
     @staticmethod
     def backward(ctx, _, disp_cot, vel_cot):
-        modes, tab, phi = ctx.saved_tensors
+        tab, phi = ctx.saved_tensors
         conf = ctx.conf
-        g = _Grid(conf, modes.device)
+        g = _Grid(conf, tab.device)
         zero = None if disp_cot is not None and vel_cot is not None else torch.zeros(
             (g.n, 3), dtype=torch.float32, device=g.dev)
         disp_cot = zero if disp_cot is None else disp_cot
@@ -269,6 +272,10 @@ class _LptFn(torch.autograd.Function):
         if create or not (_has_storage(disp_cot) and _has_storage(vel_cot)):
             # a gradient of the gradient, or many gradients at once: through the
             # torch operations
+            modes = ctx.modes
+            if modes._version != ctx.version:
+                raise RuntimeError('modes needed for this gradient were modified by an inplace '
+                                   'operation after lpt')
             with torch.enable_grad():
                 grid = Particles.gen_grid(conf, vel=True, device=g.dev)
                 kvec = fftfreq(g.shape, conf.ptcl_spacing, dtype=torch.float32, device=g.dev)

@@ -71,3 +71,19 @@ def test_negative_views(cuda, grad):
         (got,) = torch.autograd.grad(out, m, torch._neg_view(cots[0]), retain_graph=True)
         (want,) = torch.autograd.grad(out, m, -cots[0])
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize('order', [1, 2])
+def test_modes_changed_in_place_before_backward(cuda, order):
+    """The gradient is that of the call's modes, whatever their owner does with them after it;
+    a gradient that would have to read them again is refused."""
+    conf, cosmo, modes, cots = _setup(cuda, order)
+    m = modes.clone().requires_grad_()
+    p, _ = pg.lpt(m, cosmo, conf)
+    (want,) = torch.autograd.grad((p.disp, p.vel), m, (cots[0], cots[1]), retain_graph=True)
+    with torch.no_grad():
+        m.mul_(-3)
+    (got,) = torch.autograd.grad((p.disp, p.vel), m, (cots[0], cots[1]), retain_graph=True)
+    assert torch.equal(got, want)
+    with pytest.raises(RuntimeError, match='modified by an inplace operation'):
+        torch.autograd.grad(p.disp, m, cots[0], create_graph=True)
