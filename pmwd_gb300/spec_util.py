@@ -94,7 +94,8 @@ def _to_device(dev, *arrays):
     (it would wait for the transforms too): from pinned memory, which the
     caching allocator holds until the copy is done.  A capture would keep the
     copy longer than that: there the plain copy refuses, as any upload does."""
-    host = [a.reshape(-1).to(torch.float64) for a in arrays]
+    # on the CPU whatever torch's default device is
+    host = [a.reshape(-1).to('cpu', torch.float64) for a in arrays]
     packed = torch.cat(host)
     if torch.cuda.is_current_stream_capturing():
         packed = packed.to(dev)
