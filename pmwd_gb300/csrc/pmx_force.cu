@@ -1432,9 +1432,9 @@ __global__ void k_finish(const double *part, int64_t pstride, int nblk, int nblk
 // ---------------------------------------------------------------------------
 // Batched simulations: one launch serves up to BMAX simulations that share a
 // mesh shape and cell size.  blockIdx.y selects the simulation; its particle
-// arrays, particle count, CIC value and this launch's leapfrog factors come
-// from a table passed by value (__grid_constant__: read in place from the
-// parameter space), its meshes are slot blockIdx.y of the workspace buffers.
+// arrays, particle count, CIC value, deposit rule and this launch's leapfrog
+// factors come from a table passed by value (__grid_constant__: read in place
+// from the parameter space), its meshes are slot blockIdx.y of the workspace buffers.
 // Each body is the one the single-simulation kernels run, so a simulation's
 // arithmetic is the same alone and in a batch.
 // ---------------------------------------------------------------------------
@@ -1444,6 +1444,7 @@ struct SimB {
     float *disp, *vel, *acc, *dcot, *vcot, *alpha;
     int64_t n;
     float val;     // f32(mesh_size / ptcl_num) of this simulation
+    int dep;       // how its z pairs are deposited (enum Dep)
     float f[3];    // this launch's leapfrog factors (meaning per kernel)
 };
 struct BatchTab {
@@ -1459,6 +1460,7 @@ __device__ __forceinline__ T *slot_ptr(T *base, int64_t per) {
 __device__ __forceinline__ Hot sim_hot(const Hot &h, const SimB &sb) {
     Hot hh = h;
     hh.val = sb.val;
+    hh.dep = sb.dep;
     return hh;
 }
 
@@ -1496,9 +1498,12 @@ __global__ void __launch_bounds__(PT) k_ka_b(Hot h, const __grid_constant__ Batc
 }
 
 // acc_cot: the simulation's vel_cot (steps) or the given cotangent of acc
-// (the force VJP, where it is also vel_cot)
+// (the force VJP, where it is also vel_cot).  Four blocks per SM as in k_g3adj, which
+// also pays for reading the deposit rule from the table: an adjoint step of four
+// 256^3-particle simulations on 256^3 takes 11.87 ms (12.25 with three blocks; 12.12
+// with them and the rule of the batch's first simulation for all).
 template <bool AGG>
-__global__ void __launch_bounds__(PT) k_g3adj_b(Hot h, const __grid_constant__ BatchTab t,
+__global__ void __launch_bounds__(PT, 4) k_g3adj_b(Hot h, const __grid_constant__ BatchTab t,
                                                 int64_t M, const float *g, float *mcot,
                                                 double *part) {
     const SimB &sb = t.s[blockIdx.y];
@@ -1676,7 +1681,8 @@ int device_scratch(double **out) {
 #define PMX_UNPAREN(...) __VA_ARGS__
 
 // The rule of enum Dep: n particles on the workspace's mesh.
-int deposit_mode(const pmx_workspace *ws, int64_t n) {
+int deposit_rule(const pmx_workspace *ws, int64_t n) {
+    if (ws->vec) return DEP_V4;
     if (ws->M < 4 * n) return DEP_JOIN;
     return ws->n2 % 2 == 0 ? DEP_V2 : DEP_SCALAR;
 }
@@ -1709,7 +1715,7 @@ int check_hot(pmx_workspace *ws, const pmx_enmesh_spec *spec, const void *pmid, 
     h->dcomp = nullptr;
     h->vcomp = nullptr;
     h->win = ws->win;
-    h->dep = ws->vec ? DEP_V4 : deposit_mode(ws, n);
+    h->dep = deposit_rule(ws, n);
     h->agg = ws->agg;
     h->pstride = ws->pstride;
     if (ws->xfast) {
@@ -2934,6 +2940,7 @@ int batch_prepare(pmx_workspace *ws, const pmx_enmesh_spec *spec, int32_t nsim,
         sb.alpha = q.acc_cot;
         sb.n = q.n;
         sb.val = (float)((double)ws->M / (double)q.ptcl_num);
+        sb.dep = deposit_rule(ws, q.n);
         bc->c[b] = green_c(ws, q.omega_m);
         bc->fin.dots[b] = q.dots;
         bc->fin.oms[b] = om_scale(q.omega_m);
