@@ -195,7 +195,13 @@ def ptr(t):
 
 
 def stream_ptr(device=None):
-    return c_p(torch.cuda.current_stream(device).cuda_stream)
+    """Handle of the current stream of a device (default: the current one),
+    without the Stream object that torch.cuda.current_stream makes (0.4
+    instead of 2.1 us)."""
+    idx = torch.device(device).index if device is not None else None
+    if idx is None:
+        idx = torch.cuda.current_device()
+    return c_p(torch._C._cuda_getCurrentRawStream(idx))
 
 
 _LIB_STREAMS = {}

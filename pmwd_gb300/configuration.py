@@ -138,7 +138,7 @@ class Configuration:
 
     @property
     def ptcl_num(self):
-        return int(np.prod(self.ptcl_grid_shape, dtype=np.int64))
+        return math.prod(self.ptcl_grid_shape)
 
     @property
     def box_size(self):
@@ -158,7 +158,7 @@ class Configuration:
 
     @property
     def mesh_size(self):
-        return int(np.prod(self.mesh_shape, dtype=np.int64))
+        return math.prod(self.mesh_shape)
 
     @property
     def V(self):
