@@ -115,6 +115,11 @@ __device__ __forceinline__ float inv_k2(float kx, float ky, float kz) {
     return k2 != 0.f ? -1.f / k2 : 0.f;
 }
 __device__ __forceinline__ float2 scale2(float2 v, float s) { return make_float2(v.x * s, v.y * s); }
+// v times a multiple s of inv_k2: 0 where that is, also of an infinite or NaN v (the k = 0
+// mode of a spectrum like 1 / k).
+__device__ __forceinline__ float2 solve2(float2 v, float s) {
+    return s != 0.f ? scale2(v, s) : make_float2(0.f, 0.f);
+}
 
 // out[c] = -k_i k_j pot, pot = -scale modes / k^2, pairs 00 11 22 01 02 12; the
 // Nyquist entries count only on the diagonal (lpt.py:13-37).
@@ -124,7 +129,7 @@ __global__ void __launch_bounds__(LT) k_lpt_strain(const float2 *__restrict__ mo
     walk(w, [&](int i, int j, int l, int64_t o) {
         const float kx = __ldg(g.k(0) + i), ky = __ldg(g.k(1) + j), kz = __ldg(g.k(2) + l);
         const float mx = __ldg(g.kz(0) + i), my = __ldg(g.kz(1) + j), mz = __ldg(g.kz(2) + l);
-        const float2 p = scale2(modes[o], -scale * inv_k2(kx, ky, kz));   // -pot
+        const float2 p = solve2(modes[o], -scale * inv_k2(kx, ky, kz));   // -pot
         out[o] = scale2(p, kx * kx);
         out[o + w.batch] = scale2(p, ky * ky);
         out[o + 2 * w.batch] = scale2(p, kz * kz);
@@ -192,12 +197,12 @@ __global__ void __launch_bounds__(LT) k_lpt_grad(const float2 *__restrict__ mode
     walk(w, [&](int i, int j, int l, int64_t o) {
         const float ik = inv_k2(__ldg(g.k(0) + i), __ldg(g.k(1) + j), __ldg(g.k(2) + l));
         const float m[3] = {__ldg(g.kz(0) + i), __ldg(g.kz(1) + j), __ldg(g.kz(2) + l)};
-        const float2 p = scale2(modes[o], scale * ik);
+        const float2 p = solve2(modes[o], scale * ik);
 #pragma unroll
         for (int a = 0; a < 3; ++a)   // (-i k)(x + i y) = (k y, -k x)
             out[o + a * w.batch] = make_float2(m[a] * p.y, -(m[a] * p.x));
         if (src2) {
-            const float2 q = scale2(src2[i * s0 + j * s1 + l * s2], ik);
+            const float2 q = solve2(src2[i * s0 + j * s1 + l * s2], ik);
 #pragma unroll
             for (int a = 0; a < 3; ++a)
                 out[o + (3 + a) * w.batch] = make_float2(m[a] * q.y, -(m[a] * q.x));
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(LT) k_lpt_src_adj(const float2 *__restrict__ C
             re = fmaf(-m[a], c.y, re);
             im = fmaf(m[a], c.x, im);
         }
-        out[((int64_t)i * g.n1 + j) * g.n2h + l] = make_float2(re * ik, im * ik);
+        out[((int64_t)i * g.n1 + j) * g.n2h + l] = solve2(make_float2(re, im), ik);
     });
 }
 
@@ -372,8 +377,7 @@ __global__ void __launch_bounds__(LT) k_lpt_modes_adj(const float2 *__restrict__
             }
         }
         const float mult = l == 0 || 2 * l == g.n2 ? 1.f : 2.f;
-        const float f = mult * s * inv_k2(kx, ky, kz);
-        out[i * s0 + j * s1 + l * s2] = make_float2(re * f, im * f);
+        out[i * s0 + j * s1 + l * s2] = solve2(make_float2(re, im), mult * s * inv_k2(kx, ky, kz));
     });
 }
 

@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(XCol<N>::TH, col_blocks<XCol<N>>(1, modes_regs
         static_for<R2>([&](auto E) {
             const float kx = ld_tab(kt + k1 + R1 * reg_freq<R2>(E));
             const float k2 = __fadd_rn(__fadd_rn(__fmul_rn(kx, kx), ky2), kz2);
-            const float f = k2 != 0.f ? scale * (1.f / k2) : 0.f;   // k = 0 -> 0
-            p[E] = make_float2(p[E].x * f, p[E].y * f);
+            const float f = scale * (1.f / k2);   // k = 0 -> 0, whatever the mode
+            p[E] = k2 != 0.f ? make_float2(p[E].x * f, p[E].y * f) : make_float2(0.f, 0.f);
         });
     };
     constexpr bool KEEP = modes_keep<N>();
