@@ -131,8 +131,10 @@ def _bin_cuda(F, G, grid_shape, edges, right, bnum, deconv, tabs=None):
     # the per-bin sums of k N and N depend on the grid and bins only: for
     # power-of-two grids they are computed on the first call and reused
     key = (dev, grid_shape, tuple(edges.tolist()), bool(right), bnum)
-    stream = torch.cuda.current_stream(dev)
-    cached = _GEOMETRY.get(key, stream) if pow2 else None
+    cached = None
+    if pow2:
+        stream = torch.cuda.current_stream(dev)
+        cached = _GEOMETRY.get(key, stream)
     if cached is None:
         ksum = torch.zeros(bnum, dtype=torch.float64, device=dev)
         nsum = torch.zeros(bnum, dtype=torch.float64, device=dev)
@@ -172,14 +174,16 @@ class _GeometryCache:
             if entry is None:
                 return None
             self.entries.move_to_end(key)
-        sums, written = entry
-        stream.wait_event(written)
-        for t in sums:   # not reused, once given back, before this stream's read
-            t.record_stream(stream)
+        sums, written, writer = entry
+        if not written.query():
+            stream.wait_event(written)
+        if stream != writer:
+            for t in sums:   # not reused, once given back, before this stream's read
+                t.record_stream(stream)
         return tuple(t.clone() for t in sums)
 
     def put(self, key, sums, stream):
-        entry = tuple(t.clone() for t in sums), stream.record_event()
+        entry = tuple(t.clone() for t in sums), stream.record_event(), stream
         with self.lock:
             self.entries[key] = entry
             self.entries.move_to_end(key)

@@ -20,16 +20,24 @@ class _Tensor:
         self.log.append(('record_stream', self.name, stream.name))
 
 
+class _Event:
+    def __init__(self, stream, log):
+        self.stream, self.log, self.done = stream, log, False
+
+    def query(self):
+        return self.done
+
+
 class _Stream:
     def __init__(self, name, log):
         self.name, self.log = name, log
 
     def record_event(self):
         self.log.append(('record_event', self.name))
-        return 'event of ' + self.name
+        return _Event(self.name, self.log)
 
     def wait_event(self, event):
-        self.log.append(('wait_event', self.name, event))
+        self.log.append(('wait_event', self.name, event.stream))
 
 
 def test_another_stream_waits_and_gets_copies():
@@ -42,10 +50,15 @@ def test_another_stream_waits_and_gets_copies():
     assert log == [('clone', 'k'), ('clone', 'n'), ('record_event', 'a')]
     log.clear()
     k, n = cache.get('grid', b)
-    assert log[0] == ('wait_event', 'b', 'event of a')
+    assert log[0] == ('wait_event', 'b', 'a')
     assert set(log[1:3]) == {('record_stream', "k'", 'b'), ('record_stream', "n'", 'b')}
     assert log[3:] == [('clone', "k'"), ('clone', "n'")]
     assert (k.name, n.name) == ("k''", "n''")
+    # nothing to wait for once it is written, nothing to record on the writing stream itself
+    cache.entries['grid'][1].done = True
+    log.clear()
+    cache.get('grid', a)
+    assert log == [('clone', "k'"), ('clone', "n'")]
 
 
 def test_entries_are_bounded_and_the_oldest_goes():
