@@ -143,7 +143,8 @@ typedef struct pmx_workspace pmx_workspace;
                               reduction (n2 % 4 == 0; opt-in: slower on
                               GB300) */
 #define PMX_WS_NO_GRAPH 32 /* issue the slab loops of the plane transforms
-                              directly instead of replaying captured graphs */
+                              directly instead of replaying captured graphs
+                              (no effect on the library's own transforms) */
 #define PMX_WS_PLANE16 64  /* plane kernels in clusters of 16 CTAs (the
                               non-portable size) instead of 8 */
 #define PMX_WS_AGG 128     /* warp-aggregated deposits: lanes whose particles
@@ -159,7 +160,8 @@ typedef struct pmx_workspace pmx_workspace;
 /* Slab-wise plane transforms: number of concurrent chains (1..4; 0 = the
  * default 2) in bits 8..10 and log2 of the x-planes per cuFFT execution
  * (1..15; 0 = the default, the smallest power of two >= 8 reaching 32 MB) in
- * bits 12..15 of the flags.  Results do not depend on either. */
+ * bits 12..15 of the flags.  Results do not depend on either, and meshes on
+ * the library's own transforms have neither. */
 #define PMX_WS_CHAINS_SHIFT 8
 #define PMX_WS_SLAB_SHIFT 12
 #define PMX_WS_CHAINS(k) (((k) & 7) << PMX_WS_CHAINS_SHIFT)

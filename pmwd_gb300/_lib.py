@@ -253,12 +253,13 @@ class Workspace:
                  plane=False, vec=False, graphs=True, plane16=False, chains=0, slab_log2=0,
                  slots=1, agg=False, tma=False):
         """Flags of pmx_workspace_create (include/pmx.h): ``cufft3d`` 3-D
-        cuFFT plans instead of the fused x pass, ``window`` warp-window
+        cuFFT plans whatever the shape, ``window`` warp-window
         deposits, ``plane`` cluster plane kernels (``plane16``: clusters of
         16), ``vec`` vector z-pair reductions, ``agg`` warp-aggregated
         deposits, ``tma`` TMA-staged forward gathers, ``graphs`` slab loops as CUDA
         graphs, ``chains`` concurrent slab chains and ``slab_log2`` planes
-        per cuFFT execution (0: defaults).  ``slots`` > 1: a batched
+        per cuFFT execution (0: defaults); these three without effect where
+        the library's own transforms run.  ``slots`` > 1: a batched
         workspace for that many simulations of this mesh shape
         (pmx_workspace_create_batch)."""
         load()

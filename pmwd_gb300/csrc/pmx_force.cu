@@ -1829,7 +1829,7 @@ int own_meshes(pmx_workspace *ws, bool adj, int nslot, const float *c, cudaStrea
     g.unit = ws->n0 * ws->n1 * ws->n2p;
     GreenTab gt;
     for (int b = 0; b < nslot; ++b) gt.c[b] = c[b];
-    // the plane kernels write the meshes while other clusters read the spectra
+    // the plane kernels write the meshes while other blocks read the spectra
     const bool plane = ws->own_plane && !adj;
     float2 *s0 = plane ? ws->ck : reinterpret_cast<float2 *>(ws->g), *s1 = s0 + nslot * g.unit;
     const float2 *tx = ws->mtw, *ty = tx + 2 * ws->n0, *tz = ty + 2 * ws->n1;

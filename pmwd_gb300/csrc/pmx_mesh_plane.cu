@@ -260,7 +260,7 @@ k_plane_fwd(float *in, float fill, float2 *__restrict__ spec, const float2 *__re
 }
 
 // Spectra -> real planes: NC = 1, one spectrum per slot; NC = 3, G_0 (spec0) and Q
-// (spec1) -> planes (slot, x, j) of the three gradients, one cluster each.
+// (spec1) -> planes (slot, x, j) of the three gradients, one block each.
 template <int N, int NC>
 __global__ void __launch_bounds__(PlaneCfg<N>::TH)
 k_plane_inv(const float2 *__restrict__ spec0, const float2 *__restrict__ spec1,

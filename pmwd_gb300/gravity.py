@@ -1,8 +1,9 @@
 """Poisson gravity (pmwd/gravity.py:1-72).
 
-``gravity`` runs the fused CUDA force (``pmx_force``): CIC density,
-cuFFT r2c, one Fourier kernel for the Green's function and the three
-spectral gradients, batched cuFFT c2r and one 3-component CIC gather.  Its
+``gravity`` runs the fused CUDA force (``pmx_force``): CIC density, the mesh
+transforms (the library's own where they have every axis length, else cuFFT)
+with the Green's function and the three spectral gradients in between, and
+one 3-component CIC gather.  Its
 VJP (``pmx_force_vjp``) recomputes the forward force and applies the exact
 transpose of every stage, with no mesh kept between forward and backward.
 

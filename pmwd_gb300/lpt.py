@@ -1,11 +1,14 @@
 """Lagrangian perturbation theory initial conditions (pmwd/lpt.py:1-212) on
 the GPU.
 
-3-D grids on the GPU with a fixed cosmology run the stages between the
-transforms (torch.fft) as libpmx kernels, with a hand-written VJP for the
-modes (``_LptFn``); every other case (cosmology gradients, other dimensions
-and dtypes, CPU tensors) is the same computation in torch operations
-(``_lpt_device``), differentiated by autograd."""
+3-D grids on the GPU with a fixed cosmology run as libpmx kernels: without a
+gradient, where the library's own transforms have the shape and a graph does
+not replay it, in one call (``pmx_lpt_solve``); else stage by stage between
+torch.fft transforms, with a hand-written VJP for the modes (``_LptFn``).
+Every other case (cosmology gradients, other dimensions and dtypes, CPU
+tensors), a gradient of the gradient and batched cotangents are the same
+computation in torch operations (``_lpt_device``), differentiated by
+autograd."""
 
 import ctypes
 import math
@@ -244,7 +247,7 @@ class _LptFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, modes, fac, conf):
         # without a gradient no stage's result is kept, and the library's own
-        # transforms do the same with fewer passes (256^3: 1.01 against 1.87 ms)
+        # transforms do the same with fewer passes (256^3: half the time)
         out = None if ctx.needs_input_grad[0] else _lpt_solve(modes, fac, conf)
         if out is None:
             pmid, disp, vel, tab, phi = _lpt_stages(modes, fac, conf)

@@ -1,13 +1,15 @@
 """N-body time integration and its reversible adjoint (pmwd/nbody.py:1-276).
 
-The host computes every time-step factor in float64 with torch (so autograd
-reaches the cosmological parameters through the growth tables), casts them
+The host computes every time-step factor in float64, with torch where the
+cosmology needs a gradient (autograd reaches its parameters through the
+growth tables) and in NumPy otherwise (``_hostmath.op_factors``), casts them
 to float32, and drives the GPU:
 
-* default splits ((0, .5), (1, .5)) -- one fused ``pmx_nbody_step`` per step
-  (kick + drift + density deposit, r2c, Fourier kernel, batched c2r,
-  3-component gather + kick) and one fused ``pmx_nbody_adj_step`` per
-  reverse step;
+* default splits ((0, .5), (1, .5)) -- all steps of a run in one call
+  (``pmx_nbody_steps``, ``pmx_nbody_adj_steps``): kick, drift and density
+  deposit, the mesh transforms with the Fourier-space operators in between,
+  then a 3-component gather that also kicks, drifts and deposits for the
+  next step; ``kahan`` runs take one fused call per step;
 * any other ``symp_splits`` -- the reference's op sequence of ``integrate``
   / ``integrate_adj`` (nbody.py:121-162) with the single-op kernels.
 

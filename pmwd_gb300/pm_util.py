@@ -1,6 +1,6 @@
 """FFT helpers of pmwd/pm_util.py:159-344 on torch tensors (cuFFT through
 torch.fft on the GPU).  They serve the initial conditions and analysis; the
-N-body force calls cuFFT directly from libpmx."""
+N-body force transforms its meshes inside libpmx."""
 
 import math
 

@@ -17,8 +17,8 @@ server
   advances a chunk of leapfrog steps in ONE batched call
   (pmx_nbody_steps_batch / pmx_nbody_adj_steps_batch), whose particle
   kernels serve every simulation of the group in one launch and whose plane
-  transforms run over all their meshes at once; meshes the fused x pass
-  does not cover run one simulation per call;
+  transforms run over all their meshes at once; meshes that are not cubes of
+  a power of two (``batchable``) run one simulation per call;
 * lets newly admitted requests join their group at the next chunk while the
   others are mid-run (continuous batching at step granularity);
 * isolates failures: a request whose host setup or device call raises, or
@@ -106,7 +106,8 @@ def workspace_bytes(mesh_side, slots=1):
 
 
 def batchable(mesh_side):
-    """Meshes of the fused x-pass path, which batched calls need."""
+    """Cubic meshes that the server batches: all on the library's own
+    transforms (which batched calls take on any of their shapes)."""
     return mesh_side in (64, 128, 256, 512, 1024)
 
 
@@ -367,8 +368,8 @@ class BatchRejected(_lib.PmxError):
 
 class GpuEngine:
     """Device work of the scheduler.  Per request: setup, objective and
-    backprop on the request's own CUDA stream.  Groups whose mesh the fused
-    x pass covers share one batched workspace (``slots`` simulations) and
+    backprop on the request's own CUDA stream.  Groups whose mesh is
+    ``batchable`` share one batched workspace (``slots`` simulations) and
     one stream, and advance through the batched entry points; other meshes,
     and every mesh with ``batch=False`` (the plain path), run one
     simulation per call through the single-simulation entry points, on the
