@@ -2078,8 +2078,9 @@ void ws_free(pmx_workspace *ws) {
 }
 
 // Whether a workspace of this shape and flags uses the mesh transforms of
-// pmx_mesh_fft.cuh: they are faster at every supported size (a force at 64^3 40
-// against 51 us of device time, force + VJP at 1024^3 33 against 43.6 ms).
+// pmx_mesh_fft.cuh: they are faster at every supported size (forces at 64^3 28
+// against 51 us back to back, at 64 x 64 x 96 24 against 51, force + VJP at 1024^3
+// 33 against 43.6 ms).
 bool own_path(const int64_t s[3], int32_t flags) {
     return mesh_fft_supported(s[0], s[1], s[2]) && !(flags & (PMX_WS_CUFFT3D | PMX_WS_PLANE));
 }
